@@ -895,14 +895,16 @@ def main():
         # algorithmic work per launch
         N, nA, n = m.Norb, head["nA"], m.n_omega
         fam, (ms, cnt) = max(prof.items(), key=lambda kv: kv[1][0])
-        nY, Nf, nvec = nA * nA + nA * (nA + 1) // 2, head["Nf"], head["n_vec"]
+        nvec = head["n_vec"]
+        # spectra of the 12 sequences of every site pair I <= J, at twice the grid's length
+        ybytes = 12 * (nA // 2) * (nA // 2 + 1) // 2 * 2 * n * 16.0
         nh = args.nhist
         work = {  # algorithmic FLOPs (FP64 compute-bound kernels) or bytes (HBM-bound) per launch
             "dyson_gj": ("fp64", n * 8.0 * N ** 3),                       # G^r: N^3 complex MACs per energy
             "keldysh_scf2": ("fp64", n * 16.0 * nA ** 3),                 # G^< = G SL G^a: 2 nA^3 complex MACs
-            "sig2_fwdA": ("hbm", nvec * 8.0 + nY * Nf * 16.0),            # read packed G, write Y
-            "sig2_mid": ("hbm", (nY + 2.0 * nA * nA) * Nf * 16.0),         # read Y, write V
-            "sig2_invC": ("hbm", 2.0 * nA * nA * Nf * 16.0 + 2.0 * nA * nA * n * 16.0),  # read V, write Sigma
+            "sig2_fwdA": ("hbm", nvec * 8.0 + ybytes),                    # read packed G, write Y
+            "sig2_mid": ("hbm", 2.0 * ybytes),                            # read and write Y
+            "sig2_invC": ("hbm", 1.5 * ybytes),                           # read Y, write Sigma
             "broyden": ("hbm", nvec * (64.0 + 12.0 * nh) / 3.0),          # per iteration / 3 launches
         }
         # DRAM bytes per launch measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum)

@@ -229,8 +229,7 @@ void qs_server_destroy(qs_server *s);
  * core (variant 1: in shared memory, one block per SM, or in the global workspace above the
  * shared-memory limit; variant 3: in the global workspace, two blocks per SM) or unblocked
  * Gauss-Jordan (2); kind 1: Keldysh, tensor-core or CUDA-core GEMMs; kinds 2
- * and 3: the tile width 4 or 2 of the persistent Sigma2 kernels A and C, +2^20 in the key
- * for the FP32 ones; kind 4: the Keldysh step of a mixed solve's FP32 phase, variant 3 the
+ * and 3 (tiles of the Sigma2 kernels) are not decided any more; kind 4: the Keldysh step of a mixed solve's FP32 phase, variant 3 the
  * 3xTF32 kernel on the fifth-generation tensor cores, 1 / 2 the FP64 ones) are timed on the
  * first launch at a new size and the fastest is kept for the process.
  * qs_autotune(1) tunes (default), qs_autotune(0) uses the size heuristics only, 2 / 3 force

@@ -12,6 +12,7 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -58,8 +59,7 @@ def build_cuda(verbose=False, ptxas_verbose=False):
     lib = os.path.join(OUT, "libqsb200.so")
     if newer(lib, cu + hdr):
         return lib
-    objs = []
-    log = ""
+    objs, jobs = [], []
     for src in cu:
         obj = os.path.join(OUT, os.path.basename(src)[:-3] + ".o")
         cmd = [NVCC] + ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + INC,
@@ -67,8 +67,11 @@ def build_cuda(verbose=False, ptxas_verbose=False):
         if ptxas_verbose:
             cmd.insert(1, "-Xptxas=-v")
         if not newer(obj, [src] + hdr):
-            log += run(cmd, verbose)
+            jobs.append(cmd)
         objs.append(obj)
+    # the FFT instances make a few files slow to compile: all files in parallel
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        log = "".join(pool.map(lambda cmd: run(cmd, verbose), jobs))
     run([NVCC] + ARCH + ["-shared", "-o", lib] + objs + ["-lcudart"], verbose)
     if ptxas_verbose:
         print(log)

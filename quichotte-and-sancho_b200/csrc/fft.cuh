@@ -1,251 +1,204 @@
-// fft.cuh -- mixed-radix (2,3,4,5,7,8) Stockham FFTs of short sequences held in shared
-// memory, one warp per sequence.
+// fft.cuh -- transforms of length L = R1 R2 for kernels that hold many sequences side by side
+// in shared memory, two register butterflies and one shared-memory exchange per transform.
 //
 // Conventions are FFTW's, as the reference uses them (src/self_energies.f90:102-103,129,
 // 205,208): sign = -1 is the forward transform sum_j x_j exp(-2 pi i jk/L), sign = +1 the
 // backward one, both unnormalised.
 //
-// One pass of radix R over a sequence of length L with Ns = product of the radices already
-// applied (autosort Stockham, decimation in time):
-//   for j in [0, L/R):  k = j mod Ns
-//     v_r = x[j + r L/R] * exp(sign 2 pi i r k / (Ns R)),   r = 0..R-1
-//     v   = DFT_R(v)
-//     y[(j / Ns) Ns R + k + r Ns] = v_r
-// After the last pass the result is in natural order. The passes alternate between the
-// sequence and a scratch sequence of the warp (out of place), so only __syncwarp is needed
-// between them, never a block barrier.
-//
-// Shared-memory index padding: element p of a sequence lives at p + p/8 (one spare complex
-// every 8), which spreads the strided accesses of the early passes over all banks.
-//
-// Twiddles come from a table twL[m] = exp(-2 pi i m / L), m < L, that the calling kernel
-// keeps in shared memory (L1 holds little next to the sequence buffers, and a global table
-// read at stride Nf/L would miss it on every access).
+// With x[j + R2 r], j < R2, r < R1:
+//   pass 1 (R2 butterflies of radix R1):  b[q][j] = W_L^{jq} sum_r x[j + R2 r] W_R1^{rq}
+//   pass 2 (R1 butterflies of radix R2):  X[q + R1 t] = sum_j b[q][j] W_R2^{jt}
+// A thread computes one butterfly of one sequence in registers. The sequences of a tile are
+// the fastest index in shared and global memory (12 spin components of a site pair times one
+// or two neighbouring columns), so that the lanes of a warp touch consecutive 16-byte words
+// in both passes whatever the radix: no bank conflicts and no index padding.
 #pragma once
 #include "qs_common.cuh"
 
 namespace qs {
 
-__host__ __device__ __forceinline__ int pidx(int p) { return p + (p >> 3); }
-__host__ __device__ __forceinline__ int padded_len(int L) { return L + (L >> 3) + 1; }
-
-// twiddle W^m from a table for the given sign
-template <typename T> __device__ __forceinline__ cplx<T> twid(const cplx<T> *tw, int m, int sign) {
-    return sign < 0 ? tw[m] : conj(tw[m]);
-}
-
 // an FP64 twiddle at the kernel's element type
 template <typename T> __device__ __forceinline__ cplx<T> cvt(zc v) { return cplx<T>{(T)v.x, (T)v.y}; }
 
-// The shared-memory twiddle table of a length-L transform. Power-of-two lengths 64/128/256:
-// the twiddles of each pass with Ns > 1 laid out [r][k] (W_L^{r k L/(Ns R)} at r Ns + k,
-// pass Ns = 8 first, then Ns = 64), so that the lanes of a pass read consecutive entries;
-// other lengths: twL[m] = W_L^m.
-__host__ __device__ __forceinline__ int fft_table_len(int L) {
-    return L == 64 ? 64 : (L == 128 ? 192 : (L == 256 ? 320 : L));
-}
-// fill it from the FP64 table of W_Nf (tw[m * tws] = W_L^m), all threads of the block
-template <typename T> __device__ void fft_table_fill(cplx<T> *tbl, int L, const zc *__restrict__ tw, int tws) {
-    if (L == 64 || L == 128 || L == 256) {
-        for (int idx = threadIdx.x; idx < 64; idx += blockDim.x) {
-            const int r = idx >> 3, k = idx & 7;
-            tbl[idx] = cvt<T>(tw[(size_t)(r * k * (L / 64)) * tws]);
-        }
-        for (int idx = threadIdx.x; idx < L; idx += blockDim.x) {  // (L / 64) x 64
-            const int r = idx >> 6, k = idx & 63;
-            if (L > 64) tbl[64 + idx] = cvt<T>(tw[(size_t)(r * k) * tws]);
-        }
-    } else {
-        for (int m = threadIdx.x; m < L; m += blockDim.x) tbl[m] = cvt<T>(tw[(size_t)m * tws]);
+// cos(2 pi k / R); k is a constant once the loops around it are unrolled
+template <int R> __device__ __forceinline__ double cosv(int k) {
+    if constexpr (R == 3) {
+        const double t[3] = {1.0, -0.5, -0.5};
+        return t[k];
+    } else if constexpr (R == 5) {
+        const double t[5] = {1.0, 0.30901699437494745, -0.8090169943749475, -0.8090169943749475,
+            0.30901699437494745};
+        return t[k];
+    } else if constexpr (R == 6) {
+        const double t[6] = {1.0, 0.5, -0.5, -1.0, -0.5, 0.5};
+        return t[k];
+    } else if constexpr (R == 7) {
+        const double t[7] = {1.0, 0.6234898018587335, -0.2225209339563144, -0.9009688679024191,
+            -0.9009688679024191, -0.2225209339563144, 0.6234898018587335};
+        return t[k];
+    } else if constexpr (R == 9) {
+        const double t[9] = {1.0, 0.766044443118978, 0.17364817766693036, -0.5, -0.9396926207859084,
+            -0.9396926207859084, -0.5, 0.17364817766693036, 0.766044443118978};
+        return t[k];
+    } else if constexpr (R == 10) {
+        const double t[10] = {1.0, 0.8090169943749475, 0.30901699437494745, -0.30901699437494745,
+            -0.8090169943749475, -1.0, -0.8090169943749475, -0.30901699437494745, 0.30901699437494745,
+            0.8090169943749475};
+        return t[k];
+    } else if constexpr (R == 12) {
+        const double t[12] = {1.0, 0.8660254037844386, 0.5, 0.0, -0.5, -0.8660254037844386, -1.0,
+            -0.8660254037844386, -0.5, 0.0, 0.5, 0.8660254037844386};
+        return t[k];
+    } else if constexpr (R == 14) {
+        const double t[14] = {1.0, 0.9009688679024191, 0.6234898018587335, 0.2225209339563144,
+            -0.2225209339563144, -0.6234898018587335, -0.9009688679024191, -1.0, -0.9009688679024191,
+            -0.6234898018587335, -0.2225209339563144, 0.2225209339563144, 0.6234898018587335,
+            0.9009688679024191};
+        return t[k];
+    } else if constexpr (R == 16) {
+        const double t[16] = {1.0, 0.9238795325112867, 0.7071067811865476, 0.3826834323650898, 0.0,
+            -0.3826834323650898, -0.7071067811865476, -0.9238795325112867, -1.0, -0.9238795325112867,
+            -0.7071067811865476, -0.3826834323650898, 0.0, 0.3826834323650898, 0.7071067811865476,
+            0.9238795325112867};
+        return t[k];
     }
+    return 0.0;
+}
+// sin(2 pi k / R); k is a constant once the loops around it are unrolled
+template <int R> __device__ __forceinline__ double sinv(int k) {
+    if constexpr (R == 3) {
+        const double t[3] = {0.0, 0.8660254037844386, -0.8660254037844386};
+        return t[k];
+    } else if constexpr (R == 5) {
+        const double t[5] = {0.0, 0.9510565162951535, 0.5877852522924731, -0.5877852522924731,
+            -0.9510565162951535};
+        return t[k];
+    } else if constexpr (R == 6) {
+        const double t[6] = {0.0, 0.8660254037844386, 0.8660254037844386, 0.0, -0.8660254037844386,
+            -0.8660254037844386};
+        return t[k];
+    } else if constexpr (R == 7) {
+        const double t[7] = {0.0, 0.7818314824680298, 0.9749279121818236, 0.4338837391175581,
+            -0.4338837391175581, -0.9749279121818236, -0.7818314824680298};
+        return t[k];
+    } else if constexpr (R == 9) {
+        const double t[9] = {0.0, 0.6427876096865394, 0.984807753012208, 0.8660254037844386, 0.3420201433256687,
+            -0.3420201433256687, -0.8660254037844386, -0.984807753012208, -0.6427876096865394};
+        return t[k];
+    } else if constexpr (R == 10) {
+        const double t[10] = {0.0, 0.5877852522924731, 0.9510565162951535, 0.9510565162951535,
+            0.5877852522924731, 0.0, -0.5877852522924731, -0.9510565162951535, -0.9510565162951535,
+            -0.5877852522924731};
+        return t[k];
+    } else if constexpr (R == 12) {
+        const double t[12] = {0.0, 0.5, 0.8660254037844386, 1.0, 0.8660254037844386, 0.5, 0.0, -0.5,
+            -0.8660254037844386, -1.0, -0.8660254037844386, -0.5};
+        return t[k];
+    } else if constexpr (R == 14) {
+        const double t[14] = {0.0, 0.4338837391175581, 0.7818314824680298, 0.9749279121818236,
+            0.9749279121818236, 0.7818314824680298, 0.4338837391175581, 0.0, -0.4338837391175581,
+            -0.7818314824680298, -0.9749279121818236, -0.9749279121818236, -0.7818314824680298,
+            -0.4338837391175581};
+        return t[k];
+    } else if constexpr (R == 16) {
+        const double t[16] = {0.0, 0.3826834323650898, 0.7071067811865476, 0.9238795325112867, 1.0,
+            0.9238795325112867, 0.7071067811865476, 0.3826834323650898, 0.0, -0.3826834323650898,
+            -0.7071067811865476, -0.9238795325112867, -1.0, -0.9238795325112867, -0.7071067811865476,
+            -0.3826834323650898};
+        return t[k];
+    }
+    return 0.0;
+}
+// v * exp(S 2 pi i k / R) for a k known at compile time (after unrolling): no multiplication
+// for the multiples of a quarter turn, one per component for the odd eighths
+template <typename T, int R, int S> __device__ __forceinline__ cplx<T> mul_root(cplx<T> v, int k) {
+    k %= R;
+    if (S < 0) k = (R - k) % R;
+    if (k == 0) return v;
+    if (4 * k == R) return {-v.y, v.x};
+    if (2 * k == R) return {-v.x, -v.y};
+    if (4 * k == 3 * R) return {v.y, -v.x};
+    const T h = (T)0.70710678118654752440084436210484903928;
+    if (8 * k == R) return {h * (v.x - v.y), h * (v.x + v.y)};
+    if (8 * k == 3 * R) return {-h * (v.x + v.y), h * (v.x - v.y)};
+    if (8 * k == 5 * R) return {h * (v.y - v.x), -h * (v.x + v.y)};
+    if (8 * k == 7 * R) return {h * (v.x + v.y), h * (v.y - v.x)};
+    const T c = (T)cosv<R>(k), s = (T)sinv<R>(k);
+    return {v.x * c - v.y * s, v.x * s + v.y * c};
 }
 
-// multiply by sign*i
-template <typename T> __device__ __forceinline__ cplx<T> mul_si(cplx<T> a, int sign) {
-    return sign < 0 ? cplx<T>{a.y, -a.x} : cplx<T>{-a.y, a.x};
+// the inner split R = P Q of a composite radix
+__host__ __device__ constexpr int dft_p(int R) {
+    return R == 16 ? 4 : R == 14 ? 2 : R == 12 ? 3 : R == 10 ? 2 : R == 9 ? 3 : R == 8 ? 2 : R == 6 ? 2 : 1;
 }
 
-template <typename T>
-__device__ __forceinline__ void bfly4(cplx<T> &a0, cplx<T> &a1, cplx<T> &a2, cplx<T> &a3, int sign) {
-    cplx<T> s02 = a0 + a2, d02 = a0 - a2, s13 = a1 + a3, d13 = mul_si(a1 - a3, sign);
-    a0 = s02 + s13;
-    a2 = s02 - s13;
-    a1 = d02 + d13;
-    a3 = d02 - d13;
-}
-
-// DFT of R points in registers
-template <typename T, int R>
-__device__ __forceinline__ void dft(cplx<T> (&v)[R], int sign, const cplx<T> *twL, int L) {
+// DFT of R points in registers, natural order in and out
+template <typename T, int R, int S> __device__ __forceinline__ void dft(cplx<T> (&v)[R]) {
     if constexpr (R == 2) {
-        cplx<T> a = v[0], b = v[1];
+        const cplx<T> a = v[0], b = v[1];
         v[0] = a + b;
         v[1] = a - b;
     } else if constexpr (R == 4) {
-        bfly4(v[0], v[1], v[2], v[3], sign);
-    } else if constexpr (R == 8) {
-        cplx<T> e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-        cplx<T> o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-        bfly4(e0, e1, e2, e3, sign);
-        bfly4(o0, o1, o2, o3, sign);
-        const T h = (T)0.70710678118654752440084436210484903928;
-        // W8^1 = (1 + sign i)/sqrt2 ; W8^2 = sign i ; W8^3 = (-1 + sign i)/sqrt2
-        cplx<T> t1 = cplx<T>{h * (o1.x - (T)sign * o1.y), h * (o1.y + (T)sign * o1.x)};
-        cplx<T> t2 = mul_si(o2, sign);
-        cplx<T> t3 = cplx<T>{h * (-o3.x - (T)sign * o3.y), h * (-o3.y + (T)sign * o3.x)};
-        v[0] = e0 + o0;
-        v[4] = e0 - o0;
-        v[1] = e1 + t1;
-        v[5] = e1 - t1;
-        v[2] = e2 + t2;
-        v[6] = e2 - t2;
-        v[3] = e3 + t3;
-        v[7] = e3 - t3;
-    } else {  // 3, 5, 7: direct DFT with table constants W_R^m = W_L^{m L/R}
-        cplx<T> o[R];
-        const int st = L / R;
+        const cplx<T> s02 = v[0] + v[2], d02 = v[0] - v[2], s13 = v[1] + v[3], d = v[1] - v[3];
+        const cplx<T> d13 = S < 0 ? cplx<T>{d.y, -d.x} : cplx<T>{-d.y, d.x};
+        v[0] = s02 + s13;
+        v[2] = s02 - s13;
+        v[1] = d02 + d13;
+        v[3] = d02 - d13;
+    } else if constexpr (R == 3 || R == 5 || R == 7) {
+        // pairs (r, R - r): the cosine terms act on their sums, the sine terms on their differences
+        constexpr int H = R / 2;
+        cplx<T> s[H], d[H];
 #pragma unroll
-        for (int q = 0; q < R; q++) {
-            cplx<T> s = v[0];
+        for (int r = 0; r < H; r++) {
+            s[r] = v[r + 1] + v[R - 1 - r];
+            d[r] = v[r + 1] - v[R - 1 - r];
+        }
+        const cplx<T> x0 = v[0];
 #pragma unroll
-            for (int r = 1; r < R; r++) {
-                const int m = (r * q) % R;
-                if (m == 0) s = s + v[r];
-                else {
-                    cplx<T> w = sign < 0 ? twL[m * st] : conj(twL[m * st]);
-                    cfma(s, v[r], w);
-                }
+        for (int r = 0; r < H; r++) v[0] = v[0] + s[r];
+#pragma unroll
+        for (int q = 1; q <= H; q++) {
+            cplx<T> a = x0, b{0, 0};
+#pragma unroll
+            for (int r = 0; r < H; r++) {
+                const int m = ((r + 1) * q) % R;
+                const T c = (T)cosv<R>(m), sn = (T)S * (T)sinv<R>(m);
+                a.x = fma(c, s[r].x, a.x);
+                a.y = fma(c, s[r].y, a.y);
+                b.x = fma(-sn, d[r].y, b.x);  // i sn d
+                b.y = fma(sn, d[r].x, b.y);
             }
-            o[q] = s;
+            v[q] = a + b;
+            v[R - q] = a - b;
+        }
+    } else {
+        constexpr int P = dft_p(R), Q = R / P;
+        static_assert(P * Q == R && P > 1, "a composite radix of the table");
+        cplx<T> b[P][Q];
+#pragma unroll
+        for (int j = 0; j < Q; j++) {
+            cplx<T> u[P];
+#pragma unroll
+            for (int r = 0; r < P; r++) u[r] = v[j + Q * r];
+            dft<T, P, S>(u);
+#pragma unroll
+            for (int q = 0; q < P; q++) b[q][j] = mul_root<T, R, S>(u[q], j * q);
         }
 #pragma unroll
-        for (int q = 0; q < R; q++) v[q] = o[q];
-    }
-}
-
-// one radix-R pass of a warp, src -> dst (both padded); butterflies are processed one at a
-// time per lane, so only R values are live in registers
-template <typename T, int R>
-__device__ __forceinline__ void warp_pass(const cplx<T> *src, cplx<T> *dst, int L, int Ns, int sign,
-                                          const cplx<T> *twL) {
-    const int lane = threadIdx.x & 31;
-    const int nR = L / R;
-    const int ang = L / (Ns * R);
-    for (int j = lane; j < nR; j += 32) {
-        cplx<T> v[R];
+        for (int q = 0; q < P; q++) {
+            dft<T, Q, S>(b[q]);
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = src[pidx(j + r * nR)];
-        const int k = j % Ns;
-        if (k) {
-#pragma unroll
-            for (int r = 1; r < R; r++) {
-                const int m = r * k * ang;  // < R Ns ang = L
-                v[r] = v[r] * (sign < 0 ? twL[m] : conj(twL[m]));
-            }
-        }
-        dft<T, R>(v, sign, twL, L);
-        const int idxD = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; r++) dst[pidx(idxD + r * Ns)] = v[r];
-    }
-    __syncwarp();
-}
-
-// the whole transform of one padded sequence s by one warp, with the warp's own scratch
-// sequence and the length-L twiddle table twL; the result is left in s
-template <typename T>
-__device__ void warp_fft(cplx<T> *s, cplx<T> *scratch, const FftLen &P, int sign, const cplx<T> *twL) {
-    cplx<T> *a = s, *b = scratch;
-    const int L = P.L;
-    int Ns = 1;
-    unsigned code = P.code;
-    for (int p = 0; p < P.nrad; p++) {
-        const int R = code & 15u;
-        code >>= 4;
-        switch (R) {
-            case 2: warp_pass<T, 2>(a, b, L, Ns, sign, twL); break;
-            case 3: warp_pass<T, 3>(a, b, L, Ns, sign, twL); break;
-            case 4: warp_pass<T, 4>(a, b, L, Ns, sign, twL); break;
-            case 5: warp_pass<T, 5>(a, b, L, Ns, sign, twL); break;
-            case 7: warp_pass<T, 7>(a, b, L, Ns, sign, twL); break;
-            default: warp_pass<T, 8>(a, b, L, Ns, sign, twL); break;
-        }
-        cplx<T> *t = a;
-        a = b;
-        b = t;
-        Ns *= R;
-    }
-    if (a != s) {
-        const int lane = threadIdx.x & 31;
-        for (int j = lane; j < L; j += 32) s[pidx(j)] = a[pidx(j)];
-        __syncwarp();
-    }
-}
-
-// ---------------------------------------------------------------------------------
-// Power-of-two lengths L = 64, 128, 256 with compile-time passes: the warp transforms
-// P = 256 / L sequences at once (sequence q at s + q ps, q < nvalid), every lane holding 8
-// complex values per pass, in place (all loads of a pass precede its stores; no scratch).
-// Passes: radix 8 (Ns = 1), radix 8 (Ns = 8), then radix L / 64 (Ns = 64) when L > 64.
-// ---------------------------------------------------------------------------------
-template <typename T, int L, int R, int Ns>
-__device__ __forceinline__ void pow2_pass(cplx<T> *s, int ps, int nvalid, int sign, const cplx<T> *twL) {
-    static_assert(Ns == 1 || Ns == 8 || Ns == 64, "the passes of warp_fft_pow2");
-    constexpr int nR = L / R;  // butterflies per sequence
-    constexpr int U = 8 / R;   // butterflies per lane
-    const int lane = threadIdx.x & 31;
-    cplx<T> v[U][R];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        const int b = lane + 32 * u, sq = b / nR, j = b % nR;
-        const cplx<T> *x = s + sq * ps;
-#pragma unroll
-        for (int r = 0; r < R; r++) v[u][r] = (sq < nvalid) ? x[pidx(j + r * nR)] : cplx<T>{0, 0};
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        const int b = lane + 32 * u, sq = b / nR, j = b % nR;
-        const int k = j % Ns;
-        if (Ns > 1 && k) {
-            constexpr int off = (Ns == 8) ? 0 : 64;  // this pass's part of the table ([r][k])
-#pragma unroll
-            for (int r = 1; r < R; r++) v[u][r] = v[u][r] * twid(twL, off + r * Ns + k, sign);
-        }
-        dft<T, R>(v[u], sign, twL, L);
-        cplx<T> *x = s + sq * ps;
-        const int idxD = (j / Ns) * Ns * R + k;
-        if (sq < nvalid) {
-#pragma unroll
-            for (int r = 0; r < R; r++) x[pidx(idxD + r * Ns)] = v[u][r];
+            for (int t = 0; t < Q; t++) v[q + P * t] = b[q][t];
         }
     }
-    __syncwarp();
 }
 
-template <typename T, int L>
-__device__ __forceinline__ void warp_fft_pow2(cplx<T> *s, int ps, int nvalid, int sign, const cplx<T> *twL) {
-    static_assert(L == 64 || L == 128 || L == 256, "power-of-two lengths 64..256");
-    pow2_pass<T, L, 8, 1>(s, ps, nvalid, sign, twL);
-    pow2_pass<T, L, 8, 8>(s, ps, nvalid, sign, twL);
-    if constexpr (L > 64) pow2_pass<T, L, L / 64, 64>(s, ps, nvalid, sign, twL);
-}
-
-// number of sequences one warp transforms per call for length L (1 on the generic path)
-__host__ __device__ __forceinline__ int fft_group(int L) { return (L == 64 || L == 128 || L == 256) ? 256 / L : 1; }
-
-// Transform the group of up to fft_group(L) sequences at s + q ps (q < nvalid) by the
-// calling warp with the table of fft_table_fill; scratch is used by the generic path (one
-// sequence per call).
-template <typename T>
-__device__ __forceinline__ void warp_fft_group(cplx<T> *s, int ps, int nvalid, cplx<T> *scratch, const FftLen &P,
-                                               int sign, const cplx<T> *twL) {
-    switch (P.L) {
-        case 64: warp_fft_pow2<T, 64>(s, ps, nvalid, sign, twL); break;
-        case 128: warp_fft_pow2<T, 128>(s, ps, nvalid, sign, twL); break;
-        case 256: warp_fft_pow2<T, 256>(s, ps, nvalid, sign, twL); break;
-        default: warp_fft(s, scratch, P, sign, twL); break;
-    }
-}
+// The transform lengths that have kernels, and their split L = R1 R2 with R1 >= R2. The radices
+// are 4..16 and the lengths at most 14 % apart, so that a product of two of them lies a few
+// percent above any length up to 65536.
+#define QS_FFT_LENGTHS(X) \
+    X(4, 4) X(5, 4) X(6, 4) X(7, 4) X(8, 4) X(6, 6) X(8, 5) X(8, 6) X(8, 7) X(8, 8) X(9, 8) X(10, 8) X(12, 8) X(14, 8) \
+    X(16, 8) X(12, 12) X(16, 10) X(16, 12) X(16, 14) X(16, 16)
 
 }  // namespace qs

@@ -112,7 +112,6 @@ __global__ void __launch_bounds__(KT_THREADS, 1) keldysh_tf32(KeldyshArgs a) {
     const uint32_t tm = tslot, tT = tm, tL = tm + 2 * KT_M;
     const uint32_t sbase = smem_u32(sm);
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;  // this warp's TMEM lane quarter
-    const int64_t offL = 2 * (int64_t)nfull, offD = offL + (int64_t)nA * (nA - 1);
     int g = 0;  // chunks staged so far: buffer g & 1, mbarrier phase g >> 1
     bool ok = true;
     // wait (block-uniformly) until the MMAs of chunk gg have completed
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) keldysh_tf32(KeldyshArgs a) {
         const zc *G = a.G + (size_t)iw * nfull;
         const double w = a.omega[iw];
         const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
-        const zc *SL2 = a.SigL ? a.SigL + (size_t)iw * nfull : nullptr;
+        const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
         // ---- T = G SL: thread (m = tid % 128, quad tid / 128) stages A = G(m, k), thread
         // (n = tid / 4, quad tid % 4) stages B = SL(k, n)
         for (int c = 0; c < KT_NCH; c++, g++) {
@@ -152,7 +151,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) keldysh_tf32(KeldyshArgs a) {
                     if (n < nA && k < nA) {  // SL(k, n) = i (fL GamL_s + fR GamR_s) / hbar + Sigma2^<  (src/scf.f90:333-336)
                         const size_t idx = k + (size_t)n * nA;
                         const zc gl = a.GamLs[idx], gr = a.GamRs[idx];
-                        const zc s2 = SL2 ? SL2[idx] : zc{0, 0};
+                        const zc s2 = SL2 ? sig_l(SL2, k, n) : zc{0, 0};
                         s = zc{-(fL * gl.y + fR * gr.y) + s2.x, fL * gl.x + fR * gr.x + s2.y};
                     }
                     re[e] = (float)s.x;
@@ -222,19 +221,22 @@ __global__ void __launch_bounds__(KT_THREADS, 1) keldysh_tf32(KeldyshArgs a) {
                 const int c = 32 * j + i;
                 if (c >= nA || r > c) continue;
                 if (r < c) {
-                    const int64_t o = offL + 2 * ((int64_t)c * (c - 1) / 2 + r);
+                    const int o = dl_l(r, c);
                     blk[o] = xb ? (double)lr[i] - xb[o] : (double)lr[i];
                     blk[o + 1] = xb ? (double)li[i] - xb[o + 1] : (double)li[i];
                 } else {
-                    blk[offD + r] = xb ? (double)li[i] - xb[offD + r] : (double)li[i];
+                    const int o = dl_d(r);
+                    blk[o] = xb ? (double)li[i] - xb[o] : (double)li[i];
                     if (a.gLd) a.gLd[(size_t)iw * nA + r] = zc{(double)lr[i], (double)li[i]};
                 }
             }
         }
         for (int idx = tid; idx < nfull; idx += KT_THREADS) {
-            const zc gv = G[idx];
-            blk[2 * idx] = xb ? gv.x - xb[2 * idx] : gv.x;
-            blk[2 * idx + 1] = xb ? gv.y - xb[2 * idx + 1] : gv.y;
+            const int e = idx & 3, i = 2 * ((idx >> 2) % (nA >> 1)) + (e & 1), j = 2 * ((idx >> 2) / (nA >> 1)) + (e >> 1);
+            const zc gv = G[i + (size_t)j * nA];
+            const int o = dl_r(i, j);  // by 2x2 blocks, as the packed layout holds them
+            blk[o] = xb ? gv.x - xb[o] : gv.x;
+            blk[o + 1] = xb ? gv.y - xb[o + 1] : gv.y;
         }
         if (a.gRd)
             for (int i = tid; i < nA; i += KT_THREADS) a.gRd[(size_t)iw * nA + i] = G[i + (size_t)i * nA];

@@ -1,17 +1,19 @@
 // qs_common.cuh -- shared definitions of the B200 NEGF solver.
 //
 // Device data layout (HBM), with nA active states, n energies, Nf padded FFT length:
-//   X, F, Fold, xold   SCF vectors, energy-major: block w (3 nA^2 doubles) holds
-//                      [ G^r  nA^2 complex, column-major, (re,im) interleaved
-//                      | G^< strict upper triangle, column by column, complex
-//                      | Im G^<_ii, nA doubles ].
+//   X, F, Fold, xold   SCF vectors, energy-major: block w (3 nA^2 doubles) holds the site
+//                      pairs I <= J, J by J (site = two consecutive active states): for I < J
+//                      12 complex values, the 2x2 blocks G^r_IJ, G^r_JI, G^<_IJ (rows fastest);
+//                      for I = J G^r_II, the element G^<_01 of the block and its two Im G^<_aa.
 //                      This is a fixed permutation of the reference's pack_gf block
 //                      (common/linear_algebra.f90:155-191), so every Broyden quantity
 //                      (norms, dots, updates) is the reference's up to summation order.
-//   SigR, SigL         Sigma2^r, Sigma2^< as n blocks of nA x nA complex, column-major
-//                      (the reference's SigR2(nA,nA,n_omega)).
-//   Y, V               FFT intermediates, sequence-major: sequence s holds Nf complex
-//                      values ordered [l1][m2] of the four-step split Nf = N1*N2.
+//   Sig                Sigma2 for each energy: per site pair (I <= J, index J(J+1)/2 + I)
+//                      the 12 values Sigma^r_IJ, Sigma^r_JI, Sigma^<_IJ; the lower blocks of
+//                      Sigma^< follow from Sigma^<_JI = -Sigma^<_IJ^+. Zero for pairs without
+//                      interaction (written once, at creation).
+//   Y                  FFT intermediates of the interacting pairs: [pair][l1][m2][12] of the
+//                      four-step split Nf = N1*N2, spectra and inverse transforms in place.
 //   gRd, gLd           diagonals (n x nA complex) for the sanity check.
 //   onsL, dosd, atomL, trU, trD   final-sweep arrays, energy-major (reference layout).
 #pragma once
@@ -67,7 +69,35 @@ template <typename T> __device__ __forceinline__ cplx<T> crecip(cplx<T> a) {
         return {r / d, T(-1) / d};
     }
 }
-template <typename D, typename S> __host__ __device__ __forceinline__ cplx<D> cvt(cplx<S> a) { return {(D)a.x, (D)a.y}; }
+
+// offset (doubles) of the pair (I <= J) in a block of an SCF vector
+__host__ __device__ __forceinline__ int dl_block(int I, int J) { return 12 * J * J + 24 * I; }
+// offsets of G^r_ij, of G^<_ij (i < j) and of Im G^<_ii
+__host__ __device__ __forceinline__ int dl_r(int i, int j) {
+    const int I = i >> 1, J = j >> 1, e = 2 * ((i & 1) + 2 * (j & 1));
+    return I <= J ? dl_block(I, J) + e : dl_block(J, I) + 8 + e;
+}
+__host__ __device__ __forceinline__ int dl_l(int i, int j) {
+    const int I = i >> 1, J = j >> 1;
+    return I < J ? dl_block(I, J) + 16 + 2 * ((i & 1) + 2 * (j & 1)) : dl_block(I, I) + 8;
+}
+__host__ __device__ __forceinline__ int dl_d(int i) { return dl_block(i >> 1, i >> 1) + 10 + (i & 1); }
+// the pair (I <= J) in an energy's Sigma2, its values, Sigma^r_ij and Sigma^<_ij
+__host__ __device__ __forceinline__ int64_t sig_block(int I, int J) { return (int64_t)12 * (J * (J + 1) / 2 + I); }
+__host__ __device__ __forceinline__ int64_t sig_stride(int nA) { return (int64_t)3 * (nA / 2) * (nA + 2); }
+__device__ __forceinline__ zc sig_r(const zc *S, int i, int j) {
+    const int I = i >> 1, J = j >> 1, e = (i & 1) + 2 * (j & 1);
+    return S[I <= J ? sig_block(I, J) + e : sig_block(J, I) + 4 + e];
+}
+// the stored element that Sigma^<_ij equals (upper blocks) or is minus the conjugate of (lower ones)
+__device__ __forceinline__ const zc *sig_l_at(const zc *S, int i, int j) {
+    const int I = i >> 1, J = j >> 1;
+    return S + (I <= J ? sig_block(I, J) + 8 + (i & 1) + 2 * (j & 1) : sig_block(J, I) + 8 + (j & 1) + 2 * (i & 1));
+}
+__device__ __forceinline__ zc sig_l(const zc *S, int i, int j) {
+    const zc v = *sig_l_at(S, i, j);
+    return (i >> 1) <= (j >> 1) ? v : zc{-v.x, v.y};
+}
 
 // FP64 tensor-core MMA, D = A B + D with A 16x16 (row), B 16x8 (col), f64 accumulate.
 // Fragments (g = lane/4, t = lane%4): a_i = A(g + 8(i&1), t + 4(i>>1)), i < 8;
@@ -100,18 +130,9 @@ constexpr int SMEM_MAX = 232448;  // max dynamic shared memory per block on sm_1
 // next to its ~1.3 KB of static shared memory (N <= 120 in FP64).
 inline bool dyson_fits_smem(int N) { return (size_t)N * N * 16 + 1536 <= (size_t)SMEM_MAX; }
 
-// FFT plan of one length L that divides Nf (radices applied in order).
-struct FftLen {
-    int L;
-    int nrad;
-    unsigned code;  // radix of pass p in bits 4p..4p+3
-    int rad[8];     // the same radices (host side)
-};
-
-// Stockham plan for Nf = N1 * N2 and the twiddle table W[k] = exp(-2 pi i k / Nf).
+// the four-step split of the padded length Nf = N1 * N2 (>= 2 n - 1)
 struct FftPlan {
     int Nf, N1, N2;
-    FftLen p1, p2;
 };
 
 // ---------------------------------------------------------------------------------
@@ -164,14 +185,14 @@ struct qs_handle {
     void *d_hdF = nullptr, *d_hU = nullptr;  // nhist columns, float (single history) or double
     // second-order self-energies and the FFT
     qs::FftPlan fft{};
-    qs::zc *d_tw = nullptr;  // Nf twiddles
-    qs::zc *d_SigR = nullptr, *d_SigL = nullptr;
-    qs::zc *d_Y = nullptr, *d_V = nullptr;
-    size_t nY = 0, nV = 0;
-    int2 *d_ydesc = nullptr;  // per Y sequence: offsets of (re, im) in a DL block (-1 = zero)
-    double *sig2_Upair = nullptr;  // U_I U_J hbar^2 (delta/2pi)^2 / Nf per site pair
-    int2 *sig2_pairs = nullptr;    // interacting site pairs I <= J
-    int sig2_npairs = 0, sig2_SA = 1, sig2_GA = 1, sig2_GC = 1;
+    qs::zc *d_tw = nullptr;  // W_Nf^k
+    qs::zc *d_Sig = nullptr;
+    qs::zc *d_Y = nullptr;          // y_elems values: the FFT intermediates, then the sweep's scratch
+    int *d_dl_perm = nullptr;       // position in a device block of each element of a pack_gf block
+    double *sig2_scale = nullptr;   // U_I U_J hbar^2 (delta/2pi)^2 / Nf per interacting site pair
+    int2 *sig2_pairs = nullptr;     // interacting site pairs I <= J
+    int sig2_npairs = 0;
+    int sig2_occ[2][3] = {};        // resident blocks per SM of kernels A, B, C: FP32, FP64 forms
     // sweep scratch
     qs::zc *d_G = nullptr;  // Dyson output (G_AA for all energies, or full G for a chunk)
     size_t G_chunk = 0;     // energies per chunk in full-G mode
@@ -252,7 +273,8 @@ struct KeldyshArgs {
     int nA, n;
     int64_t nblk;
     const zc *G;     // G_AA per energy (nA^2 complex)
-    const zc *SigL;  // Sigma2^< per energy, or nullptr
+    const zc *Sig;   // Sigma2 per energy, or nullptr
+    int64_t sig_ld;  // its values per energy
     const zc *GamLs, *GamRs;
     const double *omega;
     double V, mu, beta;
@@ -271,12 +293,22 @@ bool keldysh_tf32_fits(int nA);
 
 // launchers (implemented in the .cu files)
 int sigma2_setup(qs_handle *h);
+// the padded transform length and its split for a grid of n energies; {0, 0, 0} if there is none
+FftPlan sigma2_plan(int n);
+// interacting site pairs I <= J of a handle
+int sigma2_count_pairs(const qs_handle *h);
+// values of the handle's d_Y and of the sweep's per-block scratch at its end (order 2)
+size_t sweep_scratch_elems(const qs_handle *h);
+size_t y_elems(const qs_handle *h);
+// Sigma2^r, Sigma2^< as n blocks of nA x nA, column-major
+int sigma2_unblock(qs_handle *h, zc *SR, zc *SL);
 // fp32: FFTs, 2x2 algebra and spectra in FP32 (QS_PREC_MIXED handles), Sigma written in FP64
 int sigma2_compute(qs_handle *h, const double *d_x, bool fp32 = false);
-// autotuner (autotune.cu): kinds of decisions and the variants they choose between
+// autotuner (autotune.cu): kinds of decisions and the variants they choose between (kinds 2 and 3
+// are no longer decided: the Sigma2 kernels have one form per length)
 // TUNE_KELDYSH32: the Keldysh step of a mixed solve's FP32 phase, where the 3xTF32 tensor-core
 // kernel (keldysh_tf32.cu) competes with the two FP64 ones
-enum TuneKind { TUNE_DYSON = 0, TUNE_KELDYSH = 1, TUNE_SIG2_A = 2, TUNE_SIG2_C = 3, TUNE_KELDYSH32 = 4 };
+enum TuneKind { TUNE_DYSON = 0, TUNE_KELDYSH = 1, TUNE_KELDYSH32 = 4 };
 // DYSON_BLOCKED2: the blocked Gauss-Jordan with its matrix in the global workspace, two
 // 8-warp blocks per SM
 enum { DYSON_BLOCKED = 1, DYSON_UNBLOCKED = 2, DYSON_BLOCKED2 = 3, KELDYSH_TC = 1, KELDYSH_CUDA = 2, KELDYSH_TF32 = 3 };
@@ -305,8 +337,8 @@ int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncol
 int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_info, zc *d_ws, int ws_slots);
 int invert_batched_ws(cudaStream_t st, int N, int batch, zc *d_A, int *d_min_info, int *d_info_each, zc *d_ws,
                       int ws_slots);
-int convert_ref_to_dl(cudaStream_t st, int nA, int64_t Nw, const double *ref, double *dl);
-int convert_dl_to_ref(cudaStream_t st, int nA, int64_t Nw, const double *dl, double *ref);
+int convert_ref_to_dl(qs_handle *h, const double *ref, double *dl);
+int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref);
 
 // check_diag_sanity (common/scf_checks.f90:59-91) from the per-state sums over energies:
 // sumL[i] = sum_w G^<_ii(w), sumRim[i] = sum_w Im G^r_ii(w); state_index maps i to the

@@ -82,15 +82,13 @@ __global__ void glt0_sigma1(const double *__restrict__ x, int64_t nblk, int n, i
                             const double *__restrict__ U, double pp, zc *__restrict__ Glt0, zc *__restrict__ Sig1) {
     __shared__ double sh[4][32];
     const int I = blockIdx.x, io = 2 * I;
-    const int64_t offL = 2 * (int64_t)nA * nA, offD = offL + (int64_t)nA * (nA - 1);
-    const int64_t o01 = offL + 2 * ((int64_t)(io + 1) * io / 2 + io);  // (io, io+1), strict upper
     double v[4] = {0, 0, 0, 0};
     for (int w = threadIdx.x; w < n; w += blockDim.x) {
-        const double *b = x + (int64_t)w * nblk;
-        v[0] += b[offD + io];
-        v[1] += b[offD + io + 1];
-        v[2] += b[o01];
-        v[3] += b[o01 + 1];
+        const double *b = x + (int64_t)w * nblk + dl_block(I, I);
+        v[0] += b[10];  // Im G^<_00, Im G^<_11, G^<_01 of the site's block
+        v[1] += b[11];
+        v[2] += b[8];
+        v[3] += b[9];
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int k = 0; k < 4; k++) {
@@ -623,12 +621,27 @@ static int fill_host(qs_handle *h, const qs_problem *p) {
     return 0;
 }
 
+namespace qs {
+// Scratch of the sweep's blocks (order 2): up to 4 per SM of the larger of N nS and nA^2 values,
+// no more than four matrices per energy
+size_t sweep_scratch_elems(const qs_handle *h) {
+    const size_t per = std::max((size_t)h->Norb * std::max(h->nS, 1), (size_t)h->nA * h->nA);
+    return per * std::min<size_t>(148 * 4, (size_t)4 * h->n);
+}
+// d_Y: the FFT intermediates; once Sigma2 is formed, G of the sweep (at least G_AA of every energy
+// and one full matrix), with the blocks' scratch behind it
+size_t y_elems(const qs_handle *h) {
+    const size_t fft = (size_t)12 * sigma2_count_pairs(h) * sigma2_plan(h->n).Nf;
+    const size_t g = std::max((size_t)h->n * h->nA * h->nA, (size_t)h->Norb * h->Norb);
+    return std::max(fft, g + sweep_scratch_elems(h));
+}
+}  // namespace qs
+
 // device bytes a solve keeps (the allocations of qs_create), after setup_storage
 static size_t handle_need(const qs_handle *h) {
     const int N = h->Norb, nA = h->nA, n = h->n;
     const size_t nn = (size_t)N * N, zc_ = sizeof(zc);
     const size_t hist_el = h->single ? 4 : 8;
-    const int Nf = (h->order == 2) ? good_fft_size_h(2 * n - 1) : 0;
     size_t need = 0;
     need += nn * zc_ * 2 + (size_t)n * 8 * 1;                                // Hemb, Sig1, omega
     need += (size_t)n * (4 * h->N_sites * zc_ + N * 8 + 16);                // onsL, dosd, trU, trD
@@ -636,11 +649,10 @@ static size_t handle_need(const qs_handle *h) {
     need += (size_t)n * std::max(nA, 1) * zc_ * 2;                           // gRd, gLd
     if (!dyson_fits_smem(N) || (N > 16 && N <= 256)) need += (size_t)148 * 2 * nn * zc_;  // Gauss-Jordan workspace
     if (h->order == 2) {
-        size_t nY = (size_t)nA * nA + (size_t)nA * (nA + 1) / 2;
         need += (size_t)h->n_vec * 8 * 4;                                     // x, F, Fold, xold
         need += (size_t)broyden_ld(h->n_vec) * hist_el * 2 * h->nhist;                    // history
-        need += (size_t)n * nA * nA * zc_ * 2;                                // SigR, SigL
-        need += (nY + (size_t)2 * nA * nA) * Nf * zc_;                        // Y, V
+        need += (size_t)n * sig_stride(nA) * zc_;                             // Sigma2
+        need += y_elems(h) * zc_;                                             // Y, sweep scratch
     } else {
         const size_t G_chunk = std::max<size_t>(1, std::min<size_t>((size_t)n, (2ull << 30) / (nn * zc_)));
         need += G_chunk * nn * zc_;                                           // full-G chunk
@@ -650,8 +662,8 @@ static size_t handle_need(const qs_handle *h) {
     }
     need += broyden_red_len() * 8 + (size_t)3 * h->nS * h->nS * zc_;        // reductions, Gamma blocks
     if (h->order == 2) {
-        size_t nY = (size_t)nA * nA + (size_t)nA * (nA + 1) / 2;
-        need += (size_t)Nf * zc_ + nY * 8 + (size_t)h->nAs * h->nAs * 16;      // twiddles, FFT tables
+        need += (size_t)sigma2_plan(n).Nf * zc_ + (size_t)3 * nA * nA * 4;    // twiddles, layout table
+        need += (size_t)h->nAs * (h->nAs + 1) / 2 * 16;                       // pair tables
     }
     need += (size_t)1 << 20;  // index tables and the allocations' 256-byte granularity
     return need;
@@ -678,7 +690,6 @@ int qs_create(const qs_problem *p, qs_handle **out) {
     const int N = h->Norb;
     const size_t nn = (size_t)N * N;
     const int nA = h->nA, nS = h->nS, n = h->n;
-    const int Nf = (h->order == 2) ? good_fft_size_h(2 * n - 1) : 0;
     const size_t zc_ = sizeof(zc);
     size_t hist_el = h->single ? 4 : 8;
     // ---- HBM admission: everything this solve keeps on the device
@@ -764,11 +775,12 @@ int qs_create(const qs_problem *p, qs_handle **out) {
                              (rc = dalloc(h, &h->d_hU, broyden_ld(h->n_vec) * hist_el * h->nhist))))
             return rc;
         if ((rc = sigma2_setup(h))) return rc;
+        const size_t scratch = sweep_scratch_elems(h), gsz = y_elems(h) - scratch;
         h->d_G = h->d_Y;
-        h->G_chunk = std::min<size_t>((size_t)n, (h->nY * (size_t)h->fft.Nf) / nn);
-        h->d_T = h->d_V;
-        h->T_bytes = h->nV * (size_t)h->fft.Nf * zc_;
-        h->T_slots = std::min<size_t>(148 * 4, h->T_bytes / (std::max(Trows, (size_t)nA * nA) * zc_));
+        h->G_chunk = std::min<size_t>((size_t)n, gsz / nn);
+        h->d_T = h->d_Y + gsz;
+        h->T_bytes = scratch * zc_;
+        h->T_slots = std::min<size_t>(148 * 4, scratch / std::max(Trows, (size_t)nA * nA));
     } else {
         if (h->order == 1) {
             int64_t nv = std::max<int64_t>(h->n_vec, 1);
@@ -843,7 +855,7 @@ int qs_profile(qs_handle *h, int enable, double *ms, int64_t *launches, int nfam
 }
 int64_t qs_vector_length(const qs_handle *h) { return h->n_vec; }
 int qs_active_states(const qs_handle *h) { return h->nA; }
-int qs_fft_length(const qs_handle *h) { return h->order == 2 ? h->fft.Nf : good_fft_size_h(2 * h->n - 1); }
+int qs_fft_length(const qs_handle *h) { return good_fft_size_h(2 * h->n - 1); }
 
 int qs_solve_scf(qs_handle *h, double Volt, int fresh_start, qs_scf_result *res) {
     QS_CUDA(h, cudaSetDevice(h->device));
@@ -945,7 +957,7 @@ int qs_initial_vector(qs_handle *h, double Volt, double *x) {
     int rc;
     if (h->order == 2) {
         if ((rc = sweep(h, M_INIT2, Volt, false, h->d_x, nullptr))) return rc;
-        if ((rc = convert_dl_to_ref(h->stream, h->nA, h->n, h->d_x, h->d_F))) return -rc;
+        if ((rc = convert_dl_to_ref(h, h->d_x, h->d_F))) return -rc;
         QS_CUDA(h, cudaMemcpyAsync(x, h->d_F, sizeof(double) * h->n_vec, cudaMemcpyDeviceToHost, h->stream));
         int info;
         return read_info(h, info);
@@ -972,13 +984,13 @@ int qs_residual(qs_handle *h, double Volt, const double *x, double *F, int *abor
     if (h->order == 2) {
         // the reference-layout x goes through d_F as staging, then into d_x (device layout)
         QS_CUDA(h, cudaMemcpyAsync(h->d_F, x, sizeof(double) * h->n_vec, cudaMemcpyHostToDevice, h->stream));
-        if ((rc = convert_ref_to_dl(h->stream, h->nA, h->n, h->d_F, h->d_x))) return -rc;
+        if ((rc = convert_ref_to_dl(h, h->d_F, h->d_x))) return -rc;
         Residual2 r;
         r.h = h;
         r.V = Volt;
         // a QS_PREC_MIXED handle evaluates the residual of its solves' FP32 phase
         if ((rc = r.eval(h->d_x, h->d_Fold, ab, h->precision == QS_PREC_MIXED))) return rc;
-        if ((rc = convert_dl_to_ref(h->stream, h->nA, h->n, h->d_Fold, h->d_F))) return -rc;
+        if ((rc = convert_dl_to_ref(h, h->d_Fold, h->d_F))) return -rc;
         QS_CUDA(h, cudaMemcpyAsync(F, h->d_F, sizeof(double) * h->n_vec, cudaMemcpyDeviceToHost, h->stream));
         QS_CUDA(h, cudaStreamSynchronize(h->stream));
         h->have_x = false;
@@ -1003,12 +1015,16 @@ int qs_self_energies(qs_handle *h, const double *x, double *SigR2, double *SigL2
     QS_CUDA(h, cudaSetDevice(h->device));
     int rc;
     QS_CUDA(h, cudaMemcpyAsync(h->d_F, x, sizeof(double) * h->n_vec, cudaMemcpyHostToDevice, h->stream));
-    if ((rc = convert_ref_to_dl(h->stream, h->nA, h->n, h->d_F, h->d_x))) return -rc;
+    if ((rc = convert_ref_to_dl(h, h->d_F, h->d_x))) return -rc;
     if ((rc = equal_time_lesser_sigma1(h, h->d_x))) return rc;
     if ((rc = sigma2_compute(h, h->d_x, h->precision == QS_PREC_MIXED))) return rc;
     const size_t bytes = sizeof(zc) * (size_t)h->n * h->nA * h->nA;
-    if (SigR2) QS_CUDA(h, cudaMemcpyAsync(SigR2, h->d_SigR, bytes, cudaMemcpyDeviceToHost, h->stream));
-    if (SigL2) QS_CUDA(h, cudaMemcpyAsync(SigL2, h->d_SigL, bytes, cudaMemcpyDeviceToHost, h->stream));
+    if (SigR2 || SigL2) {  // into the reference's layout, in two SCF vectors no longer needed
+        zc *SR = (zc *)h->d_Fold, *SL = (zc *)h->d_F;
+        if ((rc = sigma2_unblock(h, SR, SL))) return rc;
+        if (SigR2) QS_CUDA(h, cudaMemcpyAsync(SigR2, SR, bytes, cudaMemcpyDeviceToHost, h->stream));
+        if (SigL2) QS_CUDA(h, cudaMemcpyAsync(SigL2, SL, bytes, cudaMemcpyDeviceToHost, h->stream));
+    }
     if (Sig1) QS_CUDA(h, cudaMemcpyAsync(Sig1, h->d_Sig1, sizeof(zc) * (size_t)h->Norb * h->Norb, cudaMemcpyDeviceToHost, h->stream));
     QS_CUDA(h, cudaStreamSynchronize(h->stream));
     h->have_x = false;

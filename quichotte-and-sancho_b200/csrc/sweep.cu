@@ -38,7 +38,8 @@ __device__ __forceinline__ void warp_argmax(double &v, int &i) {
 
 struct DysonArgs {
     int N, nA, iw0, iw1;
-    const zc *Hemb, *Sig1, *SigR;
+    const zc *Hemb, *Sig1, *Sig;
+    int64_t sig_ld;
     const int *pos;  // full index -> active index, -1 if inactive
     const int *act;
     const double *omega;
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
             for (int idx = tid; idx < N * N; idx += nthr) M[idx] = A[idx];
         } else {
             const double w = a.omega[iw];
-            const zc *SR = a.SigR + (size_t)iw * a.nA * a.nA;
+            const zc *SR = a.Sig + iw * a.sig_ld;
             for (int idx = tid; idx < N * N; idx += nthr) {
                 int i = idx % N, j = idx / N;
                 zc v = a.Hemb[idx];
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
                     int pi = a.pos[i], pj = a.pos[j];
                     if (pi >= 0 && pj >= 0) {
                         zc s = a.Sig1[idx];
-                        if (a.order2) s = s + SR[pi + (size_t)pj * a.nA];
+                        if (a.order2) s = s + sig_r(SR, pi, pj);
                         v = v - s;
                     }
                 }
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
             for (int idx = tid; idx < N * N; idx += nthr) M[bix<GM>(idx % N, idx / N, N)] = A[idx];
         } else {
             const double w = a.omega[iw];
-            const zc *SR = a.SigR + (size_t)iw * a.nA * a.nA;
+            const zc *SR = a.Sig + iw * a.sig_ld;
 #pragma unroll 4
             for (int idx = tid; idx < N * N; idx += nthr) {
                 int i = idx % N, j = idx / N;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
                     int pi = a.pos[i], pj = a.pos[j];
                     if (pi >= 0 && pj >= 0) {
                         zc sg = a.Sig1[idx];
-                        if (a.order2) sg = sg + SR[pi + (size_t)pj * a.nA];
+                        if (a.order2) sg = sg + sig_r(SR, pi, pj);
                         v = v - sg;
                     }
                 }
@@ -541,6 +542,15 @@ __device__ void cta_gemm(int M, int N, int K, LA la, LB lb, ST st, zc *sA, zc *s
     }
 }
 
+// element idx of an nA x nA matrix walked by 2x2 site blocks (rows fastest inside a block, then
+// the blocks of a column): adjacent lanes touch whole 64-byte blocks of the packed layout and
+// runs of the column-major one
+__device__ __forceinline__ void block_order(int idx, int nA, int &i, int &j) {
+    const int e = idx & 3, q = idx >> 2, s = nA >> 1;
+    i = 2 * (q % s) + (e & 1);
+    j = 2 * (q / s) + (e >> 1);
+}
+
 // modes M_INIT2 / M_SCF2: T = G^r SL, G^< = T G^r^dagger (upper triangle), packed.
 __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
     __shared__ zc sA[TB * TK], sB[TB * TK];
@@ -550,13 +560,13 @@ __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
         const zc *G = a.G + (size_t)iw * nfull;
         const double w = a.omega[iw];
         const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
-        const zc *SL2 = a.SigL ? a.SigL + (size_t)iw * nfull : nullptr;
+        const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
         // SL = i (fL GamL_s + fR GamR_s) / hbar  (+ Sigma2^<)   (src/scf.f90:333-336)
         auto ldSL = [&](int k, int j) {
             size_t idx = k + (size_t)j * nA;
             zc g{fL * a.GamLs[idx].x + fR * a.GamRs[idx].x, fL * a.GamLs[idx].y + fR * a.GamRs[idx].y};
             zc s{-g.y, g.x};
-            if (SL2) s = s + SL2[idx];
+            if (SL2) s = s + sig_l(SL2, k, j);
             return s;
         };
         cta_gemm(
@@ -565,27 +575,29 @@ __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
         __syncthreads();
         double *blk = a.out + (size_t)iw * a.nblk;
         const double *xb = a.xsub ? a.xsub + (size_t)iw * a.nblk : nullptr;
-        const int64_t offL = 2 * (int64_t)nfull, offD = offL + (int64_t)nA * (nA - 1);
         cta_gemm(
             nA, nA, nA, [&](int i, int k) { return T[i + (size_t)k * nA]; },
             [&](int k, int j) { return conj(G[j + (size_t)k * nA]); },
             [&](int i, int j, zc v) {
                 if (i < j) {
-                    int64_t o = offL + 2 * ((int64_t)j * (j - 1) / 2 + i);
+                    const int o = dl_l(i, j);
                     blk[o] = xb ? v.x - xb[o] : v.x;
                     blk[o + 1] = xb ? v.y - xb[o + 1] : v.y;
                 } else if (i == j) {
-                    blk[offD + i] = xb ? v.y - xb[offD + i] : v.y;
+                    const int o = dl_d(i);
+                    blk[o] = xb ? v.y - xb[o] : v.y;
                     if (a.gLd) a.gLd[(size_t)iw * nA + i] = v;
                 }
             },
             sA, sB, true);
         // G^r part of the block
         for (int idx = threadIdx.x; idx < nfull; idx += blockDim.x) {
-            zc g = G[idx];
-            blk[2 * idx] = xb ? g.x - xb[2 * idx] : g.x;
-            blk[2 * idx + 1] = xb ? g.y - xb[2 * idx + 1] : g.y;
-            int i = idx % nA, j = idx / nA;
+            int i, j;
+            block_order(idx, nA, i, j);
+            const zc g = G[i + (size_t)j * nA];
+            const int o = dl_r(i, j);
+            blk[o] = xb ? g.x - xb[o] : g.x;
+            blk[o + 1] = xb ? g.y - xb[o + 1] : g.y;
             if (i == j && a.gRd) a.gRd[(size_t)iw * nA + i] = g;
         }
         __syncthreads();
@@ -608,11 +620,12 @@ __device__ __forceinline__ void cpa16(void *dst, const void *src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-// C(m0 + 0..31, n0 + 0..8NT-1) = A B over k < nA. A: nA x nA column-major; B(k, n) =
-// Bm[k + n nA], staged [n][k]; only columns nlo..nhi-1 of B are staged. Every thread of the
+// C(m0 + 0..31, n0 + 0..8NT-1) = A B over k < nA. A: nA x nA column-major; B(k, n) staged
+// [n][k], with SIG Sigma2^< of an energy (sig_l; its lower blocks are staged as stored and get
+// their sign at the fragment loads), else Bm[k + n nA]; only columns nlo..nhi-1 of B are staged. Every thread of the
 // block calls it (the panel copies); warps with !active skip the MMAs, and tiles beyond nA
 // are skipped (warp-uniform).
-template <int NT>
+template <int NT, bool SIG>
 __device__ __forceinline__ void kd_gemm(const zc *__restrict__ A, const zc *__restrict__ Bm, int nA, int nlo, int nhi,
                                         int m0, int n0, bool active, zc *sm, double (&cr)[2][NT][4],
                                         double (&ci)[2][NT][4]) {
@@ -635,7 +648,8 @@ __device__ __forceinline__ void kd_gemm(const zc *__restrict__ A, const zc *__re
         for (int idx = tid; idx < 16 * nw; idx += blockDim.x) {
             const int kk = idx & 15, nn = nlo + (idx >> 4);
             const bool v = nn < nA && k0 + kk < nA;
-            cpa16(&Bs[nn * KD_LDN + kk], v ? Bm + (k0 + kk) + (size_t)nn * nA : Bm, v);
+            const zc *src = SIG ? sig_l_at(Bm, k0 + kk, nn) : Bm + (k0 + kk) + (size_t)nn * nA;
+            cpa16(&Bs[nn * KD_LDN + kk], v ? src : Bm, v);
         }
     };
     load(0, 0);
@@ -665,7 +679,8 @@ __device__ __forceinline__ void kd_gemm(const zc *__restrict__ A, const zc *__re
                 double br[4], bi[4], nbi[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const zc v = Bs[(c0 + g) * KD_LDN + t4 + 4 * q];
+                    zc v = Bs[(c0 + g) * KD_LDN + t4 + 4 * q];
+                    if (SIG && ((16 * kc + t4 + 4 * q) >> 1) > ((c0 + g) >> 1)) v.x = -v.x;
                     br[q] = v.x;
                     bi[q] = v.y;
                     nbi[q] = -v.y;
@@ -798,19 +813,17 @@ __global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     zc *T = a.Tws + (size_t)(2 * blockIdx.x) * nfull;
     zc *S = T + nfull;
-    const int64_t offL = 2 * (int64_t)nfull, offD = offL + (int64_t)nA * (nA - 1);
     for (int iw = blockIdx.x; iw < a.n; iw += gridDim.x) {
         const zc *G = a.G + (size_t)iw * nfull;
         const double w = a.omega[iw];
         const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
-        const zc *SL2 = a.SigL ? a.SigL + (size_t)iw * nfull : nullptr;
+        const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
         // SL = i (fL GamL_s + fR GamR_s) / hbar + Sigma2^<   (src/scf.f90:333-336). With
         // few contact states (the usual case) the first product takes Sigma2^< itself as
         // its B operand and the lead term is added to the contact columns of T afterwards
         // (a rank-nc correction); otherwise SL is built in the block's scratch (the loads
         // of 8 elements a thread issued before their stores).
         const bool lowrank = SL2 && a.nc >= 0 && a.nc <= KD_NCMAX;
-        const zc *Bop = lowrank ? SL2 : S;
         for (int base = threadIdx.x; !lowrank && base < nfull; base += 8 * blockDim.x) {
             zc gl[8], gr[8], s2[8];
 #pragma unroll
@@ -819,7 +832,7 @@ __global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
                 const bool v = idx < nfull;
                 gl[u] = v ? a.GamLs[idx] : zc{0, 0};
                 gr[u] = v ? a.GamRs[idx] : zc{0, 0};
-                s2[u] = (v && SL2) ? SL2[idx] : zc{0, 0};
+                s2[u] = (v && SL2) ? sig_l(SL2, idx % nA, idx / nA) : zc{0, 0};
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
@@ -834,7 +847,8 @@ __global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
             if (64 * hh >= nA) break;
             double cr[2][4][4], ci[2][4][4];
             const int m0 = 32 * (warp & 3), n0 = 64 * hh + 32 * (warp >> 2);
-            kd_gemm<4>(G, Bop, nA, 64 * hh, 64 * hh + 64, m0, n0, m0 < nA && n0 < nA, sm, cr, ci);
+            if (lowrank) kd_gemm<4, true>(G, SL2, nA, 64 * hh, 64 * hh + 64, m0, n0, m0 < nA && n0 < nA, sm, cr, ci);
+            else kd_gemm<4, false>(G, S, nA, 64 * hh, 64 * hh + 64, m0, n0, m0 < nA && n0 < nA, sm, cr, ci);
 #pragma unroll
             for (int mi = 0; mi < 2; mi++)
 #pragma unroll
@@ -868,11 +882,12 @@ __global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
         auto put = [&](int r, int c, double vr, double vi) {
             if (r >= nA || c >= nA || r > c) return;
             if (r < c) {
-                const int64_t o = offL + 2 * ((int64_t)c * (c - 1) / 2 + r);
+                const int o = dl_l(r, c);
                 blk[o] = xb ? vr - xb[o] : vr;
                 blk[o + 1] = xb ? vi - xb[o + 1] : vi;
             } else {
-                blk[offD + r] = xb ? vi - xb[offD + r] : vi;
+                const int o = dl_d(r);
+                blk[o] = xb ? vi - xb[o] : vi;
                 if (a.gLd) a.gLd[(size_t)iw * nA + r] = zc{vr, vi};
             }
         };
@@ -880,22 +895,23 @@ __global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
         kd_upper_gemm(T, G, nA, sm, put);
         // G^r part of the block (8 elements a thread in flight)
         for (int base = threadIdx.x; base < nfull; base += 8 * blockDim.x) {
-            zc gv[8];
-            double xr[8], xi[8];
+            zc gv[8], xv[8];
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int idx = base + u * blockDim.x;
+                int i, j;
+                block_order(idx, nA, i, j);
                 const bool v = idx < nfull;
-                gv[u] = v ? G[idx] : zc{0, 0};
-                xr[u] = (v && xb) ? xb[2 * idx] : 0.0;
-                xi[u] = (v && xb) ? xb[2 * idx + 1] : 0.0;
+                gv[u] = v ? G[i + (size_t)j * nA] : zc{0, 0};
+                xv[u] = (v && xb) ? *(const zc *)(xb + dl_r(i, j)) : zc{0, 0};
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int idx = base + u * blockDim.x;
                 if (idx < nfull) {
-                    blk[2 * idx] = gv[u].x - xr[u];
-                    blk[2 * idx + 1] = gv[u].y - xi[u];
+                    int i, j;
+                    block_order(idx, nA, i, j);
+                    *(zc *)(blk + dl_r(i, j)) = gv[u] - xv[u];
                 }
             }
         }
@@ -909,7 +925,7 @@ struct FinalArgs {
     int N, nS, nA, nCL, N_sites, N_atoms, iw0, iw1, mode;
     const zc *G;  // full G per energy of the chunk
     const int *sup, *act, *pos, *cl, *site_int, *atom_first, *atom_norb, *atom_off;
-    const zc *GamLs, *GamRs, *GamLcl, *SigL;
+    const zc *GamLs, *GamRs, *GamLcl, *Sig;
     const double *omega;
     double V, mu, beta;
     zc *Tws;
@@ -931,12 +947,12 @@ __global__ void __launch_bounds__(256) final_outputs(FinalArgs a) {
         auto g = [&](int i, int j) { return G[i + (size_t)j * N]; };
         const double w = a.omega[iw];
         const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
-        const zc *SL2 = a.SigL ? a.SigL + (size_t)iw * a.nA * a.nA : nullptr;
+        const zc *SL2 = a.Sig ? a.Sig + iw * sig_stride(a.nA) : nullptr;
         auto ldSL = [&](int k, int j) {
             size_t idx = k + (size_t)j * nS;
             zc gg{fL * a.GamLs[idx].x + fR * a.GamRs[idx].x, fL * a.GamLs[idx].y + fR * a.GamRs[idx].y};
             zc s{-gg.y, gg.x};
-            if (SL2) s = s + SL2[idx];
+            if (SL2) s = s + sig_l(SL2, k, j);
             return s;
         };
         // T = w1(rows, sup) SL
@@ -1045,50 +1061,26 @@ int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncol
 }
 
 // ---------------------------------------------------------------------------------
-// pack_gf layout <-> device layout (per energy block of 3 nA^2 doubles)
-//   reference (common/linear_algebra.f90:155-191): Re G^r (row-major i,j) | Im G^r |
-//     Re G^< strict upper (row-major, j > i) | Im G^< upper (row-major, j >= i)
+// pack_gf layout <-> device layout, per energy block of 3 nA^2 doubles through the table of
+// positions (d_dl_perm, built in sigma2_setup)
 // ---------------------------------------------------------------------------------
-__global__ void ref_dl_perm(int nA, int64_t Nw, const double *__restrict__ src, double *__restrict__ dst, int to_dl) {
-    const int64_t nblk = 3 * (int64_t)nA * nA;
-    const int nfull = nA * nA, nsu = (nfull - nA) / 2;
+__global__ void ref_dl_perm(int64_t nblk, int64_t Nw, const int *__restrict__ perm, const double *__restrict__ src,
+                            double *__restrict__ dst, int to_dl) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < Nw * nblk; t += (int64_t)gridDim.x * blockDim.x) {
-        int64_t w = t / nblk;
-        int e = (int)(t - w * nblk);
-        // e indexes the reference block; compute its device position
-        int64_t dpos;
-        if (e < 2 * nfull) {
-            int part = e / nfull, r = e % nfull;  // r = i*nA + j
-            int i = r / nA, j = r % nA;
-            dpos = 2 * ((int64_t)i + (int64_t)j * nA) + part;
-        } else if (e < 2 * nfull + nsu) {
-            int r = e - 2 * nfull;  // r-th strict-upper element in row-major order
-            // row i holds nA-1-i elements
-            int i = 0, acc = 0;
-            while (acc + (nA - 1 - i) <= r) { acc += nA - 1 - i; i++; }
-            int j = i + 1 + (r - acc);
-            dpos = 2 * (int64_t)nfull + 2 * ((int64_t)j * (j - 1) / 2 + i);
-        } else {
-            int r = e - 2 * nfull - nsu;  // r-th upper element (j >= i), row-major
-            int i = 0, acc = 0;
-            while (acc + (nA - i) <= r) { acc += nA - i; i++; }
-            int j = i + (r - acc);
-            if (i == j) dpos = 2 * (int64_t)nfull + (int64_t)nA * (nA - 1) + i;
-            else dpos = 2 * (int64_t)nfull + 2 * ((int64_t)j * (j - 1) / 2 + i) + 1;
-        }
-        if (to_dl) dst[w * nblk + dpos] = src[t];
-        else dst[t] = src[w * nblk + dpos];
+        const int64_t w = t / nblk, d = w * nblk + perm[t - w * nblk];
+        if (to_dl) dst[d] = src[t];
+        else dst[t] = src[d];
     }
 }
 
-int convert_ref_to_dl(cudaStream_t st, int nA, int64_t Nw, const double *ref, double *dl) {
+int convert_ref_to_dl(qs_handle *h, const double *ref, double *dl) {
     count_launch();
-    ref_dl_perm<<<1184, 256, 0, st>>>(nA, Nw, ref, dl, 1);
+    ref_dl_perm<<<1184, 256, 0, h->stream>>>(h->nblk, h->n, h->d_dl_perm, ref, dl, 1);
     return (int)cudaGetLastError();
 }
-int convert_dl_to_ref(cudaStream_t st, int nA, int64_t Nw, const double *dl, double *ref) {
+int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref) {
     count_launch();
-    ref_dl_perm<<<1184, 256, 0, st>>>(nA, Nw, dl, ref, 0);
+    ref_dl_perm<<<1184, 256, 0, h->stream>>>(h->nblk, h->n, h->d_dl_perm, dl, ref, 0);
     return (int)cudaGetLastError();
 }
 
@@ -1234,7 +1226,8 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
     a.nA = nA;
     a.Hemb = h->d_Hemb;
     a.Sig1 = h->d_Sig1;
-    a.SigR = h->d_SigR;
+    a.Sig = h->d_Sig;
+    a.sig_ld = sig_stride(nA);
     a.pos = h->d_pos;
     a.act = h->d_act;
     a.omega = h->d_omega;
@@ -1261,7 +1254,8 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         k.n = n;
         k.nblk = h->nblk;
         k.G = h->d_G;
-        k.SigL = (use_sigma && h->order == 2) ? h->d_SigL : nullptr;
+        k.Sig = (use_sigma && h->order == 2) ? h->d_Sig : nullptr;
+        k.sig_ld = sig_stride(nA);
         k.GamLs = h->d_GamLs;
         k.GamRs = h->d_GamRs;
         k.omega = h->d_omega;
@@ -1339,7 +1333,7 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         f.GamLs = h->d_GamLs;
         f.GamRs = h->d_GamRs;
         f.GamLcl = h->d_GamLcl;
-        f.SigL = (use_sigma && h->order == 2) ? h->d_SigL : nullptr;
+        f.Sig = (use_sigma && h->order == 2) ? h->d_Sig : nullptr;
         f.omega = h->d_omega;
         f.V = V;
         f.mu = h->mu;
