@@ -2,7 +2,8 @@
 // vectors: broyden_solve (common/broyden_mixing.f90:51-184) with its history in HBM.
 //
 // Every O(n) step is an FP64 device reduction or update; the host sees only the scalars
-// it needs each step (max|F|, rms|F|, ||dF||, the nh x nh Gram column and dF^T F) and
+// it needs each step (max|F|, rms|F|, ||dF||, the nh x nh Gram column and dF^T F; the last block of
+// a kernel adds the blocks' partials, which a second kernel of one block took 40-75 us for) and
 // solves the nh x nh system (nh <= nhist) as the reference's dposv does. One pass of
 // hist_update writes the new history column pair AND accumulates its Gram column and
 // dF^T F against the whole history, so each history column is read once per step for the
@@ -14,6 +15,7 @@
 #include <cmath>
 
 #include "qs_common.cuh"
+#include "reduce.cuh"
 
 namespace qs {
 
@@ -47,10 +49,11 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sh /* [NV][RE
     __syncthreads();
 }
 
-// partials[b] = (max |F|, sum F^2, sum (F-Fold)^2)
+// out = (max |F|, sum F^2, sum (F-Fold)^2), from the blocks' partials
 __global__ void __launch_bounds__(256) vec_norms(const double *__restrict__ F, const double *__restrict__ Fold, int64_t n,
-                                                 double *__restrict__ part) {
-    __shared__ double sh[3 * 32];
+                                                 double *__restrict__ part, int *__restrict__ cnt,
+                                                 double *__restrict__ out) {
+    __shared__ double sh[256];
     double mx = 0.0, v[2] = {0.0, 0.0};
     const int64_t n2 = n / 2;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -86,6 +89,7 @@ __global__ void __launch_bounds__(256) vec_norms(const double *__restrict__ F, c
         part[3 * blockIdx.x + 1] = v[0];
         part[3 * blockIdx.x + 2] = v[1];
     }
+    if (last_block(cnt, gridDim.x)) part_reduce(part, gridDim.x, 3, 3, true, sh, out);
 }
 
 // New history pair in slot `slot` plus the Gram column and dF^T F over nh <= NH columns
@@ -182,8 +186,9 @@ __global__ void __launch_bounds__(256, NH >= 8 ? 1 : 2) hist_update(const double
                                                       const double *__restrict__ x, const double *__restrict__ xold,
                                                       int64_t n, int64_t ld, double fnorm, double alpha,
                                                       HT *__restrict__ dF, HT *__restrict__ U, int slot, int nh,
-                                                      int store, double *__restrict__ part) {
-    __shared__ double sh[2 * NH * 8];
+                                                      int store, double *__restrict__ part, int *__restrict__ cnt,
+                                                      double *__restrict__ out) {
+    __shared__ double sh[2 * NH * 8 > 256 ? 2 * NH * 8 : 256];
     double g[NH], c[NH];
 #pragma unroll
     for (int k = 0; k < NH; k++) { g[k] = 0.0; c[k] = 0.0; }
@@ -271,6 +276,7 @@ __global__ void __launch_bounds__(256, NH >= 8 ? 1 : 2) hist_update(const double
         for (int w = 0; w < nw; w++) s2 += sh[t * 8 + w];
         part[(int64_t)blockIdx.x * 2 * MAXH + t] = s2;
     }
+    if (last_block(cnt, gridDim.x)) part_reduce(part, gridDim.x, 2 * MAXH, 2 * nh, false, sh, out);
 }
 
 // The same step for long histories (NH = 16, 32) with the columns split over SPL = NH / 8
@@ -284,7 +290,8 @@ __global__ void __launch_bounds__(256, 2) hist_update_split(const double *__rest
                                                             const double *__restrict__ xold, int64_t n, int64_t ld,
                                                             double fnorm, double alpha, HT *__restrict__ dF,
                                                             HT *__restrict__ U, int slot, int nh, int store,
-                                                            double *__restrict__ part) {
+                                                            double *__restrict__ part, int *__restrict__ cnt,
+                                                            double *__restrict__ out) {
     constexpr int CPT = 8, SPL = NH / CPT, E = 4;
     __shared__ double sh[2 * NH * 8];
     const int h = threadIdx.x % SPL;  // this thread's column block: columns h CPT .. h CPT + 7
@@ -380,22 +387,26 @@ __global__ void __launch_bounds__(256, 2) hist_update_split(const double *__rest
         for (int w = 0; w < nw; w++) s2 += sh[t * 8 + w];
         part[(int64_t)blockIdx.x * 2 * MAXH + t] = s2;
     }
+    if (last_block(cnt, gridDim.x)) part_reduce(part, gridDim.x, 2 * MAXH, 2 * nh, false, sh, out);
 }
 
 template <typename HT>
 static void launch_hist(int nb, cudaStream_t st, const double *F, const double *Fold, const double *x, const double *xold,
-                        int64_t n, double fnorm, double alpha, HT *dF, HT *U, int slot, int nh, int store, double *part) {
+                        int64_t n, double fnorm, double alpha, HT *dF, HT *U, int slot, int nh, int store, double *part,
+                        int *cnt, double *out) {
     const int64_t ld = broyden_ld(n);
     if (nh <= 4)
-        hist_update<HT, 4><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh, store, part);
+        hist_update<HT, 4><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh, store, part, cnt,
+                                                     out);
     else if (nh <= 8)
-        hist_update<HT, 8><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh, store, part);
+        hist_update<HT, 8><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh, store, part, cnt,
+                                                     out);
     else if (nh <= 16)
         hist_update_split<HT, 16><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh,
-                                                               store, part);
+                                                               store, part, cnt, out);
     else
         hist_update_split<HT, 32><<<nb, RED_THREADS, 0, st>>>(F, Fold, x, xold, n, ld, fnorm, alpha, dF, U, slot, nh,
-                                                               store, part);
+                                                               store, part, cnt, out);
 }
 
 // x_new = x + alpha F - sum_k gamma_k U_k   (common/broyden_mixing.f90:165-178), the
@@ -426,19 +437,6 @@ __global__ void __launch_bounds__(256) x_update(const double *__restrict__ x, co
         for (int k = 0; k < nh; k++) xi -= (double)U[(int64_t)k * ld + i] * gs[k];
         xnew[i] = xi;
     }
-}
-
-// deterministic sum of per-block partials: out[j] = op_b part[b*stride + j]
-__global__ void part_reduce(const double *__restrict__ part, int nb, int stride, int nv, int max_first,
-                            double *__restrict__ out) {
-    int j = threadIdx.x;
-    if (j >= nv) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; b++) {
-        double v = part[(int64_t)b * stride + j];
-        s = (max_first && j == 0) ? fmax(s, v) : s + v;
-    }
-    out[j] = s;
 }
 
 // Cholesky solve of the nh x nh system (w0^2 I + dF^T dF) gamma = dF^T F, as dposv('U').
@@ -503,10 +501,8 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
         // max|F|, ||F||, ||F - Fold||
         const bool want_dn = its > 1 && nhist > 0;
         int pi = prof_begin(h, K_BROYDEN);
-        vec_norms<<<nb, RED_THREADS, 0, st>>>(d_F, want_dn ? d_Fold : nullptr, n, part);
+        vec_norms<<<nb, RED_THREADS, 0, st>>>(d_F, want_dn ? d_Fold : nullptr, n, part, h->d_rcnt, fin);
         prof_end(h, pi);
-        count_launch();
-        part_reduce<<<1, 32, 0, st>>>(part, nb, 3, 3, 1, fin);
         QS_CUDA(h, cudaGetLastError());
         QS_CUDA(h, cudaMemcpyAsync(hv.data(), fin, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
         QS_CUDA(h, cudaStreamSynchronize(st));
@@ -531,13 +527,11 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
             int pj = prof_begin(h, K_BROYDEN);
             if (sp)
                 launch_hist<float>(nb, st, d_F, d_Fold, d_x, d_xold, n, store ? fnorm : 1.0, alpha_mix, (float *)d_hdF,
-                                   (float *)d_hU, slot, nh_new, store, part);
+                                   (float *)d_hU, slot, nh_new, store, part, h->d_rcnt, fin);
             else
                 launch_hist<double>(nb, st, d_F, d_Fold, d_x, d_xold, n, store ? fnorm : 1.0, alpha_mix, (double *)d_hdF,
-                                    (double *)d_hU, slot, nh_new, store, part);
+                                    (double *)d_hU, slot, nh_new, store, part, h->d_rcnt, fin);
             prof_end(h, pj);
-            count_launch();
-            part_reduce<<<1, 2 * MAXH, 0, st>>>(part, nb, 2 * MAXH, 2 * nh_new, 0, fin);
             QS_CUDA(h, cudaGetLastError());
             QS_CUDA(h, cudaMemcpyAsync(hv.data(), fin, 2 * nh_new * sizeof(double), cudaMemcpyDeviceToHost, st));
             QS_CUDA(h, cudaStreamSynchronize(st));
@@ -583,10 +577,8 @@ int vec_maxabs(qs_handle *h, const double *d_v, int64_t n, double &mx) {
     const int nb = red_blocks(n);
     double *part = h->d_red, *fin = h->d_red + (size_t)RED_BLOCKS * 2 * MAXH;
     int pi = prof_begin(h, K_BROYDEN);
-    vec_norms<<<nb, RED_THREADS, 0, h->stream>>>(d_v, nullptr, n, part);
+    vec_norms<<<nb, RED_THREADS, 0, h->stream>>>(d_v, nullptr, n, part, h->d_rcnt, fin);
     prof_end(h, pi);
-    count_launch();
-    part_reduce<<<1, 32, 0, h->stream>>>(part, nb, 3, 3, 1, fin);
     QS_CUDA(h, cudaGetLastError());
     double hv[3];
     QS_CUDA(h, cudaMemcpyAsync(hv, fin, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));

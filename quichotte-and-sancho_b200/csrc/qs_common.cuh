@@ -205,6 +205,8 @@ struct qs_handle {
     qs::zc *d_Glt0 = nullptr;  // G^<(t=0) on-site blocks, 4 per site
     double *d_red = nullptr;   // reduction scratch
     size_t red_len = 0;
+    double *d_rpart = nullptr;  // partial sums of the reductions over energies, REDUCE_PART doubles
+    int *d_rcnt = nullptr;      // their arrival counters, REDUCE_CNT ints (zero between launches)
     int *d_info = nullptr;     // first singular energy (+1), 0 if none
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -244,6 +246,10 @@ namespace qs {
     } while (0)
 
 int dalloc(qs_handle *h, void **p, size_t bytes);
+// scratch of the reductions over energies: one partial per block for at most REDUCE_BLOCKS blocks
+// of 32 complex columns, a counter per group of blocks that share an output
+constexpr int REDUCE_BLOCKS = 592, REDUCE_PART = REDUCE_BLOCKS * 64, REDUCE_CNT = REDUCE_BLOCKS;
+int reduce_scratch(qs_handle *h);
 // The dynamic shared-memory cap of a kernel is a process-wide attribute: it is always set
 // to the device maximum (a cap, not a reservation), so that handles that size the same
 // kernel differently, on other threads, never lower it under each other's launches.
@@ -332,7 +338,9 @@ int equal_time_lesser_sigma1(qs_handle *h, const double *d_x);
 enum SweepMode { M_INIT2 = 1, M_SCF2 = 2, M_SCF1 = 3, M_FINAL = 4 };
 // fp32: the FP32 phase of a QS_PREC_MIXED solve (M_SCF2 only: tensor-core Keldysh products)
 int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const double *d_x, bool fp32 = false);
-int sum_over_energies(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out);
+// d_out[c] = sum over rows of d_A[r ld + c]; with d_B, its sums behind them at d_out[ncols + c]
+int sum_over_energies(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out,
+                      const zc *d_B = nullptr);
 int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncols, int64_t nrows, double *d_out);
 int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_info, zc *d_ws, int ws_slots);
 int invert_batched_ws(cudaStream_t st, int N, int batch, zc *d_A, int *d_min_info, int *d_info_each, zc *d_ws,

@@ -573,8 +573,7 @@ int sa_sweep(qsa_handle *h, double V, bool interacting, double *d_out, const dou
                                                 s3 ? h->d_S3L : nullptr, h->d_omega, V, h->mu, h->beta, h->d_T));
     SA_RUN(h, K_KELDYSH, sa_keldysh_pack<<<grid_for(tot), 256, 0, st>>>(Na, n, h->d_W, h->d_T, d_x, d_out, h->d_gRd, h->d_gLd));
     // check_gf_sanity sums
-    if ((rc = sum_over_energies(&h->q, h->d_gLd, Na, Na, n, h->d_sums))) return rc;
-    if ((rc = sum_over_energies(&h->q, h->d_gRd, Na, Na, n, h->d_sums + Na))) return rc;
+    if ((rc = sum_over_energies(&h->q, h->d_gLd, Na, Na, n, h->d_sums, h->d_gRd))) return rc;
     std::vector<zc> hs(2 * Na);
     QS_CUDA(&h->q, cudaMemcpyAsync(hs.data(), h->d_sums, sizeof(zc) * 2 * Na, cudaMemcpyDeviceToHost, st));
     QS_CUDA(&h->q, cudaStreamSynchronize(st));
@@ -660,7 +659,7 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         (rc = up((void **)&h->d_omega, p->omega, (size_t)n * 8)) ||
         (rc = dalloc(q, (void **)&q->d_x, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_F, n_vec * 8)) ||
         (rc = dalloc(q, (void **)&q->d_Fold, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_xold, n_vec * 8)) ||
-        (rc = dalloc(q, (void **)&q->d_red, q->red_len * 8)) ||
+        (rc = dalloc(q, (void **)&q->d_red, q->red_len * 8)) || (rc = reduce_scratch(q)) ||
         (h->nhist > 0 && ((rc = dalloc(q, &q->d_hdF, broyden_ld(n_vec) * 8 * h->nhist)) ||
                           (rc = dalloc(q, &q->d_hU, broyden_ld(n_vec) * 8 * h->nhist)))) ||
         (rc = dalloc(q, (void **)&h->d_Glt0, Na * zc_)) || (rc = dalloc(q, (void **)&h->d_W, tot * zc_)) ||

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "qs_common.cuh"
+#include "reduce.cuh"
 
 #include <atomic>
 
@@ -77,32 +78,37 @@ void release_all(qs_handle *h) {
 
 // G^<(t=0) on the on-site blocks of the active sites from the SCF vector, then Sigma1
 // (equal_time_lesser, src/green_functions.f90:192-213; sigma_first_order,
-// src/self_energies.f90:45-72). One block per active site.
-__global__ void glt0_sigma1(const double *__restrict__ x, int64_t nblk, int n, int nA, int N, const int *__restrict__ act,
-                            const double *__restrict__ U, double pp, zc *__restrict__ Glt0, zc *__restrict__ Sig1) {
-    __shared__ double sh[4][32];
-    const int I = blockIdx.x, io = 2 * I;
+// src/self_energies.f90:45-72). gridDim.y blocks of 256 energies a step share an active site; the
+// last to arrive adds their partials and forms Sigma1. (32 bytes of every energy's block are
+// read, so the bound is latency: many blocks keep many energies in flight.)
+__global__ void __launch_bounds__(256) glt0_sigma1(const double *__restrict__ x, int64_t nblk, int n, int N,
+                                                   const int *__restrict__ act, const double *__restrict__ U, double pp,
+                                                   zc *__restrict__ Glt0, zc *__restrict__ Sig1,
+                                                   double *__restrict__ part, int *__restrict__ cnt) {
+    __shared__ double sh[256], s[4];
+    const int I = blockIdx.x, io = 2 * I, RB = gridDim.y;
     double v[4] = {0, 0, 0, 0};
-    for (int w = threadIdx.x; w < n; w += blockDim.x) {
+    for (int w = blockIdx.y * 256 + threadIdx.x; w < n; w += 256 * RB) {
         const double *b = x + (int64_t)w * nblk + dl_block(I, I);
         v[0] += b[10];  // Im G^<_00, Im G^<_11, G^<_01 of the site's block
         v[1] += b[11];
         v[2] += b[8];
         v[3] += b[9];
     }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int k = 0; k < 4; k++) {
-        double t = v[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        if (lane == 0) sh[k][wid] = t;
+    for (int k = 0; k < 4; k++)
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 4; k++) sh[4 * (threadIdx.x >> 5) + k] = v[k];
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double t = 0.0;
+        for (int w = 0; w < 8; w++) t += sh[4 * w + threadIdx.x];
+        part[(I * RB + blockIdx.y) * 4 + threadIdx.x] = t;
     }
+    if (!last_block(cnt + I, RB)) return;
+    part_reduce(part + I * RB * 4, RB, 4, 4, false, sh, s);
     __syncthreads();
     if (threadIdx.x == 0) {
-        double s[4];
-        for (int k = 0; k < 4; k++) {
-            s[k] = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) s[k] += sh[k][w];
-        }
         zc g00{0.0, s[0] * pp}, g11{0.0, s[1] * pp}, g01{s[2] * pp, s[3] * pp};
         zc g10 = -conj(g01);
         Glt0[4 * I + 0] = g00;
@@ -123,8 +129,9 @@ __global__ void glt0_sigma1(const double *__restrict__ x, int64_t nblk, int n, i
 
 int equal_time_lesser_sigma1(qs_handle *h, const double *d_x) {
     int pi = prof_begin(h, K_REDUCE);
-    glt0_sigma1<<<h->nAs, 256, 0, h->stream>>>(d_x, h->nblk, h->n, h->nA, h->Norb, h->d_act, h->d_U,
-                                                h->delta / (2.0 * PI), h->d_Glt0, h->d_Sig1);
+    const int RB = std::max(1, std::min((h->n + 255) / 256, REDUCE_BLOCKS / std::max(h->nAs, 1)));
+    glt0_sigma1<<<dim3(h->nAs, RB), 256, 0, h->stream>>>(d_x, h->nblk, h->n, h->Norb, h->d_act, h->d_U,
+                                                         h->delta / (2.0 * PI), h->d_Glt0, h->d_Sig1, h->d_rpart, h->d_rcnt);
     prof_end(h, pi);
     QS_CUDA(h, cudaGetLastError());
     return 0;
@@ -211,8 +218,7 @@ int sweep_sanity_read(qs_handle *h, SanityOut &s) {
 int sweep_sanity(qs_handle *h, SanityOut &s) {
     zc *sums = (zc *)h->d_red;  // [nA] gLd sums, then [nA] gRd sums
     int rc;
-    if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, sums))) return rc;
-    if ((rc = sum_over_energies(h, h->d_gRd, h->nA, h->nA, h->n, sums + h->nA))) return rc;
+    if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, sums, h->d_gRd))) return rc;
     return sweep_sanity_read(h, s);
 }
 
@@ -309,8 +315,7 @@ int residual2_launches(qs_handle *h, double V, const double *d_x, double *d_F, b
     if ((rc = sigma2_compute(h, d_x, use32))) return rc;
     if ((rc = sweep(h, M_SCF2, V, true, d_F, d_x, use32))) return rc;
     zc *sums = (zc *)h->d_red;
-    if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, sums))) return rc;
-    if ((rc = sum_over_energies(h, h->d_gRd, h->nA, h->nA, h->n, sums + h->nA))) return rc;
+    if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, sums, h->d_gRd))) return rc;
     return 0;
 }
 
@@ -660,6 +665,7 @@ static size_t handle_need(const qs_handle *h) {
         const int64_t nv = std::max<int64_t>(h->n_vec, 1);
         if (h->order == 1) need += (size_t)nv * 8 * 4 + (size_t)broyden_ld(nv) * hist_el * 2 * h->nhist;
     }
+    need += (size_t)REDUCE_PART * 8 + REDUCE_CNT * 4;
     need += broyden_red_len() * 8 + (size_t)3 * h->nS * h->nS * zc_;        // reductions, Gamma blocks
     if (h->order == 2) {
         need += (size_t)sigma2_plan(n).Nf * zc_ + (size_t)3 * nA * nA * 4;    // twiddles, layout table
@@ -754,7 +760,7 @@ int qs_create(const qs_problem *p, qs_handle **out) {
         return rc;
     if (h->has_atomL && (rc = dalloc(h, (void **)&h->d_atomL, (size_t)n * h->atom_off.back() * zc_))) return rc;
     h->red_len = std::max<size_t>(broyden_red_len(), (size_t)2 * (4 * h->N_sites + h->atom_off.back() + 2 * N + 2 * nA + 8));
-    if ((rc = dalloc(h, (void **)&h->d_red, h->red_len * 8))) return rc;
+    if ((rc = dalloc(h, (void **)&h->d_red, h->red_len * 8)) || (rc = reduce_scratch(h))) return rc;
     if ((rc = dalloc(h, (void **)&h->d_info, sizeof(int) * 2))) return rc;
     int imax = INT_MAX;
     QS_CUDA(h, cudaMemcpyAsync(h->d_info, &imax, sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -1191,7 +1197,7 @@ int qs_broyden_solve_host(qs_residual_fn residual, void *ctx, double *x, int64_t
     h.red_len = broyden_red_len();
     if ((rc = dalloc(&h, (void **)&h.d_x, n * 8)) || (rc = dalloc(&h, (void **)&h.d_F, n * 8)) ||
         (rc = dalloc(&h, (void **)&h.d_Fold, n * 8)) || (rc = dalloc(&h, (void **)&h.d_xold, n * 8)) ||
-        (rc = dalloc(&h, (void **)&h.d_red, h.red_len * 8)) ||
+        (rc = dalloc(&h, (void **)&h.d_red, h.red_len * 8)) || (rc = reduce_scratch(&h)) ||
         (nhist > 0 && ((rc = dalloc(&h, &h.d_hdF, broyden_ld(n) * hist_el * nhist)) || (rc = dalloc(&h, &h.d_hU, broyden_ld(n) * hist_el * nhist))))) {
     } else {
         cudaMemcpyAsync(h.d_x, x, sizeof(double) * n, cudaMemcpyHostToDevice, h.stream);
