@@ -170,14 +170,10 @@ int qs_broyden_solve_host(qs_residual_fn residual, void *ctx, double *x, int64_t
  * pointers the caller owns: A holds `batch` N x N complex column-major matrices and is
  * replaced by their inverses; info[b] = 0, or k+1 for a zero pivot at step k. The work
  * runs asynchronously on `stream` (a cudaStream_t, NULL = legacy default stream); read info
- * after synchronising. The library allocates nothing: its workspace is a fixed 16 MiB
- * device array that every GPU loading the library holds until exit. Each call looks up
- * that array's address (cudaGetSymbolAddress) on the calling thread's current device; the
- * first call on a device may load the module there, so make it before any stream capture. All calls share the array, so
- * calls that overlap on the GPU (other streams or threads) race: serialise them. Limits:
- * 1 <= N <= 512 (else QS_ERR_NOALLOC_LIMIT, with a message on stderr). Returns 0 or a
- * CUDA error (< 0). */
-enum { QS_ERR_NOALLOC_LIMIT = -1001 };
+ * after synchronising. The library allocates nothing and keeps no scratch: calls on different
+ * matrices may overlap on the GPU. Limits: 1 <= N <= 512 (else QS_ERR_NOALLOC_LIMIT, with a
+ * message on stderr). Returns 0 or a CUDA error (< 0). */
+ enum { QS_ERR_NOALLOC_LIMIT = -1001 };
 int qs_invert_batched_noalloc(int N, int batch, double *A, int *info, void *stream);
 
 /* ---- memory (setup_storage's memory estimate, src/green_functions.f90:90-190) ---- */
@@ -226,9 +222,9 @@ void qs_server_destroy(qs_server *s);
 
 /* ---- autotuner (no counterpart in the reference) ----
  * Kernel variants whose relative speed depends on the size (kind 0: Dyson, blocked tensor-
- * core (variant 1: in shared memory, one block per SM, or in the global workspace above the
- * shared-memory limit; variant 3: in the global workspace, two blocks per SM) or unblocked
- * Gauss-Jordan (2); kind 1: Keldysh, tensor-core or CUDA-core GEMMs; kinds 2
+ * core Gauss-Jordan: variant 1 in shared memory up to order 120 (nothing else competes there), in
+ * the global workspace with one block per SM above it; variant 3 two blocks per SM; beyond order
+ * 256 the unblocked one (2); kind 1: Keldysh, tensor-core or CUDA-core GEMMs; kinds 2
  * and 3 (tiles of the Sigma2 kernels) are not decided any more; kind 4: the Keldysh step of a mixed solve's FP32 phase, variant 3 the
  * 3xTF32 kernel on the fifth-generation tensor cores, 1 / 2 the FP64 ones) are timed on the
  * first launch at a new size and the fastest is kept for the process.

@@ -50,6 +50,7 @@ int tune_launch(qs_handle *h, int kind, int size, const int *cand, int ncand, in
     const int mode = tune_mode();
     if (mode == 2 || mode == 3) return launch(cand[mode == 2 ? 0 : ncand - 1]);
     if (mode == 4) return launch(cand[ncand >= 3 ? 1 : 0]);
+    if (mode == 1 && ncand == 1) tune_put(kind, size, cand[0]);  // nothing to choose: recorded all the same
     if (ncand <= 1 || mode == 0) return launch(ncand == 1 ? cand[0] : fallback);
     const int known = tune_get(kind, size);
     if (known >= 0) return launch(known);

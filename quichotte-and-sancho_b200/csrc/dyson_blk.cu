@@ -1,0 +1,303 @@
+// dyson_blk.cu -- G^r(w) = [hbar w - H + (i/2hbar)(GammaL+GammaR) - Sigma^r(w)]^-1 for every energy, and
+// batched inversion (invert_complex, common/linear_algebra.f90:58-88): blocked in-place Gauss-Jordan
+// elimination with partial pivoting in shared memory, one matrix per warp (N <= 32) or block
+// (N <= 120).
+//
+// Panels of 8 columns K = [k0, k0 + 8), one column tile of the FP64 tensor cores:
+//   panel   PW = ceil(N / 32) warps hold one row of the panel per lane in registers. Per column every
+//           warp finds its best row (integer warp reductions on the bits of |Re| + |Im|) and
+//           publishes that row and its reciprocal; after one barrier every lane picks the best
+//           warp's and eliminates its own row
+//   update  every other column tile j by one warp, complex products of four real DMMAs:
+//           A[i, j] = (i a pivot row of the panel ? 0 : A[i, j]) + sum_t A[i, K_t] A[p_t, j],
+//           with the pivot rows A[p_t, j] read into registers first
+// Rows are never exchanged: a row is used once, as pivot row p_k of step k. With the pivot on
+// (p_k, k) elimination exchanges y_{p_k} and x_k, so that in the end row p_k holds row k of the
+// inverse and column k its column p_k; the output is written through that permutation. Elimination
+// is homogeneous in a row, so a pivot row is not divided by its pivot either: it keeps its values
+// (1 in column k) and gets the factor 1 / pivot on output.
+//
+// Bound: the panel's columns are a chain of about 500 cycles (search, row, barrier, 32 DFMA); the
+// update runs at the FP64 rate. Small matrices share an SM (20 of order 24, 5 of order 40), so
+// that panels and updates of different ones overlap.
+//
+// Measured on B200, batched inversion (8 N^3 flops a matrix), against the kernels this replaces
+// (row exchanges, 16-wide panels, one block a matrix, or everything through a global workspace):
+// N = 120 8.9 -> 12.9 TFLOP/s; as Dyson of 40 states x 5003 energies 0.99 -> 0.40 ms,
+// 24 x 32768 3.05 -> 0.61 ms, 48 x 4001 1.58 -> 0.38 ms. At N = 120 a matrix takes 300k cycles: the
+// panels 128k (1070 a column), the updates 141k (107k at the DMMA rate), load and output 30k.
+// Tried instead for N <= 96: the whole matrix in registers, rank-1 updates (4-9 TFLOP/s: the
+// per-step work of every warp, column and row exchange and selects, outweighs the update).
+#include <algorithm>
+#include <climits>
+
+#include "qs_common.cuh"
+
+namespace qs {
+namespace {
+
+constexpr int PB = 8;  // panel width
+
+// D = A B + D with A 16x8, B 8x8 in FP64: a_i = A(g + 8(i&1), t + 4(i>>1)), i < 4;
+// b_i = B(t + 4i, g), i < 2; c_i = C(g + 8(i>>1), 2t + (i&1)) (g = lane / 4, t = lane % 4)
+__device__ __forceinline__ void dmma1688(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// 1 / a without overflow or underflow of the intermediate |a|^2: a is scaled by the power of two
+// that brings its larger part to [1, 2)
+__device__ __forceinline__ zc scaled_recip(zc a) {
+    const unsigned h = max((unsigned)__double2hiint(a.x) & 0x7fffffffu, (unsigned)__double2hiint(a.y) & 0x7fffffffu) >> 20;
+    const double s = __hiloint2double((int)(min(max(2046 - (int)h, 1), 2046) << 20), 0);  // 2^(1023 - h)
+    const double x = a.x * s, y = a.y * s, d = s / fma(x, x, y * y);
+    return zc{x * d, -y * d};
+}
+
+// Position of element (i, j): column-major with the leading dimension padded to a multiple of 8 and
+// the row index XORed with j mod 8 (a warp's 16 x 8 fragments and its walks along a row or a column
+// then spread over the banks).
+__device__ __forceinline__ int at(int i, int j, int N) { return (i + j * ((N + 7) & ~7)) ^ (j & 7); }
+__host__ __device__ __forceinline__ int smem_units(int N) { return N * ((N + 7) & ~7); }
+
+template <int PW> struct Exchange {
+    zc row[2][PW][PB];  // each panel warp's candidate row; steps alternate between the two
+    zc inv[2][PW];
+    unsigned long long key[2][PW];
+    int idx[2][PW];
+    unsigned used[PW];      // rows (bits) that became pivot rows in this panel
+    int first_zero;         // 1 + the first step with a zero pivot (LAPACK's INFO), 0 if none
+    int pad;
+    unsigned char perm[32 * PW], step[32 * PW];  // pivot row of a step, step of a row
+};
+
+// PW panel warps, W warps a matrix, MPB matrices a block (more than one only for W = 1).
+template <int PW, int W, int MPB, int MINB>
+__global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
+    static_assert(MPB == 1 || W == 1, "several matrices a block: one warp each");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ Exchange<PW> exs[MPB];
+    const int N = a.N, nA = a.nA, slot = W == 1 ? threadIdx.x >> 5 : 0, tid = W == 1 ? threadIdx.x & 31 : threadIdx.x;
+    constexpr int nthr = 32 * W;
+    const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    Exchange<PW> &e = exs[slot];
+    zc *M = (zc *)smem_raw + (size_t)slot * smem_units(N);
+    const int mtiles = (N + 15) / 16, ntiles = (N + 7) / 8;
+    auto sync = [] {
+        if constexpr (W == 1) __syncwarp();
+        else __syncthreads();
+    };
+    auto panel_sync = [] {
+        if constexpr (W == 1) __syncwarp();
+        else if constexpr (PW == W) __syncthreads();
+        else if constexpr (PW == 1) __syncwarp();
+        else asm volatile("bar.sync 1, %0;\n" ::"n"(32 * PW) : "memory");
+    };
+    for (int iw = a.iw0 + blockIdx.x * MPB + slot; iw < a.iw1; iw += gridDim.x * MPB) {
+        if (a.Ain) {
+            const zc *A = a.Ain + (size_t)(iw - a.iw0) * N * N;
+#pragma unroll 4
+            for (int idx = tid; idx < N * N; idx += nthr) M[at(idx % N, idx / N, N)] = A[idx];
+        } else {
+            const double w = a.omega[iw];
+            const zc *SR = a.Sig + iw * a.sig_ld;
+#pragma unroll 4
+            for (int idx = tid; idx < N * N; idx += nthr) {
+                const int i = idx % N, j = idx / N;
+                zc v = a.Hemb[idx];
+                if (a.use_sigma) {
+                    const int pi = a.pos[i], pj = a.pos[j];
+                    if (pi >= 0 && pj >= 0) {
+                        zc sg = a.Sig1[idx];
+                        if (a.order2) sg = sg + sig_r(SR, pi, pj);
+                        v = v - sg;
+                    }
+                }
+                if (i == j) v.x += w;
+                M[at(i, j, N)] = v;
+            }
+        }
+        if (tid == 0) e.first_zero = 0;
+        const bool is_panel = warp < PW;
+        bool open = is_panel && tid < N;  // this lane's row is not used yet
+        zc scale{0, 0};                   // the factor it lacks since its step
+        sync();
+#pragma unroll 1
+        for (int k0 = 0; k0 < N; k0 += PB) {
+            if (is_panel) {
+                zc R[PB];
+#pragma unroll
+                for (int c = 0; c < PB; c++) R[c] = (tid < N && k0 + c < N) ? M[at(tid, k0 + c, N)] : zc{0, 0};
+                bool mine = false;
+#pragma unroll
+                for (int c = 0; c < PB; c++) {
+                    const int k = k0 + c, b = c & 1;
+                    if (k >= N) break;
+                    // |Re| + |Im| >= 0, so its bit pattern orders like its value (a NaN is a large key: a
+                    // row is always found); 0 marks a row that is used or beyond the matrix
+                    const unsigned long long key = open ? (unsigned long long)__double_as_longlong(cabs1(R[c])) + 1 : 0;
+                    const zc inv = scaled_recip(R[c]);  // in case this row is chosen
+                    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+                    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+                    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+                    const unsigned bal = __ballot_sync(0xffffffffu, hi == mh && lo == ml);
+                    if (lane == __ffs(bal) - 1) {  // the first maximum, as izamax
+#pragma unroll
+                        for (int j = 0; j < PB; j++)
+                            if (j != c) e.row[b][warp][j] = R[j];
+                        e.inv[b][warp] = inv;
+                        e.key[b][warp] = key;
+                        e.idx[b][warp] = tid;
+                    }
+                    panel_sync();
+                    int wb = 0;
+                    if constexpr (PW > 1) {
+                        unsigned long long bk = e.key[b][0];
+#pragma unroll
+                        for (int q = 1; q < PW; q++) {
+                            const unsigned long long ck = e.key[b][q];
+                            if (ck > bk) {
+                                bk = ck;
+                                wb = q;
+                            }
+                        }
+                    }
+                    const int p = e.idx[b][wb];
+                    zc pinv = e.inv[b][wb];
+                    // a pivot whose key is that of +0: singular from here on (every lane sees the same)
+                    const bool zero = e.key[b][wb] == 1;
+                    const int fz = e.first_zero;
+                    if (zero || (fz != 0 && fz <= k)) pinv = zc{0, 0};
+                    zc m = R[c] * pinv;
+                    const bool is = tid == p;
+                    R[c] = is ? zc{1, 0} : zc{0, 0};
+                    if (is) {
+                        open = false;
+                        mine = true;
+                        scale = pinv;
+                        m = zc{0, 0};
+                        e.perm[k] = (unsigned char)p;
+                        e.step[p] = (unsigned char)k;
+                        if (zero && fz == 0) e.first_zero = k + 1;
+                    }
+#pragma unroll
+                    for (int j = 0; j < PB; j++) {
+                        const zc r = j == c ? zc{1, 0} : e.row[b][wb][j];
+                        if (j == c) {
+                            R[j] = R[j] - m;
+                        } else {
+                            R[j].x = fma(-m.x, r.x, R[j].x);
+                            R[j].y = fma(-m.x, r.y, R[j].y);
+                            R[j].x = fma(m.y, r.y, R[j].x);
+                            R[j].y = fma(-m.y, r.x, R[j].y);
+                        }
+                    }
+                }
+                if (tid < N)
+#pragma unroll
+                    for (int c = 0; c < PB; c++)
+                        if (k0 + c < N) M[at(tid, k0 + c, N)] = R[c];
+                const unsigned u = __ballot_sync(0xffffffffu, mine);
+                if (lane == 0) e.used[warp] = u;
+            }
+            sync();
+            const int kb = min(PB, N - k0);
+            for (int ct = warp; ct < ntiles; ct += W) {
+                if (ct == k0 / PB) continue;
+                const int j0 = 8 * ct;
+                double br[2], bi[2], nbi[2];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int t = t4 + 4 * q;
+                    const zc v = (t < kb && j0 + g < N) ? M[at(e.perm[k0 + t], j0 + g, N)] : zc{0, 0};
+                    br[q] = v.x;
+                    bi[q] = v.y;
+                    nbi[q] = -v.y;
+                }
+                __syncwarp();  // the fragments are read before other lanes of this warp rewrite the pivot rows
+#pragma unroll 2
+                for (int rt = 0; rt < mtiles; rt++) {
+                    const int i0 = 16 * rt;
+                    const unsigned um = e.used[i0 >> 5] >> (i0 & 31);  // pivot rows of this tile
+                    double ar[4], ai[4], cr[4], ci[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int r = i0 + g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
+                        const zc v = (r < N && c < kb) ? M[at(r, k0 + c, N)] : zc{0, 0};
+                        ar[q] = v.x;
+                        ai[q] = v.y;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int dr = g + 8 * (q >> 1), r = i0 + dr, c = j0 + 2 * t4 + (q & 1);
+                        const zc v = (r < N && c < N && !((um >> dr) & 1)) ? M[at(r, c, N)] : zc{0, 0};
+                        cr[q] = v.x;
+                        ci[q] = v.y;
+                    }
+                    dmma1688(cr, ar, br);
+                    dmma1688(ci, ar, bi);
+                    dmma1688(cr, ai, nbi);
+                    dmma1688(ci, ai, br);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
+                        if (r < N && c < N) M[at(r, c, N)] = zc{cr[q], ci[q]};
+                    }
+                }
+            }
+            sync();
+        }
+        if (e.first_zero && tid == 0) {
+            if (a.info) atomicMin(a.info, iw + 1);
+            if (a.info_each) a.info_each[iw - a.iw0] = e.first_zero;
+        }
+        // scale the rows in place (their lanes know the factors), then write through the permutation
+        if (is_panel && tid < N)
+            for (int j = 0; j < N; j++) {
+                const int o = at(tid, j, N);
+                M[o] = M[o] * scale;
+            }
+        sync();
+        const int nout = a.out_mode == 0 ? nA : N;
+        zc *G = a.Gout + (a.out_mode == 0 ? (size_t)iw * nA * nA : (size_t)(iw - a.iw0) * N * N);
+#pragma unroll 4
+        for (int idx = tid; idx < nout * nout; idx += nthr) {
+            int k = idx % nout, c = idx / nout;
+            if (a.out_mode == 0) {
+                k = a.act[k];
+                c = a.act[c];
+            }
+            G[idx] = M[at(e.perm[k], e.step[c], N)];
+        }
+        sync();
+    }
+}
+
+template <int PW, int W, int MPB, int MINB> int run(cudaStream_t st, const DysonArgs &a) {
+    const void *fn = (const void *)dyson_blk<PW, W, MPB, MINB>;
+    const size_t sm = sizeof(zc) * smem_units(a.N) * MPB;
+    if (sm > 40 << 10) {
+        const cudaError_t e = smem_cap(fn);
+        if (e != cudaSuccess) return -(int)e;
+    }
+    const int need = (a.iw1 - a.iw0 + MPB - 1) / MPB;
+    dyson_blk<PW, W, MPB, MINB><<<std::min(need, 148 * 16), 32 * W * MPB, sm, st>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : -(int)e;
+}
+
+}  // namespace
+
+int launch_dyson_blk(cudaStream_t st, const DysonArgs &a) {
+    // warps: enough for the column tiles of an update in one or two rounds, few enough that several
+    // blocks share an SM as long as their matrices fit
+    const int N = a.N;
+    if (N <= 32) return run<1, 1, 4, 5>(st, a);
+    if (N <= 64) return run<2, 4, 1, 5>(st, a);
+    if (N <= 80) return run<3, 8, 1, 2>(st, a);
+    if (N <= 96) return run<3, 11, 1, 1>(st, a);
+    return run<4, 15, 1, 1>(st, a);
+}
+
+}  // namespace qs

@@ -126,9 +126,10 @@ __device__ __forceinline__ void zmma16816(double (&cr)[4], double (&ci)[4], cons
 constexpr double PI = 3.14159265358979323846;
 constexpr int SMEM_MAX = 232448;  // max dynamic shared memory per block on sm_100 (227 KB)
 
-// The Gauss-Jordan kernel keeps the N x N complex matrix in shared memory when it fits
-// next to its ~1.3 KB of static shared memory (N <= 120 in FP64).
-inline bool dyson_fits_smem(int N) { return (size_t)N * N * 16 + 1536 <= (size_t)SMEM_MAX; }
+// The Gauss-Jordan kernel keeps the N x N complex matrix in shared memory when it fits next to its
+// 1.5 KB of static shared memory.
+constexpr int DYSON_SMEM_MAXN = 120;
+inline bool dyson_fits_smem(int N) { return N <= DYSON_SMEM_MAXN; }
 
 // the four-step split of the padded length Nf = N1 * N2 (>= 2 n - 1)
 struct FftPlan {
@@ -198,7 +199,7 @@ struct qs_handle {
     size_t G_chunk = 0;     // energies per chunk in full-G mode
     qs::zc *d_T = nullptr;  // per-CTA GEMM scratch
     size_t T_slots = 0, T_bytes = 0;
-    qs::zc *d_Gws = nullptr;  // Gauss-Jordan workspace when N x N does not fit in shared memory
+    qs::zc *d_Gws = nullptr;  // Gauss-Jordan workspace for orders above the shared-memory limit when nA < N
     size_t ws_slots = 0;
     qs::zc *d_gRd = nullptr, *d_gLd = nullptr, *d_onsL = nullptr, *d_atomL = nullptr;
     double *d_dosd = nullptr, *d_trU = nullptr, *d_trD = nullptr;
@@ -274,6 +275,26 @@ __device__ __forceinline__ double fermi_d(double w, double V, double mu, double 
     return 1.0 / (exp(fmin(arg, 700.0)) + 1.0);
 }
 
+// arguments of the Gauss-Jordan kernels
+struct DysonArgs {
+    int N, nA, iw0, iw1;
+    const zc *Hemb, *Sig1, *Sig;
+    int64_t sig_ld;
+    const int *pos;  // full index -> active index, -1 if inactive
+    const int *act;
+    const double *omega;
+    int use_sigma, order2;
+    int out_mode;  // 0: G_AA for energy iw at Gout[iw*nA^2]; 1: full G at Gout[(iw-iw0)*N^2]
+    zc *Gout;
+    zc *ws;        // global workspace (N^2 per block) when the matrix is not in shared memory
+    int *info;     // min over energies of (iw + 1) with a zero pivot; INT_MAX if none
+    const zc *Ain; // batched-inversion mode: matrices to invert (nullptr for the sweep)
+    int *info_each;
+    int inplace;   // kernels whose matrix is in global memory: in Gout itself (N x N each) instead of ws
+};
+// the blocked elimination in shared memory (dyson_blk.cu), N <= DYSON_SMEM_MAXN; 0 or a CUDA error (< 0)
+int launch_dyson_blk(cudaStream_t st, const DysonArgs &a);
+
 // arguments of the Keldysh kernels (sweep modes M_INIT2 / M_SCF2)
 struct KeldyshArgs {
     int nA, n;
@@ -315,8 +336,8 @@ int sigma2_compute(qs_handle *h, const double *d_x, bool fp32 = false);
 // TUNE_KELDYSH32: the Keldysh step of a mixed solve's FP32 phase, where the 3xTF32 tensor-core
 // kernel (keldysh_tf32.cu) competes with the two FP64 ones
 enum TuneKind { TUNE_DYSON = 0, TUNE_KELDYSH = 1, TUNE_KELDYSH32 = 4 };
-// DYSON_BLOCKED2: the blocked Gauss-Jordan with its matrix in the global workspace, two
-// 8-warp blocks per SM
+// DYSON_BLOCKED: in shared memory up to DYSON_SMEM_MAXN, above in the global workspace, one block
+// per SM; DYSON_BLOCKED2: in the workspace, two 8-warp blocks per SM
 enum { DYSON_BLOCKED = 1, DYSON_UNBLOCKED = 2, DYSON_BLOCKED2 = 3, KELDYSH_TC = 1, KELDYSH_CUDA = 2, KELDYSH_TF32 = 3 };
 // the size key of a decision: the matrix order and the octave of the grid length (how many
 // energies each SM gets changes which variant wins)
@@ -342,9 +363,9 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
 int sum_over_energies(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out,
                       const zc *d_B = nullptr);
 int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncols, int64_t nrows, double *d_out);
-int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_info, zc *d_ws, int ws_slots);
-int invert_batched_ws(cudaStream_t st, int N, int batch, zc *d_A, int *d_min_info, int *d_info_each, zc *d_ws,
-                      int ws_slots);
+// batch N x N column-major matrices inverted in place; d_min (or nullptr) receives the smallest
+// 1 + b of a singular one, d_each[b] 1 + the step of its first zero pivot
+int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each);
 int convert_ref_to_dl(qs_handle *h, const double *ref, double *dl);
 int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref);
 

@@ -76,8 +76,6 @@ struct qsa_handle {
     zc *d_S2R = nullptr, *d_S2L = nullptr, *d_S3R = nullptr, *d_S3L = nullptr;  // [e + k Na^2]
     zc *d_Glt0 = nullptr;
     zc *d_W = nullptr, *d_T = nullptr;  // Dyson batch (-> G^r out), G^r Sigma^< products
-    zc *d_ws = nullptr;
-    int ws_slots = 0;
     zc *d_gRd = nullptr, *d_gLd = nullptr;  // [k*Na + i]
     double *d_spec = nullptr;
     zc *d_sums = nullptr;
@@ -562,7 +560,7 @@ int sa_sweep(qsa_handle *h, double V, bool interacting, double *d_out, const dou
                                                   s2 ? h->d_S2R : nullptr, s3 ? h->d_S3R : nullptr, h->d_U, h->d_Glt0,
                                                   h->d_W));
     const int pi = prof_begin(&h->q, K_DYSON, false);  // the inversion counts its own launch
-    int rc = invert_batched_dev(st, Na, n, h->d_W, h->d_info, h->d_ws, h->ws_slots);
+    int rc = invert_batched_dev(st, Na, n, h->d_W, h->d_info, h->d_info + 1);
     prof_end(&h->q, pi);
     if (rc) {
         h->q.err = "batched Dyson inversion failed to launch";
@@ -681,10 +679,6 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         for (int k = 0; k < 3 && !rc; k++) rc = dalloc(q, (void **)&h->d_P[k], tm * zc_);
         if (!rc) rc = dalloc(q, (void **)&h->d_S3R, tot * zc_);
         if (!rc) rc = dalloc(q, (void **)&h->d_S3L, tot * zc_);
-    }
-    if (!rc && !dyson_fits_smem(Na)) {
-        h->ws_slots = std::min(n, 148 * 2);
-        rc = dalloc(q, (void **)&h->d_ws, (size_t)h->ws_slots * nf * zc_);
     }
     if (!rc) {
         const int v = INT_MAX;

@@ -652,7 +652,7 @@ static size_t handle_need(const qs_handle *h) {
     need += (size_t)n * (4 * h->N_sites * zc_ + N * 8 + 16);                // onsL, dosd, trU, trD
     if (h->has_atomL) need += (size_t)n * h->atom_off.back() * zc_;
     need += (size_t)n * std::max(nA, 1) * zc_ * 2;                           // gRd, gLd
-    if (!dyson_fits_smem(N) || (N > 16 && N <= 256)) need += (size_t)148 * 2 * nn * zc_;  // Gauss-Jordan workspace
+    if (!dyson_fits_smem(N) && nA != N) need += (size_t)148 * 2 * nn * zc_;  // Gauss-Jordan workspace
     if (h->order == 2) {
         need += (size_t)h->n_vec * 8 * 4;                                     // x, F, Fold, xold
         need += (size_t)broyden_ld(h->n_vec) * hist_el * 2 * h->nhist;                    // history
@@ -764,9 +764,9 @@ int qs_create(const qs_problem *p, qs_handle **out) {
     if ((rc = dalloc(h, (void **)&h->d_info, sizeof(int) * 2))) return rc;
     int imax = INT_MAX;
     QS_CUDA(h, cudaMemcpyAsync(h->d_info, &imax, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    // Gauss-Jordan workspace: for matrices that do not fit in shared memory, and for the
-    // two-blocks-per-SM blocked variant (16 < N <= 256)
-    if (!dyson_fits_smem(N) || (N > 16 && N <= 256)) {
+    // Gauss-Jordan workspace: for matrices that neither fit in shared memory nor can be inverted in
+    // the place of G_AA
+    if (!dyson_fits_smem(N) && nA != N) {
         h->ws_slots = 148 * 2;
         if ((rc = dalloc(h, (void **)&h->d_Gws, h->ws_slots * nn * zc_))) return rc;
     }
@@ -1047,27 +1047,18 @@ int qs_invert_batched(int N, int batch, double *A, int *info, int precision) {
     if (N < 1 || N > 512 || batch < 0) return -1;
     if (precision != QS_PREC_FP64) return -1;
     if (batch == 0) return 0;
-    zc *dA = nullptr, *ws = nullptr;
+    zc *dA = nullptr;
     int *dinfo = nullptr;
     size_t bytes = sizeof(zc) * (size_t)N * N * batch;
     cudaError_t e;
     if ((e = cudaMalloc(&dA, bytes)) != cudaSuccess) return simple_fail("malloc", e);
     if ((e = cudaMalloc(&dinfo, sizeof(int) * (batch + 1))) != cudaSuccess) { cudaFree(dA); return simple_fail("malloc", e); }
-    int ws_slots = 0;
-    if (!dyson_fits_smem(N)) {
-        ws_slots = std::min(batch, 148 * 2);
-        if ((e = cudaMalloc(&ws, sizeof(zc) * (size_t)N * N * ws_slots)) != cudaSuccess) {
-            cudaFree(dA);
-            cudaFree(dinfo);
-            return simple_fail("malloc", e);
-        }
-    }
     int rc = 0;
     std::vector<int> hinfo(batch + 1, 0);
     hinfo[0] = INT_MAX;
     cudaMemcpy(dA, A, bytes, cudaMemcpyHostToDevice);
     cudaMemcpy(dinfo, hinfo.data(), sizeof(int) * (batch + 1), cudaMemcpyHostToDevice);
-    rc = invert_batched_dev(0, N, batch, dA, dinfo, ws, ws_slots);
+    rc = invert_batched_dev(0, N, batch, dA, dinfo, dinfo + 1);
     if (rc == 0) {
         e = cudaMemcpy(A, dA, bytes, cudaMemcpyDeviceToHost);
         if (e == cudaSuccess) e = cudaMemcpy(hinfo.data(), dinfo, sizeof(int) * (batch + 1), cudaMemcpyDeviceToHost);
@@ -1077,7 +1068,6 @@ int qs_invert_batched(int N, int batch, double *A, int *info, int precision) {
         for (int b = 0; b < batch; b++) info[b] = hinfo[b + 1];
     cudaFree(dA);
     cudaFree(dinfo);
-    if (ws) cudaFree(ws);
     if (rc == 0 && hinfo[0] != INT_MAX) rc = 1;
     return rc;
 }

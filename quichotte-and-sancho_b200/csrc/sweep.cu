@@ -1,10 +1,10 @@
 // sweep.cu -- the energy sweep (sweep / G_at_energy, src/scf.f90:280-415) as batched
 // kernels over the whole energy grid:
-//   dyson_gj        G^r(w) = [hbar w - H + (i/2hbar)(GammaL+GammaR) - Sigma^r(w)]^-1 by
-//                   in-place Gauss-Jordan elimination with partial pivoting, one thread
-//                   block per energy, the matrix staged in shared memory (global
-//                   workspace when N^2 complex does not fit), pivot search by warp
-//                   shuffles (invert_complex, common/linear_algebra.f90:58-88)
+//   dyson_bgj,      G^r(w) = [hbar w - H + (i/2hbar)(GammaL+GammaR) - Sigma^r(w)]^-1 by
+//   dyson_gj        in-place Gauss-Jordan elimination with partial pivoting for the orders
+//                   that do not fit in shared memory, one block per energy with the matrix in a
+//                   global workspace (invert_complex, common/linear_algebra.f90:58-88);
+//                   dyson_blk.cu has the smaller ones
 //   keldysh_scf2    G^< = G^r Sigma^< G^a on the active block as two complex GEMMs per
 //                   energy, written straight into the SCF vector with its diagonals
 //                   (modes M_INIT2 / M_SCF2, src/scf.f90:340-355)
@@ -37,27 +37,8 @@ __device__ __forceinline__ void warp_argmax(double &v, int &i) {
     }
 }
 
-struct DysonArgs {
-    int N, nA, iw0, iw1;
-    const zc *Hemb, *Sig1, *Sig;
-    int64_t sig_ld;
-    const int *pos;  // full index -> active index, -1 if inactive
-    const int *act;
-    const double *omega;
-    int use_sigma, order2;
-    int out_mode;  // 0: G_AA for energy iw at Gout[iw*nA^2]; 1: full G at Gout[(iw-iw0)*N^2]
-    zc *Gout;
-    zc *ws;        // global workspace (N^2 per block) when the matrix is not in shared memory
-    int *info;     // min over energies of (iw + 1) with a zero pivot; INT_MAX if none
-    const zc *Ain; // batched-inversion mode: matrices to invert (nullptr for the sweep)
-    int *info_each;
-};
-
 __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = a.N;
-    const bool in_smem = (a.ws == nullptr);
-    zc *M = in_smem ? (zc *)smem_raw : a.ws + (size_t)blockIdx.x * N * N;
     __shared__ unsigned short perm[512];
     __shared__ double wv[16];
     __shared__ int wi[16];
@@ -68,8 +49,10 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
     const bool upd = mygrp < NG;
 
     for (int iw = a.iw0 + blockIdx.x; iw < a.iw1; iw += gridDim.x) {
+        zc *M = a.inplace ? a.Gout + (size_t)(iw - a.iw0) * N * N : a.ws + (size_t)blockIdx.x * N * N;
         // ---- build w1 = Hemb - (Sig1 + Sigma2^r(w)) on act x act, + hbar w on the diagonal
-        if (a.Ain) {
+        if (a.Ain && a.inplace) {  // the matrix is there
+        } else if (a.Ain) {
             const zc *A = a.Ain + (size_t)(iw - a.iw0) * N * N;
             for (int idx = tid; idx < N * N; idx += nthr) M[idx] = A[idx];
         } else {
@@ -164,11 +147,12 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
         }
         __syncthreads();
         if (singular && tid == 0) {
-            atomicMin(a.info, iw + 1);
+            if (a.info) atomicMin(a.info, iw + 1);
             if (a.info_each) a.info_each[iw - a.iw0] = first_zero;
         }
         // ---- output
-        if (a.out_mode == 0) {
+        if (a.inplace) {
+        } else if (a.out_mode == 0) {
             const int nA = a.nA;
             zc *G = a.Gout + (size_t)iw * nA * nA;
             for (int idx = tid; idx < nA * nA; idx += nthr) {
@@ -183,25 +167,7 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
     }
 }
 
-// ---------------------------------------------------------------------------------
-// Blocked Gauss-Jordan (panel width GJ_B) for matrices held in shared memory. For every
-// panel K = [k0, k0+b): warp 0 factors the N x b panel (pivot search by shuffles, full-row
-// interchanges, scaling and elimination restricted to the panel columns); then the whole
-// block applies the panel's transformation to the other columns as one rank-b update,
-//   A[i, j] += sum_t A[i, K_t] A[K_t, j]            (i, j outside K; register tiles 4 x 4)
-//   A[K, j]  = A[K, K] A[K, j]                       (the pivot rows, one column per thread)
-// which equals the unblocked elimination (row interchanges commute with the deferred update
-// because they act on whole rows). Interchanges are undone on the columns at the end.
-// ---------------------------------------------------------------------------------
-constexpr int GJ_B = 16;  // panel width = the k extent of one FP64 tensor-core MMA
-
-// shared-memory position of element (i, j): column-major with the leading dimension padded
-// to a multiple of 8 units (16 B each) and the unit index XORed with (j mod 8), so that a
-// warp walking along a row (fixed i, consecutive j) hits all banks; columns start on
-// 128-byte boundaries, so the XOR stays inside the column and the map is one-to-one
-__host__ __device__ __forceinline__ int swz_ld(int N) { return ((N + 7) / 8) * 8; }
-__device__ __forceinline__ int swz(int i, int j, int N) { return (i + j * swz_ld(N)) ^ (j & 7); }
-__host__ __device__ __forceinline__ int swz_units(int N) { return N * swz_ld(N); }
+constexpr int GJ_B = 16;  // panel width of dyson_bgj = the k extent of one FP64 tensor-core MMA
 
 // 15 warps: one per 8-column tile of a 120-column matrix in the update, and 136 registers a
 // thread for the panel's register-resident rows
@@ -210,32 +176,13 @@ constexpr int BGJ_THREADS = 480;
 // named barrier of the panel warps (ids 1.. are free; 0 is __syncthreads)
 __device__ __forceinline__ void panel_bar(int nthreads) { asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory"); }
 
-// argmax over a warp with the result in every lane (first maximum wins)
-__device__ __forceinline__ void warp_argmax_all(double &v, int &i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        if (v2 > v || (v2 == v && i2 < i)) {
-            v = v2;
-            i = i2;
-        }
-    }
-}
-
-// Storage of the matrix of the blocked Gauss-Jordan: GM = false, the swizzled shared-memory
-// layout above (16 <= N <= 120 in FP64); GM = true, column-major in the block's slot of a
-// global workspace (120 < N <= 256: the working set of the concurrent blocks stays largely in
-// L2, and every access of the update is a 128-byte run of 8 consecutive rows).
-template <bool GM> __device__ __forceinline__ int bix(int i, int j, int N) { return GM ? i + j * N : swz(i, j, N); }
-// panel warps: one thread per row
-template <bool GM> __host__ __device__ __forceinline__ int bgj_pw(int N) { return GM ? (N + 31) / 32 : 4; }
 constexpr int BGJ_MAXN_GM = 256;
 
-// Blocked Gauss-Jordan inversion with the matrix in (swizzled) shared memory (GM = false,
-// 16 <= N <= 120) or in a global workspace (GM = true, 120 < N <= 256). Per panel
+// Blocked Gauss-Jordan inversion of orders 121..256 with the matrix column-major in the block's slot
+// of a global workspace (the working set of the concurrent blocks stays largely in L2, and every
+// access of the update is a 128-byte run of 8 consecutive rows). Per panel
 // K = [k0, k0 + 16):
-//   panel   the panel warps (4, or ceil(N/32) <= 8), thread i holding row i of the panel
+//   panel   the panel warps (ceil(N/32) <= 8), thread i holding row i of the panel
 //           columns in registers: per column
 //           k the pivot search, the exchange of rows k and p (the panel part through shared
 //           memory, the rest of the two rows in place), and the elimination restricted to
@@ -245,17 +192,13 @@ constexpr int BGJ_MAXN_GM = 256;
 //           tensor cores; the warp reads its A[K, j] fragment before it rewrites those rows,
 //           so no block barrier separates the two
 // The row interchanges are undone by column interchanges in reverse order at the end.
-// NT = 480 (15 warps, one block per SM) or, with the matrix in the global workspace, NT = 256
-// (8 warps, two blocks per SM: one block's latency-bound panel overlaps the other's update).
-template <bool GM, int NT = BGJ_THREADS>
+// NT = 480 (15 warps, one block per SM) or NT = 256 (8 warps, two blocks per SM: one block's
+// latency-bound panel overlaps the other's update).
+template <int NT>
 __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PWM = GM ? 8 : 4;  // panel warps at most
+    constexpr int PWM = 8;  // panel warps at most
     const int N = a.N;
-    zc *M = GM ? a.ws + (size_t)blockIdx.x * N * N : (zc *)smem_raw;
-    // static shared memory of the shared-memory form stays below 1536 bytes (use_blocked):
-    // N = 120 takes the rest
-    __shared__ unsigned char perm[GM ? BGJ_MAXN_GM : 128];
+    __shared__ unsigned char perm[BGJ_MAXN_GM];
     __shared__ unsigned long long cand_k[PWM];  // each panel warp's pivot key (0: no row searched)
     __shared__ int cand_i[PWM];
     __shared__ zc cand_row[PWM][GJ_B];  // each panel warp's pivot candidate row (panel part)
@@ -264,12 +207,14 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int g = lane >> 2, t4 = lane & 3;
     const int mtiles = (N + 15) / 16, ntiles = (N + 7) / 8;
-    const int npw = bgj_pw<GM>(N);  // panel warps
+    const int npw = (N + 31) / 32;  // panel warps
 
     for (int iw = a.iw0 + blockIdx.x; iw < a.iw1; iw += gridDim.x) {
-        if (a.Ain) {
+        zc *M = a.inplace ? a.Gout + (size_t)(iw - a.iw0) * N * N : a.ws + (size_t)blockIdx.x * N * N;
+        if (a.Ain && a.inplace) {  // the matrix is there
+        } else if (a.Ain) {
             const zc *A = a.Ain + (size_t)(iw - a.iw0) * N * N;
-            for (int idx = tid; idx < N * N; idx += nthr) M[bix<GM>(idx % N, idx / N, N)] = A[idx];
+            for (int idx = tid; idx < N * N; idx += nthr) M[idx] = A[idx];
         } else {
             const double w = a.omega[iw];
             const zc *SR = a.Sig + iw * a.sig_ld;
@@ -286,7 +231,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
                     }
                 }
                 if (i == j) v.x += w;
-                M[bix<GM>(i, j, N)] = v;
+                M[i + j * N] = v;
             }
         }
         if (tid == 0) first_zero_s = 0;
@@ -301,7 +246,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
                 // R[0] and the step loop need not be unrolled (padding columns stay zero)
                 zc R[GJ_B];
 #pragma unroll
-                for (int c = 0; c < GJ_B; c++) R[c] = (i < N && c < kb) ? M[bix<GM>(i, k0 + c, N)] : zc{0, 0};
+                for (int c = 0; c < GJ_B; c++) R[c] = (i < N && c < kb) ? M[i + (k0 + c) * N] : zc{0, 0};
 #pragma unroll 1
                 for (int c = 0; c < kb; c++) {
                     const int k = k0 + c;
@@ -388,9 +333,9 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
                     // the rest of rows k and p (thread i moves column i, its own earlier
                     // exchanges first)
                     if (p != k && i < N && (i < k0 || i >= k0 + kb)) {
-                        zc tt = M[bix<GM>(k, i, N)];
-                        M[bix<GM>(k, i, N)] = M[bix<GM>(p, i, N)];
-                        M[bix<GM>(p, i, N)] = tt;
+                        zc tt = M[k + i * N];
+                        M[k + i * N] = M[p + i * N];
+                        M[p + i * N] = tt;
                     }
                     panel_bar(32 * npw);  // cand_row and krow are rewritten by the next column
                 }
@@ -399,7 +344,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                     for (int j = 0; j < GJ_B; j++) {
                         const int c = (kb + j) & (GJ_B - 1);
-                        if (c < kb) M[bix<GM>(i, k0 + c, N)] = R[j];
+                        if (c < kb) M[i + (k0 + c) * N] = R[j];
                     }
                 }
             }
@@ -412,7 +357,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int kr = t4 + 4 * q, c = j0 + g;
-                    zc v = (kr < kb && c < N) ? M[bix<GM>(k0 + kr, c, N)] : zc{0, 0};
+                    zc v = (kr < kb && c < N) ? M[k0 + kr + c * N] : zc{0, 0};
                     br[q] = v.x;
                     bi[q] = v.y;
                 }
@@ -424,7 +369,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
                         const int r = i0 + g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
-                        zc v = (r < N && c < kb) ? M[bix<GM>(r, k0 + c, N)] : zc{0, 0};
+                        zc v = (r < N && c < kb) ? M[r + (k0 + c) * N] : zc{0, 0};
                         ar[q] = v.x;
                         ai[q] = v.y;
                     }
@@ -433,7 +378,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
                     for (int q = 0; q < 4; q++) {
                         const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
                         own[q] = r < N && c < N && (r < k0 || r >= k0 + kb) && (c < k0 || c >= k0 + kb);
-                        zc v = own[q] ? M[bix<GM>(r, c, N)] : zc{0, 0};
+                        zc v = own[q] ? M[r + c * N] : zc{0, 0};
                         cr[q] = v.x;
                         ci[q] = v.y;
                     }
@@ -441,7 +386,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                        if (own[q]) M[bix<GM>(r, c, N)] = zc{cr[q], ci[q]};
+                        if (own[q]) M[r + c * N] = zc{cr[q], ci[q]};
                     }
                 }
                 // the pivot rows
@@ -449,7 +394,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     const int r = g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
-                    zc v = (r < kb && c < kb) ? M[bix<GM>(k0 + r, k0 + c, N)] : zc{0, 0};
+                    zc v = (r < kb && c < kb) ? M[k0 + r + (k0 + c) * N] : zc{0, 0};
                     ar[q] = v.x;
                     ai[q] = v.y;
                 }
@@ -457,7 +402,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int r = g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                    if (r < kb && c < N && (c < k0 || c >= k0 + kb)) M[bix<GM>(k0 + r, c, N)] = zc{cr[q], ci[q]};
+                    if (r < kb && c < N && (c < k0 || c >= k0 + kb)) M[k0 + r + c * N] = zc{cr[q], ci[q]};
                 }
             }
             __syncthreads();
@@ -467,27 +412,28 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a
             for (int k = N - 1; k >= 0; k--) {
                 int p = perm[k];
                 if (p != k) {
-                    zc tt = M[bix<GM>(tid, k, N)];
-                    M[bix<GM>(tid, k, N)] = M[bix<GM>(tid, p, N)];
-                    M[bix<GM>(tid, p, N)] = tt;
+                    zc tt = M[tid + k * N];
+                    M[tid + k * N] = M[tid + p * N];
+                    M[tid + p * N] = tt;
                 }
             }
         }
         __syncthreads();
         if (first_zero_s && tid == 0) {
-            atomicMin(a.info, iw + 1);
+            if (a.info) atomicMin(a.info, iw + 1);
             if (a.info_each) a.info_each[iw - a.iw0] = first_zero_s;
         }
-        if (a.out_mode == 0) {
+        if (a.inplace) {
+        } else if (a.out_mode == 0) {
             const int nA = a.nA;
             zc *G = a.Gout + (size_t)iw * nA * nA;
             for (int idx = tid; idx < nA * nA; idx += nthr) {
                 int p = idx % nA, q = idx / nA;
-                G[idx] = M[bix<GM>(a.act[p], a.act[q], N)];
+                G[idx] = M[a.act[p] + a.act[q] * N];
             }
         } else {
             zc *G = a.Gout + (size_t)(iw - a.iw0) * N * N;
-            for (int idx = tid; idx < N * N; idx += nthr) G[idx] = M[bix<GM>(idx % N, idx / N, N)];
+            for (int idx = tid; idx < N * N; idx += nthr) G[idx] = M[idx];
         }
         __syncthreads();
     }
@@ -1116,132 +1062,53 @@ int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref) {
 // ---------------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------------
-static int dyson_threads(int N) { return N <= 128 ? (N <= 64 ? 256 : 512) : 512; }
-static size_t dyson_smem(int N) { return sizeof(zc) * (size_t)N * N; }
-static bool dyson_fits(int N) { return dyson_fits_smem(N); }
+// the blocked kernel with the matrix in the global workspace: orders above the shared-memory limit
+static bool use_bgj(int N) { return !dyson_fits_smem(N) && N <= BGJ_MAXN_GM; }
+constexpr int BGJ_THREADS2 = 256;  // the two-blocks-per-SM form
+constexpr int GJ_THREADS = 512;    // the unblocked kernel, N <= 512
 
-static bool use_blocked(int N) { return N >= 16 && N <= 128 && (size_t)swz_units(N) * 16 + 1536 <= (size_t)SMEM_MAX; }
-// the blocked kernel with the matrix in the global workspace: orders above the shared-memory
-// limit up to 256
-static bool use_blocked_gm(int N) { return !use_blocked(N) && N > 16 && N <= BGJ_MAXN_GM; }
-static inline auto dyson_bgj = dyson_bgj_t<false>;
-constexpr int BGJ_THREADS2 = 256;  // the two-blocks-per-SM form (workspace)
-// the workspace form runs for 16 < N <= 256 (also below the shared-memory limit, as the
-// two-blocks-per-SM variant of the tuner)
-static bool use_bgj_ws(int N) { return N > 16 && N <= BGJ_MAXN_GM; }
+// orders above the shared-memory limit on at most nblocks blocks; variant as in the autotuner
+static void dyson_gm(cudaStream_t st, const DysonArgs &a, int variant, int nblocks) {
+    if (use_bgj(a.N) && variant == DYSON_BLOCKED2)
+        dyson_bgj_t<BGJ_THREADS2><<<std::min(nblocks, 2 * 148), BGJ_THREADS2, 0, st>>>(a);
+    else if (use_bgj(a.N) && variant == DYSON_BLOCKED)  // the concurrent matrices (148 x N^2 x 16 B) stay mostly in L2
+        dyson_bgj_t<BGJ_THREADS><<<std::min(nblocks, 148), BGJ_THREADS, 0, st>>>(a);
+    else
+        dyson_gj<<<nblocks, GJ_THREADS, 0, st>>>(a);
+}
 
-static int launch_dyson(qs_handle *h, DysonArgs &a, int nblocks, int variant) {
-    const int N = a.N;
-    if (variant == DYSON_BLOCKED2 && use_bgj_ws(N) && h->d_Gws) {
-        // two blocks of 8 warps per SM, each matrix in its block's slot of the workspace
-        a.ws = h->d_Gws;
-        nblocks = std::min<int>(std::min(nblocks, 2 * 148), (int)h->ws_slots);
-        int pi = prof_begin(h, K_DYSON);
-        dyson_bgj_t<true, BGJ_THREADS2><<<nblocks, BGJ_THREADS2, 0, h->stream>>>(a);
-        prof_end(h, pi);
-        QS_CUDA(h, cudaGetLastError());
-        return 0;
-    }
-    if (variant == DYSON_BLOCKED && use_blocked_gm(N) && h->d_Gws) {
-        // one block per SM: the concurrent matrices (148 x N^2 x 16 B) stay mostly in L2
-        a.ws = h->d_Gws;
-        nblocks = std::min<int>(std::min(nblocks, 148), (int)h->ws_slots);
-        int pi = prof_begin(h, K_DYSON);
-        dyson_bgj_t<true><<<nblocks, BGJ_THREADS, 0, h->stream>>>(a);
-        prof_end(h, pi);
-        QS_CUDA(h, cudaGetLastError());
-        return 0;
-    }
-    if (variant == DYSON_BLOCKED && use_blocked(N)) {
-        size_t sm = (size_t)swz_units(N) * sizeof(zc);
-        QS_CUDA(h, smem_cap((const void *)dyson_bgj));
-        a.ws = nullptr;
-        int pi = prof_begin(h, K_DYSON);
-        dyson_bgj<<<nblocks, BGJ_THREADS, sm, h->stream>>>(a);
-        prof_end(h, pi);
-        QS_CUDA(h, cudaGetLastError());
-        return 0;
-    }
-    int thr = dyson_threads(N);
-    size_t sm = 0;
-    if (dyson_fits(N)) {
-        sm = dyson_smem(N);
-        QS_CUDA(h, smem_cap((const void *)dyson_gj));
-        a.ws = nullptr;
-    } else {
-        nblocks = std::min<int>(nblocks, (int)h->ws_slots);
-        a.ws = h->d_Gws;
-    }
+static int launch_dyson(qs_handle *h, DysonArgs &a, int variant) {
     int pi = prof_begin(h, K_DYSON);
-    dyson_gj<<<nblocks, thr, sm, h->stream>>>(a);
+    int rc = 0;
+    if (dyson_fits_smem(a.N)) {
+        rc = launch_dyson_blk(h->stream, a);
+    } else {
+        // the matrices are built and inverted where G goes if G has their order: one copy less, and no
+        // slot that the next matrix of the block waits for (192 x 192: 9.2 -> 11.3 TFLOP/s)
+        a.inplace = a.out_mode == 1 || a.nA == a.N;
+        a.ws = h->d_Gws;
+        dyson_gm(h->stream, a, variant, std::min(a.iw1 - a.iw0, 2 * 148));
+    }
     prof_end(h, pi);
+    QS_CUDA(h, (cudaError_t)-rc);
     QS_CUDA(h, cudaGetLastError());
     return 0;
 }
 
-int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_info, zc *d_ws, int ws_slots) {
+int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each) {
     DysonArgs a{};
     a.N = N;
-    a.iw0 = 0;
     a.iw1 = batch;
     a.Ain = d_A;
     a.out_mode = 1;
     a.Gout = d_A;
-    a.info = d_info;
-    a.info_each = d_info + 1;
-    int thr = dyson_threads(N);
-    int nb = std::min(batch, 148 * 8);
-    size_t sm = 0;
-    if (use_blocked(N)) {
-        sm = (size_t)swz_units(N) * sizeof(zc);
-        cudaError_t e = smem_cap((const void *)dyson_bgj);
-        if (e != cudaSuccess) return -(int)e;
-        count_launch();
-        dyson_bgj<<<nb, BGJ_THREADS, sm, st>>>(a);
-        e = cudaGetLastError();
-        return e == cudaSuccess ? 0 : -(int)e;
-    }
-    if (use_blocked_gm(N) && d_ws && ws_slots > 0) {
-        a.ws = d_ws;
-        nb = std::min(std::min(nb, 148), ws_slots);
-        count_launch();
-        dyson_bgj_t<true><<<nb, BGJ_THREADS, 0, st>>>(a);
-        cudaError_t e = cudaGetLastError();
-        return e == cudaSuccess ? 0 : -(int)e;
-    }
-    if (dyson_fits(N)) {
-        sm = dyson_smem(N);
-        cudaError_t e = smem_cap((const void *)dyson_gj);
-        if (e != cudaSuccess) return -(int)e;
-    } else {
-        a.ws = d_ws;
-        nb = std::min(nb, ws_slots);
-    }
+    a.info = d_min;
+    a.info_each = d_each;
+    a.inplace = 1;
     count_launch();
-    dyson_gj<<<nb, thr, sm, st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : -(int)e;
-}
-
-// Batched inversion with every matrix in the given global workspace (ws_slots matrices
-// of N x N complex, reused round-robin by the blocks), whatever N is.
-int invert_batched_ws(cudaStream_t st, int N, int batch, zc *d_A, int *d_min_info, int *d_info_each, zc *d_ws,
-                      int ws_slots) {
-    DysonArgs a{};
-    a.N = N;
-    a.iw0 = 0;
-    a.iw1 = batch;
-    a.Ain = d_A;
-    a.out_mode = 1;
-    a.Gout = d_A;
-    a.info = d_min_info;
-    a.info_each = d_info_each;
-    a.ws = d_ws;
-    int nb = std::min(std::min(batch, 148 * 8), ws_slots);
-    if (nb < 1) return -1;
-    count_launch();
-    dyson_gj<<<nb, dyson_threads(N), 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
+    if (dyson_fits_smem(N)) return launch_dyson_blk(st, a);
+    dyson_gm(st, a, DYSON_BLOCKED2, std::min(batch, 2 * 148));
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : -(int)e;
 }
 
@@ -1270,12 +1137,13 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         a.out_mode = 0;
         a.Gout = h->d_G;
         {
-            int cand[3], nc = 0;
-            if (use_blocked(N) || (use_blocked_gm(N) && h->d_Gws)) cand[nc++] = DYSON_BLOCKED;
-            if (use_bgj_ws(N) && h->d_Gws) cand[nc++] = DYSON_BLOCKED2;
-            cand[nc++] = DYSON_UNBLOCKED;
-            rc = tune_launch(h, TUNE_DYSON, tune_key(N, n), cand, nc, nc > 1 ? cand[0] : DYSON_UNBLOCKED,
-                             [&](int v) { return launch_dyson(h, a, std::min(n, 148 * 16), v); });
+            // one form in shared memory; above, the two blocked ones on the workspace, and beyond
+            // their order the unblocked one
+            int cand[2], nc = 0;
+            if (dyson_fits_smem(N) || use_bgj(N)) cand[nc++] = DYSON_BLOCKED;
+            if (use_bgj(N)) cand[nc++] = DYSON_BLOCKED2;
+            if (!nc) cand[nc++] = DYSON_UNBLOCKED;
+            rc = tune_launch(h, TUNE_DYSON, tune_key(N, n), cand, nc, cand[0], [&](int v) { return launch_dyson(h, a, v); });
             if (rc) return rc;
         }
         KeldyshArgs k{};
@@ -1339,7 +1207,7 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         a.iw1 = iw1;
         a.out_mode = 1;
         a.Gout = h->d_G;
-        if ((rc = launch_dyson(h, a, std::min(iw1 - iw0, 148 * 16), DYSON_BLOCKED))) return rc;
+        if ((rc = launch_dyson(h, a, DYSON_BLOCKED))) return rc;
         FinalArgs f{};
         f.N = N;
         f.nS = h->nS;
