@@ -23,28 +23,21 @@
 //
 // Measured on B200, batched inversion (8 N^3 flops a matrix), against the kernels this replaces
 // (row exchanges, 16-wide panels, one block a matrix, or everything through a global workspace):
-// N = 120 8.9 -> 12.9 TFLOP/s; as Dyson of 40 states x 5003 energies 0.99 -> 0.40 ms,
-// 24 x 32768 3.05 -> 0.61 ms, 48 x 4001 1.58 -> 0.38 ms. At N = 120 a matrix takes 300k cycles: the
-// panels 128k (1070 a column), the updates 141k (107k at the DMMA rate), load and output 30k.
+// N = 120 8.9 -> 13.9 TFLOP/s; as Dyson of 40 states x 5003 energies 0.99 -> 0.39 ms,
+// 24 x 32768 3.05 -> 0.54 ms, 48 x 4001 1.58 -> 0.36 ms. At N = 120 a matrix takes 280k cycles: the
+// panels 128k (1070 a column), the updates 125k (107k at the DMMA rate), load and output 30k.
 // Tried instead for N <= 96: the whole matrix in registers, rank-1 updates (4-9 TFLOP/s: the
 // per-step work of every warp, column and row exchange and selects, outweighs the update).
 #include <algorithm>
 #include <climits>
 
 #include "qs_common.cuh"
+#include "zmma.cuh"
 
 namespace qs {
 namespace {
 
 constexpr int PB = 8;  // panel width
-
-// D = A B + D with A 16x8, B 8x8 in FP64: a_i = A(g + 8(i&1), t + 4(i>>1)), i < 4;
-// b_i = B(t + 4i, g), i < 2; c_i = C(g + 8(i>>1), 2t + (i&1)) (g = lane / 4, t = lane % 4)
-__device__ __forceinline__ void dmma1688(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
 
 // 1 / a without overflow or underflow of the intermediate |a|^2: a is scaled by the power of two
 // that brings its larger part to [1, 2)
@@ -54,12 +47,6 @@ __device__ __forceinline__ zc scaled_recip(zc a) {
     const double x = a.x * s, y = a.y * s, d = s / fma(x, x, y * y);
     return zc{x * d, -y * d};
 }
-
-// Position of element (i, j): column-major with the leading dimension padded to a multiple of 8 and
-// the row index XORed with j mod 8 (a warp's 16 x 8 fragments and its walks along a row or a column
-// then spread over the banks).
-__device__ __forceinline__ int at(int i, int j, int N) { return (i + j * ((N + 7) & ~7)) ^ (j & 7); }
-__host__ __device__ __forceinline__ int smem_units(int N) { return N * ((N + 7) & ~7); }
 
 template <int PW> struct Exchange {
     zc row[2][PW][PB];  // each panel warp's candidate row; steps alternate between the two
@@ -118,6 +105,8 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
                 M[at(i, j, N)] = v;
             }
         }
+        // the columns that pad the last tile: zero operands (rows beyond N reach rows beyond N only)
+        for (int t = N * smem_ld(N) + tid; t < smem_units(N); t += nthr) M[t] = zc{0, 0};
         if (tid == 0) e.first_zero = 0;
         const bool is_panel = warp < PW;
         bool open = is_panel && tid < N;  // this lane's row is not used yet
@@ -202,47 +191,39 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
                 if (lane == 0) e.used[warp] = u;
             }
             sync();
-            const int kb = min(PB, N - k0);
+            // the lane's places in the fragments of column tile 0: A(g, t4 [+ 4]), C(g, 2 t4 [+ 1])
+            const int ld = smem_ld(N), kb = min(PB, N - k0);
+            const int a0 = (g ^ xr(t4)) + t4 * ld, a1 = (g ^ xr(t4 + 4)) + (t4 + 4) * ld;
+            const int e0 = (g ^ xr(2 * t4)) + 2 * t4 * ld, e1 = (g ^ xr(2 * t4 + 1)) + (2 * t4 + 1) * ld;
+            const int p0 = t4 < kb ? e.perm[k0 + t4] : -1, p1 = t4 + 4 < kb ? e.perm[k0 + t4 + 4] : -1;
             for (int ct = warp; ct < ntiles; ct += W) {
                 if (ct == k0 / PB) continue;
                 const int j0 = 8 * ct;
-                double br[2], bi[2], nbi[2];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const int t = t4 + 4 * q;
-                    const zc v = (t < kb && j0 + g < N) ? M[at(e.perm[k0 + t], j0 + g, N)] : zc{0, 0};
-                    br[q] = v.x;
-                    bi[q] = v.y;
-                    nbi[q] = -v.y;
-                }
+                const zc v0 = p0 >= 0 ? M[j0 * ld + g * ld + (p0 ^ xr(g))] : zc{0, 0};
+                const zc v1 = p1 >= 0 ? M[j0 * ld + g * ld + (p1 ^ xr(g))] : zc{0, 0};
+                const double br[2] = {v0.x, v1.x}, bi[2] = {v0.y, v1.y}, nbi[2] = {-v0.y, -v1.y};
                 __syncwarp();  // the fragments are read before other lanes of this warp rewrite the pivot rows
+                const zc *Ap0 = M + k0 * ld + a0, *Ap1 = M + k0 * ld + a1;
+                zc *Cp0 = M + j0 * ld + e0, *Cp1 = M + j0 * ld + e1;
 #pragma unroll 2
                 for (int rt = 0; rt < mtiles; rt++) {
                     const int i0 = 16 * rt;
                     const unsigned um = e.used[i0 >> 5] >> (i0 & 31);  // pivot rows of this tile
-                    double ar[4], ai[4], cr[4], ci[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = i0 + g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
-                        const zc v = (r < N && c < kb) ? M[at(r, k0 + c, N)] : zc{0, 0};
-                        ar[q] = v.x;
-                        ai[q] = v.y;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int dr = g + 8 * (q >> 1), r = i0 + dr, c = j0 + 2 * t4 + (q & 1);
-                        const zc v = (r < N && c < N && !((um >> dr) & 1)) ? M[at(r, c, N)] : zc{0, 0};
-                        cr[q] = v.x;
-                        ci[q] = v.y;
-                    }
+                    const bool ug = (um >> g) & 1, uh = (um >> (g + 8)) & 1, low = i0 + 8 < N;
+                    const zc u0 = Ap0[i0], u1 = Ap0[i0 + 8], u2 = Ap1[i0], u3 = Ap1[i0 + 8];
+                    const double ar[4] = {u0.x, u1.x, u2.x, u3.x}, ai[4] = {u0.y, u1.y, u2.y, u3.y};
+                    const zc w0 = Cp0[i0], w1 = Cp1[i0], w2 = Cp0[i0 + 8], w3 = Cp1[i0 + 8];
+                    double cr[4] = {ug ? 0.0 : w0.x, ug ? 0.0 : w1.x, uh ? 0.0 : w2.x, uh ? 0.0 : w3.x};
+                    double ci[4] = {ug ? 0.0 : w0.y, ug ? 0.0 : w1.y, uh ? 0.0 : w2.y, uh ? 0.0 : w3.y};
                     dmma1688(cr, ar, br);
                     dmma1688(ci, ar, bi);
                     dmma1688(cr, ai, nbi);
                     dmma1688(ci, ai, br);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                        if (r < N && c < N) M[at(r, c, N)] = zc{cr[q], ci[q]};
+                    Cp0[i0] = zc{cr[0], ci[0]};
+                    Cp1[i0] = zc{cr[1], ci[1]};
+                    if (low) {  // (the last tile's lower half may lie in the next column)
+                        Cp0[i0 + 8] = zc{cr[2], ci[2]};
+                        Cp1[i0 + 8] = zc{cr[3], ci[3]};
                     }
                 }
             }

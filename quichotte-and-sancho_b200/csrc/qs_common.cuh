@@ -313,6 +313,9 @@ struct KeldyshArgs {
     const int *cidx;    // the contact states: rows/columns where GamLs or GamRs is non-zero
     int nc;             // their number (-1: not known)
 };
+// the Keldysh step with both operands in shared memory (keldysh_sm.cu): nA <= 80
+int launch_keldysh_sm(qs_handle *h, const KeldyshArgs &k);
+bool keldysh_sm_fits(int nA);
 // the FP32-phase Keldysh step of a QS_PREC_MIXED solve on the fifth-generation tensor cores
 // (keldysh_tf32.cu): 32 <= nA <= 128; returns -1 for other sizes
 int launch_keldysh_tf32(qs_handle *h, const KeldyshArgs &k);

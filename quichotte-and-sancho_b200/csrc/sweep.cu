@@ -1172,6 +1172,7 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         auto launch_k = [&](int v) -> int {
             int pi;
             if (v == KELDYSH_TF32) return launch_keldysh_tf32(h, k);
+            if (v == KELDYSH_TC && keldysh_sm_fits(nA)) return launch_keldysh_sm(h, k);
             if (v == KELDYSH_TC) {
                 QS_CUDA(h, smem_cap((const void *)keldysh_tc));
                 pi = prof_begin(h, K_KELDYSH);
@@ -1184,19 +1185,19 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
             QS_CUDA(h, cudaGetLastError());
             return 0;
         };
-        const bool tc_ok = nA >= 32 && nA <= KD_MP && h->T_slots >= (size_t)(2 * nbt);
-        const int fallback = (tc_ok && nA >= 48) ? KELDYSH_TC : KELDYSH_CUDA;
+        const bool sm = keldysh_sm_fits(nA), tc_ok = sm || (nA <= KD_MP && h->T_slots >= (size_t)(2 * nbt));
+        const int fallback = tc_ok ? KELDYSH_TC : KELDYSH_CUDA;
         // the FP32 phase of a QS_PREC_MIXED solve: the 3xTF32 kernel on the fifth-generation
         // tensor cores is a candidate too, kept only where it is the fastest
         if (fp32 && mode == M_SCF2 && keldysh_tf32_fits(nA)) {
             int c3[3], nc = 0;
             c3[nc++] = KELDYSH_TF32;
             if (tc_ok) c3[nc++] = KELDYSH_TC;
-            c3[nc++] = KELDYSH_CUDA;
+            if (!sm) c3[nc++] = KELDYSH_CUDA;
             return tune_launch(h, TUNE_KELDYSH32, tune_key(nA, n), c3, nc, fallback, launch_k);
         }
         const int cand[2] = {KELDYSH_TC, KELDYSH_CUDA};
-        return tune_launch(h, TUNE_KELDYSH, tune_key(nA, n), tc_ok ? cand : cand + 1, tc_ok ? 2 : 1, fallback,
+        return tune_launch(h, TUNE_KELDYSH, tune_key(nA, n), tc_ok ? cand : cand + 1, tc_ok && !sm ? 2 : 1, fallback,
                            launch_k);
     }
     // chunked full inversion + per-energy outputs
