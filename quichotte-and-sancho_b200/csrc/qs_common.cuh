@@ -316,6 +316,9 @@ struct KeldyshArgs {
 // the Keldysh step with both operands in shared memory (keldysh_sm.cu): nA <= 80
 int launch_keldysh_sm(qs_handle *h, const KeldyshArgs &k);
 bool keldysh_sm_fits(int nA);
+// the same by blocks of 32 rows (keldysh_rows.cu): nA <= 256
+int launch_keldysh_rows(qs_handle *h, const KeldyshArgs &k);
+bool keldysh_rows_fits(int nA);
 // the FP32-phase Keldysh step of a QS_PREC_MIXED solve on the fifth-generation tensor cores
 // (keldysh_tf32.cu): 32 <= nA <= 128; returns -1 for other sizes
 int launch_keldysh_tf32(qs_handle *h, const KeldyshArgs &k);

@@ -551,323 +551,6 @@ __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
     }
 }
 
-// ---------------------------------------------------------------------------------
-// The same step on the FP64 tensor cores for 48 <= nA <= 128: T = G^r SL and the upper
-// triangle of G^< = T G^r^dagger as complex m16n8k16 MMAs (4 real MMAs per complex tile),
-// operands padded to 128 and staged through shared memory in 16-wide k panels by cp.async,
-// double-buffered. 8 warps, one block per SM walking the energies; a warp owns a 32-row
-// block of 8-column tiles. SL and T go through two scratch matrices of the block (L2).
-// ---------------------------------------------------------------------------------
-constexpr int KD_MP = 128, KD_LDA = 130, KD_LDN = 20;  // padded order; [k][m] / [n][k] panel strides
-constexpr int KD_ASZ = 16 * KD_LDA, KD_BSZ = KD_MP * KD_LDN, KD_STAGE = KD_ASZ + KD_BSZ;
-constexpr size_t KD_SMEM = 2 * KD_STAGE * sizeof(zc);
-
-__device__ __forceinline__ void cpa16(void *dst, const void *src, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-
-// C(m0 + 0..31, n0 + 0..8NT-1) = A B over k < nA. A: nA x nA column-major; B(k, n) staged
-// [n][k], with SIG Sigma2^< of an energy (sig_l; its lower blocks are staged as stored and get
-// their sign at the fragment loads), else Bm[k + n nA]; only columns nlo..nhi-1 of B are staged. Every thread of the
-// block calls it (the panel copies); warps with !active skip the MMAs, and tiles beyond nA
-// are skipped (warp-uniform).
-template <int NT, bool SIG>
-__device__ __forceinline__ void kd_gemm(const zc *__restrict__ A, const zc *__restrict__ Bm, int nA, int nlo, int nhi,
-                                        int m0, int n0, bool active, zc *sm, double (&cr)[2][NT][4],
-                                        double (&ci)[2][NT][4]) {
-    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int nk = (nA + 15) / 16, nw = nhi - nlo;
-#pragma unroll
-    for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-        for (int ni = 0; ni < NT; ni++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) cr[mi][ni][q] = ci[mi][ni][q] = 0.0;
-    auto load = [&](int kc, int st) {
-        zc *As = sm + st * KD_STAGE, *Bs = As + KD_ASZ;
-        const int k0 = kc * 16;
-        for (int idx = tid; idx < 16 * KD_MP; idx += blockDim.x) {
-            const int m = idx & (KD_MP - 1), kk = idx >> 7;
-            const bool v = m < nA && k0 + kk < nA;
-            cpa16(&As[kk * KD_LDA + m], v ? A + m + (size_t)(k0 + kk) * nA : A, v);
-        }
-        for (int idx = tid; idx < 16 * nw; idx += blockDim.x) {
-            const int kk = idx & 15, nn = nlo + (idx >> 4);
-            const bool v = nn < nA && k0 + kk < nA;
-            const zc *src = SIG ? sig_l_at(Bm, k0 + kk, nn) : Bm + (k0 + kk) + (size_t)nn * nA;
-            cpa16(&Bs[nn * KD_LDN + kk], v ? src : Bm, v);
-        }
-    };
-    load(0, 0);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    for (int kc = 0; kc < nk; kc++) {
-        if (kc + 1 < nk) load(kc + 1, (kc + 1) & 1);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        __syncthreads();
-        if (active) {
-            const zc *As = sm + (kc & 1) * KD_STAGE, *Bs = As + KD_ASZ;
-            double ar[2][8], ai[2][8];
-#pragma unroll
-            for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const zc v = As[(t4 + 4 * (q >> 1)) * KD_LDA + m0 + 16 * mi + g + 8 * (q & 1)];
-                    ar[mi][q] = v.x;
-                    ai[mi][q] = v.y;
-                }
-#pragma unroll
-            for (int ni = 0; ni < NT; ni++) {
-                const int c0 = n0 + 8 * ni;
-                if (c0 >= nA) continue;
-                const bool t0 = m0 < nA, t1 = m0 + 16 < nA;
-                if (!t0 && !t1) continue;
-                double br[4], bi[4], nbi[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    zc v = Bs[(c0 + g) * KD_LDN + t4 + 4 * q];
-                    if (SIG && ((16 * kc + t4 + 4 * q) >> 1) > ((c0 + g) >> 1)) v.x = -v.x;
-                    br[q] = v.x;
-                    bi[q] = v.y;
-                    nbi[q] = -v.y;
-                }
-                if (t0 && t1) {  // the two row tiles interleaved: dependent MMAs are three apart
-                    dmma16816(cr[0][ni], ar[0], br);
-                    dmma16816(cr[1][ni], ar[1], br);
-                    dmma16816(ci[0][ni], ar[0], bi);
-                    dmma16816(ci[1][ni], ar[1], bi);
-                    dmma16816(cr[0][ni], ai[0], nbi);
-                    dmma16816(cr[1][ni], ai[1], nbi);
-                    dmma16816(ci[0][ni], ai[0], br);
-                    dmma16816(ci[1][ni], ai[1], br);
-                } else if (t0) {
-                    dmma16816(cr[0][ni], ar[0], br);
-                    dmma16816(ci[0][ni], ar[0], bi);
-                    dmma16816(cr[0][ni], ai[0], nbi);
-                    dmma16816(ci[0][ni], ai[0], br);
-                } else {
-                    dmma16816(cr[1][ni], ar[1], br);
-                    dmma16816(ci[1][ni], ar[1], bi);
-                    dmma16816(cr[1][ni], ai[1], nbi);
-                    dmma16816(ci[1][ni], ai[1], br);
-                }
-            }
-        }
-        __syncthreads();  // the stage is refilled two chunks later
-    }
-}
-
-// The upper triangle of G^< = T G^dagger as a list of 16 x 8 tiles (row tile rt, column
-// tile ct with 16 rt <= 8 ct + 7, inside nA): pass p gives warp w the tiles p*64 + 8 s + w,
-// s < 8, so the warps share every pass evenly. Operand panels as in kd_gemm (B conjugate-
-// transposed from G); put(i, j, re, im) receives every element of the warp's tiles.
-constexpr int KD_SLOTS = 8;
-constexpr int KD_NCMAX = 16;  // contact states up to which the lead term is a low-rank correction
-__device__ __forceinline__ int kd_upper_tiles(int nA) {
-    int cnt = 0;
-    for (int ct = 0; 8 * ct < nA; ct++) cnt += min((8 * ct + 7) / 16 + 1, (nA + 15) / 16);
-    return cnt;
-}
-// the t-th upper tile in column-major order of tiles
-__device__ __forceinline__ void kd_upper_tile(int nA, int t, int &rt, int &ct) {
-    for (ct = 0; 8 * ct < nA; ct++) {
-        const int h = min((8 * ct + 7) / 16 + 1, (nA + 15) / 16);
-        if (t < h) {
-            rt = t;
-            return;
-        }
-        t -= h;
-    }
-    rt = -1;
-}
-
-template <class PUT>
-__device__ __forceinline__ void kd_upper_gemm(const zc *__restrict__ T, const zc *__restrict__ G, int nA, zc *sm,
-                                              PUT put) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-    const int nk = (nA + 15) / 16, ntl = kd_upper_tiles(nA);
-    for (int base = 0; base < ntl; base += 8 * KD_SLOTS) {
-        int rts[KD_SLOTS], cts[KD_SLOTS];
-#pragma unroll
-        for (int q = 0; q < KD_SLOTS; q++) {
-            const int t = base + 8 * q + warp;
-            if (t < ntl) kd_upper_tile(nA, t, rts[q], cts[q]);
-            else rts[q] = -1;
-        }
-        double cr[KD_SLOTS][4], ci[KD_SLOTS][4];
-#pragma unroll
-        for (int q = 0; q < KD_SLOTS; q++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) cr[q][e] = ci[q][e] = 0.0;
-        auto load = [&](int kc, int st) {
-            zc *As = sm + st * KD_STAGE, *Bs = As + KD_ASZ;
-            const int k0 = kc * 16;
-            for (int idx = tid; idx < 16 * KD_MP; idx += blockDim.x) {
-                const int m = idx & (KD_MP - 1), kk = idx >> 7;
-                const bool v = m < nA && k0 + kk < nA;
-                cpa16(&As[kk * KD_LDA + m], v ? T + m + (size_t)(k0 + kk) * nA : T, v);
-                cpa16(&Bs[kk * KD_LDA + m], v ? G + m + (size_t)(k0 + kk) * nA : G, v);
-            }
-        };
-        load(0, 0);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        for (int kc = 0; kc < nk; kc++) {
-            if (kc + 1 < nk) load(kc + 1, (kc + 1) & 1);
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-            __syncthreads();
-            const zc *As = sm + (kc & 1) * KD_STAGE, *Bs = As + KD_ASZ;
-#pragma unroll
-            for (int q = 0; q < KD_SLOTS; q++) {
-                if (rts[q] < 0) continue;
-                const int r0 = 16 * rts[q], c0 = 8 * cts[q];
-                double ar[8], ai[8], br[4], bi[4], nbi[4];
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const zc v = As[(t4 + 4 * (e >> 1)) * KD_LDA + r0 + g + 8 * (e & 1)];
-                    ar[e] = v.x;
-                    ai[e] = v.y;
-                }
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const zc v = Bs[(t4 + 4 * e) * KD_LDA + c0 + g];  // B(k, n) = conj(G(n, k))
-                    br[e] = v.x;
-                    bi[e] = -v.y;
-                    nbi[e] = v.y;
-                }
-                dmma16816(cr[q], ar, br);
-                dmma16816(ci[q], ar, bi);
-                dmma16816(cr[q], ai, nbi);
-                dmma16816(ci[q], ai, br);
-            }
-            __syncthreads();  // the stage is refilled two chunks later
-        }
-#pragma unroll
-        for (int q = 0; q < KD_SLOTS; q++) {
-            if (rts[q] < 0) continue;
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                put(16 * rts[q] + g + 8 * (e >> 1), 8 * cts[q] + 2 * t4 + (e & 1), cr[q][e], ci[q][e]);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256, 1) keldysh_tc(KeldyshArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    zc *sm = (zc *)smem_raw;
-    const int nA = a.nA, nfull = nA * nA;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-    zc *T = a.Tws + (size_t)(2 * blockIdx.x) * nfull;
-    zc *S = T + nfull;
-    for (int iw = blockIdx.x; iw < a.n; iw += gridDim.x) {
-        const zc *G = a.G + (size_t)iw * nfull;
-        const double w = a.omega[iw];
-        const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
-        const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
-        // SL = i (fL GamL_s + fR GamR_s) / hbar + Sigma2^<   (src/scf.f90:333-336). With
-        // few contact states (the usual case) the first product takes Sigma2^< itself as
-        // its B operand and the lead term is added to the contact columns of T afterwards
-        // (a rank-nc correction); otherwise SL is built in the block's scratch (the loads
-        // of 8 elements a thread issued before their stores).
-        const bool lowrank = SL2 && a.nc >= 0 && a.nc <= KD_NCMAX;
-        for (int base = threadIdx.x; !lowrank && base < nfull; base += 8 * blockDim.x) {
-            zc gl[8], gr[8], s2[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int idx = base + u * blockDim.x;
-                const bool v = idx < nfull;
-                gl[u] = v ? a.GamLs[idx] : zc{0, 0};
-                gr[u] = v ? a.GamRs[idx] : zc{0, 0};
-                s2[u] = (v && SL2) ? sig_l(SL2, idx % nA, idx / nA) : zc{0, 0};
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int idx = base + u * blockDim.x;
-                if (idx < nfull) S[idx] = zc{-(fL * gl[u].y + fR * gr[u].y) + s2[u].x, fL * gl[u].x + fR * gr[u].x + s2[u].y};
-            }
-        }
-        __threadfence_block();
-        __syncthreads();
-        // T = G SL, in two column halves of 64
-        for (int hh = 0; hh < 2; hh++) {
-            if (64 * hh >= nA) break;
-            double cr[2][4][4], ci[2][4][4];
-            const int m0 = 32 * (warp & 3), n0 = 64 * hh + 32 * (warp >> 2);
-            if (lowrank) kd_gemm<4, true>(G, SL2, nA, 64 * hh, 64 * hh + 64, m0, n0, m0 < nA && n0 < nA, sm, cr, ci);
-            else kd_gemm<4, false>(G, S, nA, 64 * hh, 64 * hh + 64, m0, n0, m0 < nA && n0 < nA, sm, cr, ci);
-#pragma unroll
-            for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-                for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = m0 + 16 * mi + g + 8 * (q >> 1), c = n0 + 8 * ni + 2 * t4 + (q & 1);
-                        if (r < nA && c < nA) T[r + (size_t)c * nA] = zc{cr[mi][ni][q], ci[mi][ni][q]};
-                    }
-        }
-        __threadfence_block();
-        __syncthreads();
-        if (lowrank && a.nc > 0) {
-            // T(r, b) += sum over contact states c of G(r, c) i (fL GamL_s + fR GamR_s)(c, b), b a contact state
-            for (int t = threadIdx.x; t < nA * a.nc; t += blockDim.x) {
-                const int r = t % nA, b = a.cidx[t / nA];
-                zc acc = T[r + (size_t)b * nA];
-                for (int q = 0; q < a.nc; q++) {
-                    const int c = a.cidx[q];
-                    const size_t cb = c + (size_t)b * nA;
-                    const zc gl = a.GamLs[cb], gr = a.GamRs[cb];
-                    cfma(acc, G[r + (size_t)c * nA], zc{-(fL * gl.y + fR * gr.y), fL * gl.x + fR * gr.x});
-                }
-                T[r + (size_t)b * nA] = acc;
-            }
-            __threadfence_block();
-            __syncthreads();
-        }
-        double *blk = a.out + (size_t)iw * a.nblk;
-        const double *xb = a.xsub ? a.xsub + (size_t)iw * a.nblk : nullptr;
-        auto put = [&](int r, int c, double vr, double vi) {
-            if (r >= nA || c >= nA || r > c) return;
-            if (r < c) {
-                const int o = dl_l(r, c);
-                blk[o] = xb ? vr - xb[o] : vr;
-                blk[o + 1] = xb ? vi - xb[o + 1] : vi;
-            } else {
-                const int o = dl_d(r);
-                blk[o] = xb ? vi - xb[o] : vi;
-                if (a.gLd) a.gLd[(size_t)iw * nA + r] = zc{vr, vi};
-            }
-        };
-        // upper triangle of G^< = T G^dagger, 16 x 8 tiles shared evenly by the warps
-        kd_upper_gemm(T, G, nA, sm, put);
-        // G^r part of the block (8 elements a thread in flight)
-        for (int base = threadIdx.x; base < nfull; base += 8 * blockDim.x) {
-            zc gv[8], xv[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int idx = base + u * blockDim.x;
-                int i, j;
-                block_order(idx, nA, i, j);
-                const bool v = idx < nfull;
-                gv[u] = v ? G[i + (size_t)j * nA] : zc{0, 0};
-                xv[u] = (v && xb) ? *(const zc *)(xb + dl_r(i, j)) : zc{0, 0};
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int idx = base + u * blockDim.x;
-                if (idx < nfull) {
-                    int i, j;
-                    block_order(idx, nA, i, j);
-                    *(zc *)(blk + dl_r(i, j)) = gv[u] - xv[u];
-                }
-            }
-        }
-        if (a.gRd)
-            for (int i = threadIdx.x; i < nA; i += blockDim.x) a.gRd[(size_t)iw * nA + i] = G[i + (size_t)i * nA];
-        __syncthreads();  // S and T are rewritten for the next energy
-    }
-}
-
 struct FinalArgs {
     int N, nS, nA, nCL, N_sites, N_atoms, iw0, iw1, mode;
     const zc *G;  // full G per energy of the chunk
@@ -1167,38 +850,24 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         k.err = h->d_info + 1;
         k.cidx = h->d_kd_cidx;
         k.nc = (h->nS == nA) ? h->kd_nc : -1;
-        const int nb = (int)std::min<size_t>(h->T_slots, (size_t)n);
-        const int nbt = std::min(n, 148);
         auto launch_k = [&](int v) -> int {
-            int pi;
             if (v == KELDYSH_TF32) return launch_keldysh_tf32(h, k);
-            if (v == KELDYSH_TC && keldysh_sm_fits(nA)) return launch_keldysh_sm(h, k);
-            if (v == KELDYSH_TC) {
-                QS_CUDA(h, smem_cap((const void *)keldysh_tc));
-                pi = prof_begin(h, K_KELDYSH);
-                keldysh_tc<<<nbt, 256, KD_SMEM, h->stream>>>(k);
-            } else {
-                pi = prof_begin(h, K_KELDYSH);
-                keldysh_scf2<<<nb, 256, 0, h->stream>>>(k);
-            }
+            if (v == KELDYSH_TC) return keldysh_sm_fits(nA) ? launch_keldysh_sm(h, k) : launch_keldysh_rows(h, k);
+            int pi = prof_begin(h, K_KELDYSH);
+            keldysh_scf2<<<(int)std::min<size_t>(h->T_slots, (size_t)n), 256, 0, h->stream>>>(k);
             prof_end(h, pi);
             QS_CUDA(h, cudaGetLastError());
             return 0;
         };
-        const bool sm = keldysh_sm_fits(nA), tc_ok = sm || (nA <= KD_MP && h->T_slots >= (size_t)(2 * nbt));
-        const int fallback = tc_ok ? KELDYSH_TC : KELDYSH_CUDA;
+        // one FP64 form per order
+        const int fp64 = keldysh_rows_fits(nA) ? KELDYSH_TC : KELDYSH_CUDA;
         // the FP32 phase of a QS_PREC_MIXED solve: the 3xTF32 kernel on the fifth-generation
         // tensor cores is a candidate too, kept only where it is the fastest
         if (fp32 && mode == M_SCF2 && keldysh_tf32_fits(nA)) {
-            int c3[3], nc = 0;
-            c3[nc++] = KELDYSH_TF32;
-            if (tc_ok) c3[nc++] = KELDYSH_TC;
-            if (!sm) c3[nc++] = KELDYSH_CUDA;
-            return tune_launch(h, TUNE_KELDYSH32, tune_key(nA, n), c3, nc, fallback, launch_k);
+            const int c3[2] = {KELDYSH_TF32, fp64};
+            return tune_launch(h, TUNE_KELDYSH32, tune_key(nA, n), c3, 2, fp64, launch_k);
         }
-        const int cand[2] = {KELDYSH_TC, KELDYSH_CUDA};
-        return tune_launch(h, TUNE_KELDYSH, tune_key(nA, n), tc_ok ? cand : cand + 1, tc_ok && !sm ? 2 : 1, fallback,
-                           launch_k);
+        return tune_launch(h, TUNE_KELDYSH, tune_key(nA, n), &fp64, 1, fp64, launch_k);
     }
     // chunked full inversion + per-energy outputs
     const int Mrows = (mode == M_FINAL) ? N : nA;
