@@ -31,22 +31,11 @@
 #include <algorithm>
 #include <climits>
 
-#include "qs_common.cuh"
+#include "gauss.cuh"
 #include "zmma.cuh"
 
 namespace qs {
 namespace {
-
-constexpr int PB = 8;  // panel width
-
-// 1 / a without overflow or underflow of the intermediate |a|^2: a is scaled by the power of two
-// that brings its larger part to [1, 2)
-__device__ __forceinline__ zc scaled_recip(zc a) {
-    const unsigned h = max((unsigned)__double2hiint(a.x) & 0x7fffffffu, (unsigned)__double2hiint(a.y) & 0x7fffffffu) >> 20;
-    const double s = __hiloint2double((int)(min(max(2046 - (int)h, 1), 2046) << 20), 0);  // 2^(1023 - h)
-    const double x = a.x * s, y = a.y * s, d = s / fma(x, x, y * y);
-    return zc{x * d, -y * d};
-}
 
 template <int PW> struct Exchange {
     zc row[2][PW][PB];  // each panel warp's candidate row; steps alternate between the two
@@ -123,15 +112,9 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
                 for (int c = 0; c < PB; c++) {
                     const int k = k0 + c, b = c & 1;
                     if (k >= N) break;
-                    // |Re| + |Im| >= 0, so its bit pattern orders like its value (a NaN is a large key: a
-                    // row is always found); 0 marks a row that is used or beyond the matrix
-                    const unsigned long long key = open ? (unsigned long long)__double_as_longlong(cabs1(R[c])) + 1 : 0;
+                    const unsigned long long key = pivot_key(R[c], open);
                     const zc inv = scaled_recip(R[c]);  // in case this row is chosen
-                    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-                    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-                    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-                    const unsigned bal = __ballot_sync(0xffffffffu, hi == mh && lo == ml);
-                    if (lane == __ffs(bal) - 1) {  // the first maximum, as izamax
+                    if (lane == warp_pivot(key)) {
 #pragma unroll
                         for (int j = 0; j < PB; j++)
                             if (j != c) e.row[b][warp][j] = R[j];
@@ -170,18 +153,7 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
                         e.step[p] = (unsigned char)k;
                         if (zero && fz == 0) e.first_zero = k + 1;
                     }
-#pragma unroll
-                    for (int j = 0; j < PB; j++) {
-                        const zc r = j == c ? zc{1, 0} : e.row[b][wb][j];
-                        if (j == c) {
-                            R[j] = R[j] - m;
-                        } else {
-                            R[j].x = fma(-m.x, r.x, R[j].x);
-                            R[j].y = fma(-m.x, r.y, R[j].y);
-                            R[j].x = fma(m.y, r.y, R[j].x);
-                            R[j].y = fma(-m.y, r.x, R[j].y);
-                        }
-                    }
+                    eliminate(R, c, m, e.row[b][wb]);
                 }
                 if (tid < N)
 #pragma unroll

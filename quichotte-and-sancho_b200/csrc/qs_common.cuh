@@ -99,30 +99,6 @@ __device__ __forceinline__ zc sig_l(const zc *S, int i, int j) {
     return (i >> 1) <= (j >> 1) ? v : zc{-v.x, v.y};
 }
 
-// FP64 tensor-core MMA, D = A B + D with A 16x16 (row), B 16x8 (col), f64 accumulate.
-// Fragments (g = lane/4, t = lane%4): a_i = A(g + 8(i&1), t + 4(i>>1)), i < 8;
-// b_i = B(t + 4i, g), i < 4; c_i = C(g + 8(i>>1), 2t + (i&1)), i < 4.
-// (not volatile: the compiler may schedule independent MMAs between dependent ones)
-__device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
-    asm(
-        "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
-        "{%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
-          "d"(b[2]), "d"(b[3]));
-}
-// complex 16x8 tile update C += A B from split real/imaginary fragments (4 real MMAs)
-__device__ __forceinline__ void zmma16816(double (&cr)[4], double (&ci)[4], const double (&ar)[8], const double (&ai)[8],
-                                          const double (&br)[4], const double (&bi)[4]) {
-    double nai[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) nai[k] = -ai[k];
-    dmma16816(cr, ar, br);
-    dmma16816(cr, nai, bi);
-    dmma16816(ci, ar, bi);
-    dmma16816(ci, ai, br);
-}
-
 constexpr double PI = 3.14159265358979323846;
 constexpr int SMEM_MAX = 232448;  // max dynamic shared memory per block on sm_100 (227 KB)
 
@@ -294,6 +270,10 @@ struct DysonArgs {
 };
 // the blocked elimination in shared memory (dyson_blk.cu), N <= DYSON_SMEM_MAXN; 0 or a CUDA error (< 0)
 int launch_dyson_blk(cudaStream_t st, const DysonArgs &a);
+// the same with the matrix in global memory (dyson_l2.cu), 16 < N <= 256; DYSON_L2_SLOTS workspaces unless inplace
+constexpr int DYSON_L2_SLOTS = 2 * 148;
+int launch_dyson_l2(cudaStream_t st, const DysonArgs &a);
+bool dyson_l2_fits(int N);
 
 // arguments of the Keldysh kernels (sweep modes M_INIT2 / M_SCF2)
 struct KeldyshArgs {
@@ -342,9 +322,8 @@ int sigma2_compute(qs_handle *h, const double *d_x, bool fp32 = false);
 // TUNE_KELDYSH32: the Keldysh step of a mixed solve's FP32 phase, where the 3xTF32 tensor-core
 // kernel (keldysh_tf32.cu) competes with the two FP64 ones
 enum TuneKind { TUNE_DYSON = 0, TUNE_KELDYSH = 1, TUNE_KELDYSH32 = 4 };
-// DYSON_BLOCKED: in shared memory up to DYSON_SMEM_MAXN, above in the global workspace, one block
-// per SM; DYSON_BLOCKED2: in the workspace, two 8-warp blocks per SM
-enum { DYSON_BLOCKED = 1, DYSON_UNBLOCKED = 2, DYSON_BLOCKED2 = 3, KELDYSH_TC = 1, KELDYSH_CUDA = 2, KELDYSH_TF32 = 3 };
+// DYSON_BLOCKED: dyson_blk or dyson_l2 by the order
+enum { DYSON_BLOCKED = 1, DYSON_UNBLOCKED = 2, KELDYSH_TC = 1, KELDYSH_CUDA = 2, KELDYSH_TF32 = 3 };
 // the size key of a decision: the matrix order and the octave of the grid length (how many
 // energies each SM gets changes which variant wins)
 inline int tune_key(int order, int n) {

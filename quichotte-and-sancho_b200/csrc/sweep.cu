@@ -1,13 +1,13 @@
 // sweep.cu -- the energy sweep (sweep / G_at_energy, src/scf.f90:280-415) as batched
 // kernels over the whole energy grid:
-//   dyson_bgj,      G^r(w) = [hbar w - H + (i/2hbar)(GammaL+GammaR) - Sigma^r(w)]^-1 by
-//   dyson_gj        in-place Gauss-Jordan elimination with partial pivoting for the orders
-//                   that do not fit in shared memory, one block per energy with the matrix in a
-//                   global workspace (invert_complex, common/linear_algebra.f90:58-88);
-//                   dyson_blk.cu has the smaller ones
+//   dyson_gj        G^r(w) = [hbar w - H + (i/2hbar)(GammaL+GammaR) - Sigma^r(w)]^-1 by
+//                   in-place Gauss-Jordan elimination with partial pivoting for orders above
+//                   256, one block per energy (invert_complex, common/linear_algebra.f90:58-88);
+//                   dyson_blk.cu and dyson_l2.cu have the smaller ones
 //   keldysh_scf2    G^< = G^r Sigma^< G^a on the active block as two complex GEMMs per
 //                   energy, written straight into the SCF vector with its diagonals
-//                   (modes M_INIT2 / M_SCF2, src/scf.f90:340-355)
+//                   (modes M_INIT2 / M_SCF2, src/scf.f90:340-355), for blocks above 256 states;
+//                   keldysh_sm.cu and keldysh_rows.cu have the smaller ones
 //   final_outputs   modes M_SCF1 / M_FINAL (src/scf.f90:357-410): on-site and intra-atom
 //                   blocks of G^<, Im G^r_ii, the current integrand
 // plus the reductions over energies (equal_time_lesser, gather_onsite, gather_atoms,
@@ -158,278 +158,6 @@ __global__ void __launch_bounds__(512) dyson_gj(DysonArgs a) {
             for (int idx = tid; idx < nA * nA; idx += nthr) {
                 int p = idx % nA, q = idx / nA;
                 G[idx] = M[a.act[p] + (size_t)a.act[q] * N];
-            }
-        } else {
-            zc *G = a.Gout + (size_t)(iw - a.iw0) * N * N;
-            for (int idx = tid; idx < N * N; idx += nthr) G[idx] = M[idx];
-        }
-        __syncthreads();
-    }
-}
-
-constexpr int GJ_B = 16;  // panel width of dyson_bgj = the k extent of one FP64 tensor-core MMA
-
-// 15 warps: one per 8-column tile of a 120-column matrix in the update, and 136 registers a
-// thread for the panel's register-resident rows
-constexpr int BGJ_THREADS = 480;
-
-// named barrier of the panel warps (ids 1.. are free; 0 is __syncthreads)
-__device__ __forceinline__ void panel_bar(int nthreads) { asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory"); }
-
-constexpr int BGJ_MAXN_GM = 256;
-
-// Blocked Gauss-Jordan inversion of orders 121..256 with the matrix column-major in the block's slot
-// of a global workspace (the working set of the concurrent blocks stays largely in L2, and every
-// access of the update is a 128-byte run of 8 consecutive rows). Per panel
-// K = [k0, k0 + 16):
-//   panel   the panel warps (ceil(N/32) <= 8), thread i holding row i of the panel
-//           columns in registers: per column
-//           k the pivot search, the exchange of rows k and p (the panel part through shared
-//           memory, the rest of the two rows in place), and the elimination restricted to
-//           the panel columns; two 128-thread barriers per column
-//   update  every warp owns 16 x 8 column tiles j outside K: A[i, j] += A[i, K] A[K, j] for
-//           rows i outside K, then A[K, j] = A[K, K] A[K, j], complex products on the FP64
-//           tensor cores; the warp reads its A[K, j] fragment before it rewrites those rows,
-//           so no block barrier separates the two
-// The row interchanges are undone by column interchanges in reverse order at the end.
-// NT = 480 (15 warps, one block per SM) or NT = 256 (8 warps, two blocks per SM: one block's
-// latency-bound panel overlaps the other's update).
-template <int NT>
-__global__ void __launch_bounds__(NT, NT <= 256 ? 2 : 1) dyson_bgj_t(DysonArgs a) {
-    constexpr int PWM = 8;  // panel warps at most
-    const int N = a.N;
-    __shared__ unsigned char perm[BGJ_MAXN_GM];
-    __shared__ unsigned long long cand_k[PWM];  // each panel warp's pivot key (0: no row searched)
-    __shared__ int cand_i[PWM];
-    __shared__ zc cand_row[PWM][GJ_B];  // each panel warp's pivot candidate row (panel part)
-    __shared__ zc krow[GJ_B];           // the panel part of row k before the exchange
-    __shared__ int first_zero_s;
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int mtiles = (N + 15) / 16, ntiles = (N + 7) / 8;
-    const int npw = (N + 31) / 32;  // panel warps
-
-    for (int iw = a.iw0 + blockIdx.x; iw < a.iw1; iw += gridDim.x) {
-        zc *M = a.inplace ? a.Gout + (size_t)(iw - a.iw0) * N * N : a.ws + (size_t)blockIdx.x * N * N;
-        if (a.Ain && a.inplace) {  // the matrix is there
-        } else if (a.Ain) {
-            const zc *A = a.Ain + (size_t)(iw - a.iw0) * N * N;
-            for (int idx = tid; idx < N * N; idx += nthr) M[idx] = A[idx];
-        } else {
-            const double w = a.omega[iw];
-            const zc *SR = a.Sig + iw * a.sig_ld;
-#pragma unroll 4
-            for (int idx = tid; idx < N * N; idx += nthr) {
-                int i = idx % N, j = idx / N;
-                zc v = a.Hemb[idx];
-                if (a.use_sigma) {
-                    int pi = a.pos[i], pj = a.pos[j];
-                    if (pi >= 0 && pj >= 0) {
-                        zc sg = a.Sig1[idx];
-                        if (a.order2) sg = sg + sig_r(SR, pi, pj);
-                        v = v - sg;
-                    }
-                }
-                if (i == j) v.x += w;
-                M[i + j * N] = v;
-            }
-        }
-        if (tid == 0) first_zero_s = 0;
-        bool singular = false;
-        __syncthreads();
-        for (int k0 = 0; k0 < N; k0 += GJ_B) {
-            const int kb = min(GJ_B, N - k0);
-            // ---- panel
-            if (warp < npw) {
-                const int i = tid;  // this thread's row
-                // R[j] holds panel column (c + j) mod 16 at step c: the current column is always
-                // R[0] and the step loop need not be unrolled (padding columns stay zero)
-                zc R[GJ_B];
-#pragma unroll
-                for (int c = 0; c < GJ_B; c++) R[c] = (i < N && c < kb) ? M[i + (k0 + c) * N] : zc{0, 0};
-#pragma unroll 1
-                for (int c = 0; c < kb; c++) {
-                    const int k = k0 + c;
-                    const bool valid = (i >= k && i < N);
-                    // every thread prepares 1 / R[0] in case its row becomes the pivot row; the
-                    // division overlaps the pivot search
-                    const bool z = (R[0].x == 0.0 && R[0].y == 0.0);
-                    zc inv_own{0.0, 0.0};
-                    if (!singular && !z) {
-                        const double id = 1.0 / fma(R[0].x, R[0].x, R[0].y * R[0].y);
-                        inv_own = zc{R[0].x * id, -R[0].y * id};
-                    }
-                    // pivot search: the warp maximum of cabs1, then its lowest lane (first
-                    // maximum). cabs1 >= 0, so its bit pattern orders like its value: two
-                    // integer warp reductions (high word + 1, 0 for rows not searched; then the
-                    // low word among the lanes holding the maximal high word) replace a chain
-                    // of FP64 shuffles
-                    // (a NaN is an ordinary large key here, so a pivot row is always found)
-                    const double v = valid ? cabs1(R[0]) : 0.0;
-                    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-                    const unsigned hk = valid ? min((unsigned)(bits >> 32), 0xfffffffeu) + 1u : 0u, lk = (unsigned)bits;
-                    const unsigned mh = __reduce_max_sync(0xffffffffu, hk);
-                    const unsigned ml = __reduce_max_sync(0xffffffffu, hk == mh ? lk : 0u);
-                    const unsigned bal = __ballot_sync(0xffffffffu, valid && hk == mh && lk == ml);
-                    const int wl = bal ? __ffs(bal) - 1 : 32;
-                    if (lane == 0) {
-                        cand_k[warp] = ((unsigned long long)mh << 32) | ml;
-                        cand_i[warp] = bal ? 32 * warp + wl : N;
-                    }
-                    if (lane == wl) {  // this warp's candidate publishes its scaled row
-#pragma unroll
-                        for (int j = 0; j < GJ_B; j++) cand_row[warp][j] = (j == 0) ? inv_own : R[j] * inv_own;
-                    }
-                    if (i == k) {
-#pragma unroll
-                        for (int j = 0; j < GJ_B; j++) krow[j] = R[j];
-                    }
-                    panel_bar(32 * npw);
-                    // the largest key; on a tie the lower warp (lower rows) wins, as the first
-                    // maximum. The warp holding row k has a key > 0, so p is a row in [k, N).
-                    unsigned long long bk = cand_k[0];
-                    int wb = 0;
-                    for (int q = 1; q < npw; q++) {
-                        const unsigned long long ck = cand_k[q];
-                        if (ck > bk) {
-                            bk = ck;
-                            wb = q;
-                        }
-                    }
-                    const int p = cand_i[wb];
-                    if (bk == (1ull << 32) && !singular) {  // cabs1 of the pivot is +0
-                        singular = true;           // every panel thread sees the same pivot
-                        if (tid == 0) first_zero_s = k + 1;
-                    }
-                    if (tid == 0) perm[k] = (unsigned char)p;
-                    // rows k and p exchange their panel parts: row p takes the old row k
-                    if (p != k && i == p) {
-#pragma unroll
-                        for (int j = 0; j < GJ_B; j++) R[j] = krow[j];
-                    }
-                    // eliminate with the scaled pivot row S (S_0 = 1 / pivot), then rotate the
-                    // window by one column
-                    const zc *S = cand_row[wb];
-                    const zc f = R[0];
-                    const bool pr = (i == k);
-                    zc first;
-#pragma unroll
-                    for (int j = 0; j < GJ_B; j++) {
-                        const zc r = S[j];
-                        zc tt;
-                        if (pr) {
-                            tt = r;
-                        } else {
-                            tt = (j == 0) ? zc{0.0, 0.0} : R[j];
-                            tt.x = fma(-f.x, r.x, tt.x);
-                            tt.x = fma(f.y, r.y, tt.x);
-                            tt.y = fma(-f.x, r.y, tt.y);
-                            tt.y = fma(-f.y, r.x, tt.y);
-                        }
-                        if (j == 0) first = tt;
-                        else R[j - 1] = tt;
-                    }
-                    R[GJ_B - 1] = first;
-                    // the rest of rows k and p (thread i moves column i, its own earlier
-                    // exchanges first)
-                    if (p != k && i < N && (i < k0 || i >= k0 + kb)) {
-                        zc tt = M[k + i * N];
-                        M[k + i * N] = M[p + i * N];
-                        M[p + i * N] = tt;
-                    }
-                    panel_bar(32 * npw);  // cand_row and krow are rewritten by the next column
-                }
-                // after kb steps R[j] holds column (kb + j) mod 16
-                if (i < N) {
-#pragma unroll
-                    for (int j = 0; j < GJ_B; j++) {
-                        const int c = (kb + j) & (GJ_B - 1);
-                        if (c < kb) M[i + (k0 + c) * N] = R[j];
-                    }
-                }
-            }
-            __syncthreads();
-            // ---- update, one 16 x 8 column tile at a time per warp
-            for (int ct = warp; ct < ntiles; ct += nwarps) {
-                const int j0 = 8 * ct;
-                if (j0 >= k0 && j0 + 8 <= k0 + kb) continue;  // the whole column tile is in K
-                double br[4], bi[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int kr = t4 + 4 * q, c = j0 + g;
-                    zc v = (kr < kb && c < N) ? M[k0 + kr + c * N] : zc{0, 0};
-                    br[q] = v.x;
-                    bi[q] = v.y;
-                }
-#pragma unroll 1
-                for (int rt = 0; rt < mtiles; rt++) {
-                    const int i0 = 16 * rt;
-                    if (i0 >= k0 && i0 + 16 <= k0 + kb) continue;  // the whole row tile is in K
-                    double ar[8], ai[8], cr[4], ci[4];
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const int r = i0 + g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
-                        zc v = (r < N && c < kb) ? M[r + (k0 + c) * N] : zc{0, 0};
-                        ar[q] = v.x;
-                        ai[q] = v.y;
-                    }
-                    bool own[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                        own[q] = r < N && c < N && (r < k0 || r >= k0 + kb) && (c < k0 || c >= k0 + kb);
-                        zc v = own[q] ? M[r + c * N] : zc{0, 0};
-                        cr[q] = v.x;
-                        ci[q] = v.y;
-                    }
-                    zmma16816(cr, ci, ar, ai, br, bi);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = i0 + g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                        if (own[q]) M[r + c * N] = zc{cr[q], ci[q]};
-                    }
-                }
-                // the pivot rows
-                double ar[8], ai[8], cr[4] = {0, 0, 0, 0}, ci[4] = {0, 0, 0, 0};
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int r = g + 8 * (q & 1), c = t4 + 4 * (q >> 1);
-                    zc v = (r < kb && c < kb) ? M[k0 + r + (k0 + c) * N] : zc{0, 0};
-                    ar[q] = v.x;
-                    ai[q] = v.y;
-                }
-                zmma16816(cr, ci, ar, ai, br, bi);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int r = g + 8 * (q >> 1), c = j0 + 2 * t4 + (q & 1);
-                    if (r < kb && c < N && (c < k0 || c >= k0 + kb)) M[k0 + r + c * N] = zc{cr[q], ci[q]};
-                }
-            }
-            __syncthreads();
-        }
-        // undo the row interchanges by column interchanges in reverse order
-        if (tid < N) {
-            for (int k = N - 1; k >= 0; k--) {
-                int p = perm[k];
-                if (p != k) {
-                    zc tt = M[tid + k * N];
-                    M[tid + k * N] = M[tid + p * N];
-                    M[tid + p * N] = tt;
-                }
-            }
-        }
-        __syncthreads();
-        if (first_zero_s && tid == 0) {
-            if (a.info) atomicMin(a.info, iw + 1);
-            if (a.info_each) a.info_each[iw - a.iw0] = first_zero_s;
-        }
-        if (a.inplace) {
-        } else if (a.out_mode == 0) {
-            const int nA = a.nA;
-            zc *G = a.Gout + (size_t)iw * nA * nA;
-            for (int idx = tid; idx < nA * nA; idx += nthr) {
-                int p = idx % nA, q = idx / nA;
-                G[idx] = M[a.act[p] + a.act[q] * N];
             }
         } else {
             zc *G = a.Gout + (size_t)(iw - a.iw0) * N * N;
@@ -745,36 +473,29 @@ int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref) {
 // ---------------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------------
-// the blocked kernel with the matrix in the global workspace: orders above the shared-memory limit
-static bool use_bgj(int N) { return !dyson_fits_smem(N) && N <= BGJ_MAXN_GM; }
-constexpr int BGJ_THREADS2 = 256;  // the two-blocks-per-SM form
-constexpr int GJ_THREADS = 512;    // the unblocked kernel, N <= 512
+constexpr int GJ_THREADS = 512;  // the unblocked kernel, N <= 512
 
-// orders above the shared-memory limit on at most nblocks blocks; variant as in the autotuner
-static void dyson_gm(cudaStream_t st, const DysonArgs &a, int variant, int nblocks) {
-    if (use_bgj(a.N) && variant == DYSON_BLOCKED2)
-        dyson_bgj_t<BGJ_THREADS2><<<std::min(nblocks, 2 * 148), BGJ_THREADS2, 0, st>>>(a);
-    else if (use_bgj(a.N) && variant == DYSON_BLOCKED)  // the concurrent matrices (148 x N^2 x 16 B) stay mostly in L2
-        dyson_bgj_t<BGJ_THREADS><<<std::min(nblocks, 148), BGJ_THREADS, 0, st>>>(a);
-    else
-        dyson_gj<<<nblocks, GJ_THREADS, 0, st>>>(a);
+// Up to 80 states several matrices share an SM's memory (dyson_blk: 80 x 4000 1.31 ms, dyson_l2 1.22, but
+// 50 x 4000 0.46 and 0.52). From there to DYSON_SMEM_MAXN dyson_blk holds one matrix an SM, the faster
+// form while there is one for each SM at most (96 x 148 0.110 ms, dyson_l2 0.136; 120 x 200 0.288 and
+// 0.272, 96 x 4000 2.77 and 1.60); it is also the one that needs no workspace when G is a part of the matrix.
+static int run_dyson(cudaStream_t st, const DysonArgs &a) {
+    if (a.N <= 80 || (dyson_fits_smem(a.N) && (!a.inplace || a.iw1 - a.iw0 <= 148))) return launch_dyson_blk(st, a);
+    if (dyson_l2_fits(a.N)) return launch_dyson_l2(st, a);
+    dyson_gj<<<std::min(a.iw1 - a.iw0, DYSON_L2_SLOTS), GJ_THREADS, 0, st>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : -(int)e;
 }
 
-static int launch_dyson(qs_handle *h, DysonArgs &a, int variant) {
+static int launch_dyson(qs_handle *h, DysonArgs &a) {
     int pi = prof_begin(h, K_DYSON);
-    int rc = 0;
-    if (dyson_fits_smem(a.N)) {
-        rc = launch_dyson_blk(h->stream, a);
-    } else {
-        // the matrices are built and inverted where G goes if G has their order: one copy less, and no
-        // slot that the next matrix of the block waits for (192 x 192: 9.2 -> 11.3 TFLOP/s)
-        a.inplace = a.out_mode == 1 || a.nA == a.N;
-        a.ws = h->d_Gws;
-        dyson_gm(h->stream, a, variant, std::min(a.iw1 - a.iw0, 2 * 148));
-    }
+    // in global memory the matrices are built and inverted where G goes if G has their order: one
+    // copy less, and no slot that the next matrix of the block waits for
+    a.inplace = a.out_mode == 1 || a.nA == a.N;
+    a.ws = h->d_Gws;
+    const int rc = run_dyson(h->stream, a);
     prof_end(h, pi);
     QS_CUDA(h, (cudaError_t)-rc);
-    QS_CUDA(h, cudaGetLastError());
     return 0;
 }
 
@@ -789,10 +510,7 @@ int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, i
     a.info_each = d_each;
     a.inplace = 1;
     count_launch();
-    if (dyson_fits_smem(N)) return launch_dyson_blk(st, a);
-    dyson_gm(st, a, DYSON_BLOCKED2, std::min(batch, 2 * 148));
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : -(int)e;
+    return run_dyson(st, a);
 }
 
 // sweep(mode) over all energies (src/scf.f90:280-290).
@@ -819,16 +537,10 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         a.iw1 = n;
         a.out_mode = 0;
         a.Gout = h->d_G;
-        {
-            // one form in shared memory; above, the two blocked ones on the workspace, and beyond
-            // their order the unblocked one
-            int cand[2], nc = 0;
-            if (dyson_fits_smem(N) || use_bgj(N)) cand[nc++] = DYSON_BLOCKED;
-            if (use_bgj(N)) cand[nc++] = DYSON_BLOCKED2;
-            if (!nc) cand[nc++] = DYSON_UNBLOCKED;
-            rc = tune_launch(h, TUNE_DYSON, tune_key(N, n), cand, nc, cand[0], [&](int v) { return launch_dyson(h, a, v); });
-            if (rc) return rc;
-        }
+        // one form per order
+        const int form = dyson_l2_fits(N) ? DYSON_BLOCKED : DYSON_UNBLOCKED;
+        rc = tune_launch(h, TUNE_DYSON, tune_key(N, n), &form, 1, form, [&](int) { return launch_dyson(h, a); });
+        if (rc) return rc;
         KeldyshArgs k{};
         k.nA = nA;
         k.n = n;
@@ -877,7 +589,7 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         a.iw1 = iw1;
         a.out_mode = 1;
         a.Gout = h->d_G;
-        if ((rc = launch_dyson(h, a, DYSON_BLOCKED))) return rc;
+        if ((rc = launch_dyson(h, a))) return rc;
         FinalArgs f{};
         f.N = N;
         f.nS = h->nS;
