@@ -1,4 +1,5 @@
-// keldysh_rows.cu -- the Keldysh step of the sweep (modes M_INIT2 / M_SCF2, src/scf.f90:333-355) for
+// keldysh_rows.cu -- products with the rows of T = G^r SL in shared memory: the outputs of the final sweep
+// (final_rows, below) and the Keldysh step of the sweep (modes M_INIT2 / M_SCF2, src/scf.f90:333-355) for
 // active blocks of 81 to 256 states: G^< = G^r SL G^r^dagger with SL = i (f_L Gamma_L + f_R Gamma_R) +
 // Sigma2^<, written with G^r into the packed vector minus x.
 //
@@ -96,21 +97,18 @@ __device__ __forceinline__ void panel_product(const zc *P, unsigned kmask, const
     }
 }
 
-__global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned char contact[256];  // 1 + index of a contact state, 0 for the others
-    const int N = a.nA, tid = threadIdx.x, nthr = blockDim.x;
+// The rows r0 .. r0 + 31 of T = G SL in the panel P ((r, k) at at(r, k, RB)), with hook() called while it holds
+// those of G. kmask: the k steps in which T has columns other than zero; cr, ci are scratch.
+template <class HOOK>
+__device__ __forceinline__ void rows_of_T(zc *P, unsigned char (&contact)[256], int N, int r0, const zc *G, const zc *SL,
+                                          const zc *GamLs, const zc *GamRs, const int *cidx, int nc, double fL, double fR,
+                                          unsigned &kmask, double (&cr)[CT][2][4], double (&ci)[CT][2][4], HOOK hook) {
+    const int tid = threadIdx.x, nthr = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, nw = nthr >> 5;
-    const int nk = (N + 7) / 8, nrb = (N + RB - 1) / RB;
-    const int iw = blockIdx.x / nrb, r0 = RB * (blockIdx.x % nrb), rows = min(RB, N - r0), mrows = (rows + 15) / 16;
-    const bool corr = a.nc >= 0 && a.nc <= NC_CORR;  // else the leads enter as a matrix
-    zc *P = (zc *)smem_raw;                           // rows r0 .. r0 + 31 of G^r, then of T: (r, k) at at(r, k, RB)
-    const zc *G = a.G + (size_t)iw * N * N;
-    const zc *SL = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
-    const double w = a.omega[iw];
-    const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
+    const int nk = (N + 7) / 8, rows = min(RB, N - r0), mrows = (rows + 15) / 16;
+    const bool corr = nc >= 0 && nc <= NC_CORR;  // else the leads enter as a matrix
     auto lead = [&](int k, int j) {
-        const zc gl = a.GamLs[k + j * N], gr = a.GamRs[k + j * N];
+        const zc gl = GamLs[k + j * N], gr = GamRs[k + j * N];
         return zc{-(fL * gl.y + fR * gr.y), fL * gl.x + fR * gr.x};
     };
     for (int k = warp; k < 8 * nk; k += nw) {
@@ -120,39 +118,17 @@ __global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     for (int i = tid; i < 256; i += nthr) contact[i] = 0;
     __syncthreads();
-    if (corr && tid < a.nc) contact[a.cidx[tid]] = (unsigned char)(tid + 1);
+    if (corr && tid < nc) contact[cidx[tid]] = 1;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    double *blk = a.out + (size_t)iw * a.nblk;
-    const double *xb = a.xsub ? a.xsub + (size_t)iw * a.nblk : nullptr;
-    // ---- G^r minus x, by 2x2 site blocks: a warp takes the rows' 16 blocks of a site column as two
-    // halves, four columns at a time
-    for (int J0 = warp; J0 < N / 2; J0 += 4 * nw) {
-        zc xv[8];
-        int o[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int J = J0 + (u >> 1) * nw, i = 16 * (u & 1) + 2 * (lane >> 2) + (lane & 1), j = 2 * J + ((lane >> 1) & 1);
-            o[u] = i < rows && J < N / 2 ? dl_r(r0 + i, j) : -1;
-            xv[u] = xb && o[u] >= 0 ? *(const zc *)(xb + o[u]) : zc{0, 0};
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (o[u] < 0) continue;
-            const int J = J0 + (u >> 1) * nw, i = 16 * (u & 1) + 2 * (lane >> 2) + (lane & 1), j = 2 * J + ((lane >> 1) & 1);
-            const zc v = P[at(i, j, RB)];
-            *(zc *)(blk + o[u]) = v - xv[u];
-            if (r0 + i == j && a.gRd) a.gRd[(size_t)iw * N + j] = v;
-        }
-    }
-    // ---- T = G SL; the k steps: all, or those with a contact if T has only their columns
+    hook();
+    // the k steps: all, or those with a contact if T has only their columns
     const unsigned all = nk == 32 ? 0xffffffffu : (1u << nk) - 1;
-    unsigned kmask = all;
+    kmask = all;
     if (!SL && corr) {
         kmask = 0;
-        for (int q = 0; q < a.nc; q++) kmask |= 1u << (a.cidx[q] >> 3);
+        for (int q = 0; q < nc; q++) kmask |= 1u << (cidx[q] >> 3);
     }
-    double cr[CT][2][4], ci[CT][2][4];
     {
         int mt[CT];
 #pragma unroll
@@ -180,8 +156,8 @@ __global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
             for (int e = 0; e < 2; e++) {
                 const int c = 8 * (warp + u * nw) + 2 * t4 + e;
                 if (c >= N || !contact[c]) continue;
-                for (int q = 0; q < a.nc; q++) {
-                    const int k = a.cidx[q];
+                for (int q = 0; q < nc; q++) {
+                    const int k = cidx[q];
                     const zc l = lead(k, c);
 #pragma unroll
                     for (int m = 0; m < 2; m++)
@@ -205,6 +181,45 @@ __global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
                 for (int q = 0; q < 4; q++)
                     P[at(16 * m + 8 * (q >> 1) + g, 8 * (warp + u * nw) + 2 * t4 + (q & 1), RB)] = zc{cr[u][m][q], ci[u][m][q]};
     __syncthreads();
+}
+
+__global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned char contact[256];  // 1 for a contact state
+    const int N = a.nA, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, nw = blockDim.x >> 5;
+    const int nk = (N + 7) / 8, nrb = (N + RB - 1) / RB;
+    const int iw = blockIdx.x / nrb, r0 = RB * (blockIdx.x % nrb), rows = min(RB, N - r0), mrows = (rows + 15) / 16;
+    zc *P = (zc *)smem_raw;
+    const zc *G = a.G + (size_t)iw * N * N;
+    const double w = a.omega[iw];
+    double *blk = a.out + (size_t)iw * a.nblk;
+    const double *xb = a.xsub ? a.xsub + (size_t)iw * a.nblk : nullptr;
+    // G^r minus x, by 2x2 site blocks: a warp takes the rows' 16 blocks of a site column as two
+    // halves, four columns at a time
+    auto pack = [&]() {
+        for (int J0 = warp; J0 < N / 2; J0 += 4 * nw) {
+            zc xv[8];
+            int o[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int J = J0 + (u >> 1) * nw, i = 16 * (u & 1) + 2 * (lane >> 2) + (lane & 1), j = 2 * J + ((lane >> 1) & 1);
+                o[u] = i < rows && J < N / 2 ? dl_r(r0 + i, j) : -1;
+                xv[u] = xb && o[u] >= 0 ? *(const zc *)(xb + o[u]) : zc{0, 0};
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (o[u] < 0) continue;
+                const int J = J0 + (u >> 1) * nw, i = 16 * (u & 1) + 2 * (lane >> 2) + (lane & 1), j = 2 * J + ((lane >> 1) & 1);
+                const zc v = P[at(i, j, RB)];
+                *(zc *)(blk + o[u]) = v - xv[u];
+                if (r0 + i == j && a.gRd) a.gRd[(size_t)iw * N + j] = v;
+            }
+        }
+    };
+    unsigned kmask;
+    double cr[CT][2][4], ci[CT][2][4];
+    rows_of_T(P, contact, N, r0, G, a.Sig ? a.Sig + iw * a.sig_ld : nullptr, a.GamLs, a.GamRs, a.cidx, a.nc,
+              fermi_d(w, a.V, a.mu, a.beta), fermi_d(w, 0.0, a.mu, a.beta), kmask, cr, ci, pack);
     // ---- G^< = T G^+ in the column tiles from the diagonal on
     int mt[CT];
 #pragma unroll
@@ -254,15 +269,106 @@ __global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
         }
 }
 
+// mode M_FINAL (src/scf.f90:357-410) where every state is active: the blocks of G^< that the outputs need are dot
+// products of rows of T and of G, four lanes each. The block whose rows hold the left contact states does the
+// current integrand. Per launch, against one block an energy with CUDA-core tiles and T in global scratch:
+// 24 states x 32768 energies 0.98 -> 0.53 ms, 40 x 5003 0.65 -> 0.27, 120 x 4096 5.7 -> 2.5, 192 x 1201 6.7 -> 3.0.
+__global__ void __launch_bounds__(512, 1) final_rows(FinalArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned char contact[256];
+    __shared__ double Xs[32 * 32];  // nCL <= 32 (checked in qs_create)
+    const int N = a.N, tid = threadIdx.x, nthr = blockDim.x, nrb = (N + RB - 1) / RB;
+    const int iw = a.iw0 + blockIdx.x / nrb, r0 = RB * (blockIdx.x % nrb), rows = min(RB, N - r0);
+    zc *P = (zc *)smem_raw;
+    const zc *G = a.G + (size_t)(iw - a.iw0) * N * N;
+    const double w = a.omega[iw];
+    const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
+    unsigned kmask;
+    double cr[CT][2][4], ci[CT][2][4];
+    rows_of_T(P, contact, N, r0, G, a.Sig ? a.Sig + iw * sig_stride(N) : nullptr, a.GamLs, a.GamRs, a.cidx, a.nc, fL, fR,
+              kmask, cr, ci, [&]() {
+                  for (int i = tid; i < rows; i += nthr) a.dosd[(size_t)iw * N + r0 + i] = P[at(i, r0 + i, RB)].y;
+              });
+    // G^<(r, c), r = r0 + i; all four lanes of a group get it
+    const int sub = tid & 3;
+    auto dot = [&](int i, int c) {
+        zc v{0, 0};
+#pragma unroll 4
+        for (int q = sub; q < N; q += 4) cfma_conj(v, P[at(i, q, RB)], G[c + q * N]);
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        return v;
+    };
+    // the groups of a warp stay together: the last ones repeat an entry
+    auto each = [&](int count, auto entry) {
+        for (int t0 = tid >> 5 << 3; t0 < count; t0 += nthr >> 2) {
+            const int t = t0 + ((tid & 31) >> 2);
+            entry(min(t, count - 1), t < count && sub == 0);
+        }
+    };
+    each(2 * rows, [&](int t, bool keep) {
+        const int s = (r0 >> 1) + (t >> 2), aa = t & 1, bb = (t >> 1) & 1;
+        const zc v = dot(2 * (t >> 2) + aa, 2 * s + bb);
+        if (keep) a.onsL[(size_t)iw * 4 * a.N_sites + 4 * s + aa + 2 * bb] = v;
+    });
+    if (a.atomL) {
+        for (int k = 0; k < a.N_atoms; k++) {
+            const int lo = 2 * (a.atom_first[k] - 1), m = 2 * a.atom_norb[k];
+            const int b0 = max(lo, r0), b1 = min(lo + m, r0 + rows);  // its rows in this block
+            if (b0 >= b1) continue;
+            each((b1 - b0) * m, [&](int t, bool keep) {
+                const int r = b0 + t % (b1 - b0), c = lo + t / (b1 - b0);
+                const zc v = dot(r - r0, c);
+                if (keep) a.atomL[(size_t)iw * a.atomL_ld + a.atom_off[k] + (r - lo) + (c - lo) * m] = v;
+            });
+        }
+    }
+    // current integrand through the left lead (src/scf.f90:390-409)
+    const int nCL = a.nCL;
+    if (nCL == 0 ? r0 != 0 : a.cl[0] / RB != r0 / RB) return;
+    if (nCL > 0)
+        each(nCL * nCL, [&](int t, bool keep) {
+            const int k = t % nCL, aa = t / nCL, ck = a.cl[k], ca = a.cl[aa];
+            const zc glc = dot(ck - r0, ca), gg = glc + G[ck + ca * N] - conj(G[ca + ck * N]);
+            const zc x{(fL - 1.0) * glc.x - fL * gg.x, (fL - 1.0) * glc.y - fL * gg.y};
+            const zc m = a.GamLcl[aa + k * nCL] * x;
+            if (keep) Xs[t] = -m.y;  // Re i GammaL x
+        });
+    __syncthreads();
+    if (tid < 2) {  // spin up: even states
+        double tr = 0;
+        for (int aa = 0; aa < nCL; aa++)
+            if ((a.cl[aa] & 1) == tid)
+                for (int k = 0; k < nCL; k++) tr += Xs[k + aa * nCL];
+        (tid ? a.trD : a.trU)[iw] = tr / (2.0 * PI);
+    }
+}
+
 }  // namespace
+
+static int rows_threads(int N) { return 32 * (((N + 7) / 8 + CT - 1) / CT); }
+static size_t rows_smem(int N) { return sizeof(zc) * RB * 8 * ((N + 7) / 8); }
+
 
 bool keldysh_rows_fits(int nA) { return nA <= 256; }
 
 int launch_keldysh_rows(qs_handle *h, const KeldyshArgs &k) {
-    const int nk = (k.nA + 7) / 8, nrb = (k.nA + RB - 1) / RB;
+    const int nrb = (k.nA + RB - 1) / RB;
     QS_CUDA(h, smem_cap((const void *)keldysh_rows));
     int pi = prof_begin(h, K_KELDYSH);
-    keldysh_rows<<<k.n * nrb, 32 * ((nk + CT - 1) / CT), sizeof(zc) * RB * 8 * nk, h->stream>>>(k);
+    keldysh_rows<<<k.n * nrb, rows_threads(k.nA), rows_smem(k.nA), h->stream>>>(k);
+    prof_end(h, pi);
+    QS_CUDA(h, cudaGetLastError());
+    return 0;
+}
+
+int launch_final_rows(qs_handle *h, const FinalArgs &f) {
+    QS_CUDA(h, smem_cap((const void *)final_rows));
+    int pi = prof_begin(h, K_FINAL);
+    final_rows<<<(f.iw1 - f.iw0) * ((f.N + RB - 1) / RB), rows_threads(f.N), rows_smem(f.N), h->stream>>>(f);
     prof_end(h, pi);
     QS_CUDA(h, cudaGetLastError());
     return 0;

@@ -293,12 +293,28 @@ struct KeldyshArgs {
     const int *cidx;    // the contact states: rows/columns where GamLs or GamRs is non-zero
     int nc;             // their number (-1: not known)
 };
+// arguments of the per-energy outputs (sweep modes M_SCF1 / M_FINAL)
+struct FinalArgs {
+    int N, nS, nA, nCL, N_sites, N_atoms, iw0, iw1, mode;
+    const zc *G;  // full G per energy of the chunk
+    const int *sup, *act, *pos, *cl, *site_int, *atom_first, *atom_norb, *atom_off;
+    const zc *GamLs, *GamRs, *GamLcl, *Sig;
+    const double *omega;
+    double V, mu, beta;
+    zc *Tws;
+    double *dosd, *trU, *trD;
+    zc *onsL, *atomL, *gRd, *gLd;
+    int atomL_ld;
+    const int *cidx;  // the contact states, as in KeldyshArgs
+    int nc;
+};
 // the Keldysh step with both operands in shared memory (keldysh_sm.cu): nA <= 80
 int launch_keldysh_sm(qs_handle *h, const KeldyshArgs &k);
 bool keldysh_sm_fits(int nA);
 // the same by blocks of 32 rows (keldysh_rows.cu): nA <= 256
 int launch_keldysh_rows(qs_handle *h, const KeldyshArgs &k);
 bool keldysh_rows_fits(int nA);
+int launch_final_rows(qs_handle *h, const FinalArgs &f);
 // the FP32-phase Keldysh step of a QS_PREC_MIXED solve on the fifth-generation tensor cores
 // (keldysh_tf32.cu): 32 <= nA <= 128; returns -1 for other sizes
 int launch_keldysh_tf32(qs_handle *h, const KeldyshArgs &k);

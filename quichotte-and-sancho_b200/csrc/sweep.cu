@@ -279,19 +279,6 @@ __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
     }
 }
 
-struct FinalArgs {
-    int N, nS, nA, nCL, N_sites, N_atoms, iw0, iw1, mode;
-    const zc *G;  // full G per energy of the chunk
-    const int *sup, *act, *pos, *cl, *site_int, *atom_first, *atom_norb, *atom_off;
-    const zc *GamLs, *GamRs, *GamLcl, *Sig;
-    const double *omega;
-    double V, mu, beta;
-    zc *Tws;
-    double *dosd, *trU, *trD;
-    zc *onsL, *atomL, *gRd, *gLd;
-    int atomL_ld;
-};
-
 // modes M_SCF1 and M_FINAL (src/scf.f90:357-410)
 __global__ void __launch_bounds__(256) final_outputs(FinalArgs a) {
     __shared__ zc sA[TB * TK], sB[TB * TK];
@@ -513,6 +500,12 @@ int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, i
     return run_dyson(st, a);
 }
 
+// final_rows (keldysh_rows.cu): every state active, the left contact states within one block of 32 rows
+static bool final_rows_fits(const qs_handle *h, int mode) {
+    return mode == M_FINAL && h->order == 2 && h->nA == h->Norb && h->nS == h->Norb && keldysh_rows_fits(h->Norb) &&
+           (h->cl.empty() || h->cl.front() / 32 == h->cl.back() / 32);
+}
+
 // sweep(mode) over all energies (src/scf.f90:280-290).
 //   M_INIT2 / M_SCF2: output into d_out (SCF vector, DL); M_SCF2 subtracts d_x.
 //   M_SCF1 / M_FINAL: per-energy arrays of the handle.
@@ -626,6 +619,12 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         f.atomL_ld = h->has_atomL ? h->atom_off.back() : 0;
         f.gRd = h->d_gRd;
         f.gLd = h->d_gLd;
+        f.cidx = h->d_kd_cidx;
+        f.nc = h->kd_nc;
+        if (final_rows_fits(h, mode)) {
+            if ((rc = launch_final_rows(h, f))) return rc;
+            continue;
+        }
         size_t per = (size_t)Mrows * h->nS;
         int nb = (int)std::min<size_t>(std::min<size_t>(h->T_bytes / (sizeof(zc) * std::max<size_t>(per, 1)), 148 * 8),
                                        (size_t)(iw1 - iw0));
