@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(512, 1) keldysh_rows(KeldyshArgs a) {
     unsigned kmask;
     double cr[CT][2][4], ci[CT][2][4];
     rows_of_T(P, contact, N, r0, G, a.Sig ? a.Sig + iw * a.sig_ld : nullptr, a.GamLs, a.GamRs, a.cidx, a.nc,
-              fermi_d(w, a.V, a.mu, a.beta), fermi_d(w, 0.0, a.mu, a.beta), kmask, cr, ci, pack);
+              fermi_d(w, *a.V, a.mu, a.beta), fermi_d(w, 0.0, a.mu, a.beta), kmask, cr, ci, pack);
     // ---- G^< = T G^+ in the column tiles from the diagonal on
     int mt[CT];
 #pragma unroll

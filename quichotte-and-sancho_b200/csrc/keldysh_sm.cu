@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(MAXT, MINB) keldysh_sm(KeldyshArgs a) {
     for (int iw = blockIdx.x; iw < a.n; iw += gridDim.x) {
         const zc *Gg = a.G + (size_t)iw * N * N;
         const double w = a.omega[iw];
-        const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
+        const double fL = fermi_d(w, *a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
         for (int j = warp; j < N; j += nw)
             for (int i = lane; i < N; i += 32) cpa16(&G[at(i, j, N)], Gg + i + j * N);
         asm volatile("cp.async.commit_group;\n" ::: "memory");

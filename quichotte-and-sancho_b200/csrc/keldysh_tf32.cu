@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) keldysh_tf32(KeldyshArgs a) {
     for (int iw = blockIdx.x; iw < a.n && ok; iw += gridDim.x) {
         const zc *G = a.G + (size_t)iw * nfull;
         const double w = a.omega[iw];
-        const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
+        const double fL = fermi_d(w, *a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
         const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
         // ---- T = G SL: thread (m = tid % 128, quad tid / 128) stages A = G(m, k), thread
         // (n = tid / 4, quad tid % 4) stages B = SL(k, n)

@@ -17,6 +17,7 @@
 //   gRd, gLd           diagonals (n x nA complex) for the sanity check.
 //   onsL, dosd, atomL, trU, trD   final-sweep arrays, energy-major (reference layout).
 #pragma once
+#include <cmath>
 #include <functional>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -195,17 +196,17 @@ struct qs_handle {
     std::string err;
     size_t bytes_allocated = 0;
     std::vector<void *> allocs;
-    // CUDA graphs of the FP64 residual's launches, one per (x, F, V) the Broyden loop uses
-    // (x and F alternate between two buffers each): replayed instead of re-launching
+    // CUDA graphs of the FP64 residual's launches, one per (x, F) the Broyden loop uses (x and F
+    // alternate between two buffers each): replayed instead of re-launching, at every voltage
     struct ResidualGraph {
         const double *x = nullptr;
         double *F = nullptr;
-        double V = 0.0;
         cudaGraphExec_t exec = nullptr;
         int64_t launches = 0;  // kernels in the graph (added to the launch count per replay)
     };
-    ResidualGraph graphs[2];
-    int graph_next = 0;
+    ResidualGraph graphs[4];
+    double *d_V = nullptr;     // the voltage the Keldysh kernels read, and its value (NaN: none yet)
+    double V_dev = NAN;
     bool graphs_off = false;   // a capture failed: eager launches from then on
     int64_t graph_replays = 0;
 };
@@ -284,7 +285,8 @@ struct KeldyshArgs {
     int64_t sig_ld;  // its values per energy
     const zc *GamLs, *GamRs;
     const double *omega;
-    double V, mu, beta;
+    const double *V;    // in device memory: a captured step serves every voltage
+    double mu, beta;
     double *out;        // DL blocks (SCF vector)
     const double *xsub; // subtracted (F = out - x), or nullptr
     zc *gRd, *gLd;      // diagonals, or nullptr
@@ -357,6 +359,8 @@ int tune_launch(qs_handle *h, int kind, int size, const int *cand, int ncand, in
 // max |v_i| over a device vector (uses the Broyden reduction scratch)
 int vec_maxabs(qs_handle *h, const double *d_v, int64_t n, double &mx);
 int equal_time_lesser_sigma1(qs_handle *h, const double *d_x);
+// h->d_V = V, on the handle's stream
+int set_voltage(qs_handle *h, double V);
 enum SweepMode { M_INIT2 = 1, M_SCF2 = 2, M_SCF1 = 3, M_FINAL = 4 };
 // fp32: the FP32 phase of a QS_PREC_MIXED solve (M_SCF2 only: tensor-core Keldysh products)
 int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const double *d_x, bool fp32 = false);

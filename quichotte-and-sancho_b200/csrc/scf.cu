@@ -319,24 +319,31 @@ int residual2_launches(qs_handle *h, double V, const double *d_x, double *d_F, b
     return 0;
 }
 
-// The FP64 residual's launches replayed from a CUDA graph: captured at the second evaluation
-// of an (x, F, V) (the first one has made every autotuner decision of the sizes), replayed
-// afterwards. Not with per-launch profiling on (its events are per launch) nor in the FP32
-// phase; a capture that fails turns graphs off for the handle (eager launches, same results).
-int residual2_graphed(qs_handle *h, double V, const double *d_x, double *d_F) {
+// The FP64 residual's launches replayed from a CUDA graph: captured once per (x, F) of the handle, not
+// at the first evaluation of a solve (that one has made every autotuner decision of the sizes). Not
+// with per-launch profiling on (its events are per launch) nor in the FP32 phase; a capture that fails
+// turns graphs off for the handle (eager launches, same results). The voltage is read from device
+// memory: with it in the launches' arguments every solve at a new voltage captured two graphs (16 states
+// x 329 energies, 6 steps: 0.35 ms more a solve).
+qs_handle::ResidualGraph *residual2_graph(qs_handle *h, const double *d_x, const double *d_F) {
     for (auto &g : h->graphs)
-        if (g.exec && g.x == d_x && g.F == d_F && g.V == V) {
-            QS_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
-            count_launches(g.launches);
-            h->graph_replays++;
-            return 0;
-        }
-    auto &g = h->graphs[h->graph_next];
-    h->graph_next ^= 1;
-    if (g.exec) {
-        cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
+        if (g.exec && g.x == d_x && g.F == d_F) return &g;
+    return nullptr;
+}
+int residual2_graphed(qs_handle *h, double V, const double *d_x, double *d_F) {
+    int rc;
+    if ((rc = set_voltage(h, V))) return rc;  // (outside the graph)
+    if (auto *g = residual2_graph(h, d_x, d_F)) {
+        QS_CUDA(h, cudaGraphLaunch(g->exec, h->stream));
+        count_launches(g->launches);
+        h->graph_replays++;
+        return 0;
     }
+    qs_handle::ResidualGraph *slot = nullptr;
+    for (auto &g : h->graphs)
+        if (!g.exec && !slot) slot = &g;
+    if (!slot) return residual2_launches(h, V, d_x, d_F, false);
+    auto &g = *slot;
     const int64_t l0 = qs_kernel_launches();
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -344,7 +351,7 @@ int residual2_graphed(qs_handle *h, double V, const double *d_x, double *d_F) {
         h->graphs_off = true;
         return residual2_launches(h, V, d_x, d_F, false);
     }
-    int rc = residual2_launches(h, V, d_x, d_F, false);
+    rc = residual2_launches(h, V, d_x, d_F, false);
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
     const int64_t captured = qs_kernel_launches() - l0;
     if (rc == 0 && e == cudaSuccess && graph) e = cudaGraphInstantiate(&g.exec, graph, 0);
@@ -358,7 +365,6 @@ int residual2_graphed(qs_handle *h, double V, const double *d_x, double *d_F) {
     }
     g.x = d_x;
     g.F = d_F;
-    g.V = V;
     g.launches = captured;
     QS_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
     h->graph_replays++;
@@ -374,11 +380,11 @@ struct Residual2 : BroydenResidual {
     double best = HUGE_VAL;
     int since_best = 0;
     int last_prec = -1, cur_prec = -1;  // 1 = FP32 phase, 0 = FP64, of the last two evaluations
-    int evals64 = 0;                    // FP64 evaluations of this solve (the first runs eagerly)
+    int evals64 = 0;                    // FP64 evaluations of this solve (the first one captures nothing)
     bool precision_changed() const override { return last_prec >= 0 && last_prec != cur_prec; }
     int eval(const double *d_x, double *d_F, bool &abort, bool use32) {
         int rc;
-        const bool graph = !use32 && !h->prof_on && !h->graphs_off && evals64 > 0;
+        const bool graph = !use32 && !h->prof_on && !h->graphs_off && (evals64 > 0 || residual2_graph(h, d_x, d_F));
         if (!use32) evals64++;
         if (graph) {
             if ((rc = residual2_graphed(h, V, d_x, d_F))) return rc;
@@ -761,7 +767,7 @@ int qs_create(const qs_problem *p, qs_handle **out) {
     if (h->has_atomL && (rc = dalloc(h, (void **)&h->d_atomL, (size_t)n * h->atom_off.back() * zc_))) return rc;
     h->red_len = std::max<size_t>(broyden_red_len(), (size_t)2 * (4 * h->N_sites + h->atom_off.back() + 2 * N + 2 * nA + 8));
     if ((rc = dalloc(h, (void **)&h->d_red, h->red_len * 8)) || (rc = reduce_scratch(h))) return rc;
-    if ((rc = dalloc(h, (void **)&h->d_info, sizeof(int) * 2))) return rc;
+    if ((rc = dalloc(h, (void **)&h->d_info, sizeof(int) * 2)) || (rc = dalloc(h, (void **)&h->d_V, sizeof(double)))) return rc;
     int imax = INT_MAX;
     QS_CUDA(h, cudaMemcpyAsync(h->d_info, &imax, sizeof(int), cudaMemcpyHostToDevice, h->stream));
     // Gauss-Jordan workspace: for matrices that neither fit in shared memory nor can be inverted in

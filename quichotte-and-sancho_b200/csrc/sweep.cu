@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256) keldysh_scf2(KeldyshArgs a) {
     for (int iw = blockIdx.x; iw < a.n; iw += gridDim.x) {
         const zc *G = a.G + (size_t)iw * nfull;
         const double w = a.omega[iw];
-        const double fL = fermi_d(w, a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
+        const double fL = fermi_d(w, *a.V, a.mu, a.beta), fR = fermi_d(w, 0.0, a.mu, a.beta);
         const zc *SL2 = a.Sig ? a.Sig + iw * a.sig_ld : nullptr;
         // SL = i (fL GamL_s + fR GamR_s) / hbar  (+ Sigma2^<)   (src/scf.f90:333-336)
         auto ldSL = [&](int k, int j) {
@@ -500,6 +500,13 @@ int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, i
     return run_dyson(st, a);
 }
 
+int set_voltage(qs_handle *h, double V) {
+    if (V == h->V_dev) return 0;
+    QS_CUDA(h, cudaMemcpyAsync(h->d_V, &V, sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    h->V_dev = V;
+    return 0;
+}
+
 // final_rows (keldysh_rows.cu): every state active, the left contact states within one block of 32 rows
 static bool final_rows_fits(const qs_handle *h, int mode) {
     return mode == M_FINAL && h->order == 2 && h->nA == h->Norb && h->nS == h->Norb && keldysh_rows_fits(h->Norb) &&
@@ -544,7 +551,8 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
         k.GamLs = h->d_GamLs;
         k.GamRs = h->d_GamRs;
         k.omega = h->d_omega;
-        k.V = V;
+        if ((rc = set_voltage(h, V))) return rc;
+        k.V = h->d_V;
         k.mu = h->mu;
         k.beta = h->beta;
         k.out = d_out;
