@@ -484,7 +484,8 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
     const int nb = red_blocks(n);
     double *part = h->d_red, *fin = h->d_red + (size_t)RED_BLOCKS * 2 * MAXH;
     double *gam = fin + 2 * MAXH;
-    std::vector<double> hv(2 * MAXH + 4);
+    static_assert(PIN_BROYDEN >= 4 + 3 * MAXH, "norms, pairs, gamma");
+    double *norms = pin_broyden(h), *hv = norms + 4, *hgam = hv + 2 * MAXH;
     int nstored = 0, nh = 0;
     out = BroydenOut{};
     out.fmax = HUGE_VAL;
@@ -504,9 +505,14 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
         vec_norms<<<nb, RED_THREADS, 0, st>>>(d_F, want_dn ? d_Fold : nullptr, n, part, h->d_rcnt, fin);
         prof_end(h, pi);
         QS_CUDA(h, cudaGetLastError());
-        QS_CUDA(h, cudaMemcpyAsync(hv.data(), fin, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        QS_CUDA(h, cudaMemcpyAsync(norms, fin, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
         QS_CUDA(h, cudaStreamSynchronize(st));
-        double fmax = hv[0], rms = std::sqrt(hv[1]) / std::sqrt((double)n), fnorm = std::sqrt(hv[2]);
+        if ((rc = res.complete(abort))) return rc;
+        if (abort) {
+            out.aborted = true;
+            break;
+        }
+        double fmax = norms[0], rms = std::sqrt(norms[1]) / std::sqrt((double)n), fnorm = std::sqrt(norms[2]);
         out.fmax = fmax;
         out.log.push_back({its, fmax, rms, std::min(nstored, nhist)});
         if (fmax < tolf) {
@@ -533,7 +539,7 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
                                     (double *)d_hU, slot, nh_new, store, part, h->d_rcnt, fin);
             prof_end(h, pj);
             QS_CUDA(h, cudaGetLastError());
-            QS_CUDA(h, cudaMemcpyAsync(hv.data(), fin, 2 * nh_new * sizeof(double), cudaMemcpyDeviceToHost, st));
+            QS_CUDA(h, cudaMemcpyAsync(hv, fin, 2 * nh_new * sizeof(double), cudaMemcpyDeviceToHost, st));
             QS_CUDA(h, cudaStreamSynchronize(st));
         }
         if (store) {
@@ -556,7 +562,8 @@ int broyden_solve_dev(qs_handle *h, BroydenResidual &res, double *&d_x, double *
                 nh = 0;
                 out.n_resets++;
             } else {
-                QS_CUDA(h, cudaMemcpyAsync(gam, b.data(), nh * sizeof(double), cudaMemcpyHostToDevice, st));
+                std::copy(b.begin(), b.end(), hgam);
+                QS_CUDA(h, cudaMemcpyAsync(gam, hgam, nh * sizeof(double), cudaMemcpyHostToDevice, st));
             }
         }
         // x_new into the xold buffer, then rotate: xold <- x, x <- x_new, Fold <- F
@@ -580,7 +587,7 @@ int vec_maxabs(qs_handle *h, const double *d_v, int64_t n, double &mx) {
     vec_norms<<<nb, RED_THREADS, 0, h->stream>>>(d_v, nullptr, n, part, h->d_rcnt, fin);
     prof_end(h, pi);
     QS_CUDA(h, cudaGetLastError());
-    double hv[3];
+    double *hv = pin_broyden(h);
     QS_CUDA(h, cudaMemcpyAsync(hv, fin, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     QS_CUDA(h, cudaStreamSynchronize(h->stream));
     mx = hv[0];

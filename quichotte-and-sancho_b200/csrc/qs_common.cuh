@@ -186,6 +186,11 @@ struct qs_handle {
     double *d_rpart = nullptr;  // partial sums of the reductions over energies, REDUCE_PART doubles
     int *d_rcnt = nullptr;      // their arrival counters, REDUCE_CNT ints (zero between launches)
     int *d_info = nullptr;     // first singular energy (+1), 0 if none
+    // page-locked host memory of the values read in every step (host_scratch): 4 doubles a state
+    // (the sanity sums), then d_info, the norms, the Gram column and gamma
+    double *pin = nullptr;
+    int pin_states = 0;
+    std::vector<double> pin_own;  // in its place when the pool has no slot
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // host state
@@ -227,7 +232,15 @@ int dalloc(qs_handle *h, void **p, size_t bytes);
 // scratch of the reductions over energies: one partial per block for at most REDUCE_BLOCKS blocks
 // of 32 complex columns, a counter per group of blocks that share an output
 constexpr int REDUCE_BLOCKS = 592, REDUCE_PART = REDUCE_BLOCKS * 64, REDUCE_CNT = REDUCE_BLOCKS;
-int reduce_scratch(qs_handle *h);
+int reduce_scratch(qs_handle *h, int states);
+// h->pin from a process-wide pool of page-locked slots (64 of 20 KB, allocated with the first handle), so that
+// the small copies of a step neither block the host nor synchronise; a handle that gets no slot uses
+// ordinary memory. Returned by release_all.
+void host_scratch(qs_handle *h, int states);
+void host_scratch_release(qs_handle *h);
+inline int *pin_info(qs_handle *h) { return (int *)(h->pin + 4 * (size_t)h->pin_states); }
+inline double *pin_broyden(qs_handle *h) { return h->pin + 4 * (size_t)h->pin_states + 1; }
+constexpr int PIN_BROYDEN = 4 + 3 * 32;  // norms, (Gram, dF^T F) pairs, gamma
 // The dynamic shared-memory cap of a kernel is a process-wide attribute: it is always set
 // to the device maximum (a cap, not a reservation), so that handles that size the same
 // kernel differently, on other threads, never lower it under each other's launches.
@@ -390,6 +403,8 @@ void release_all(qs_handle *h);
 // that fills F (device) from x (device) and may set abort.
 struct BroydenResidual {
     virtual int operator()(const double *d_x, double *d_F, bool &abort) = 0;
+    // called once the stream has been waited for after operator(): what it left to be read then
+    virtual int complete(bool &abort) { return 0; }
     // true if the residual just evaluated used another precision than the one before: the
     // (dF, u) pair of this step would mix two different residual functions and is not
     // stored, and the history built on the other function is dropped

@@ -558,23 +558,10 @@ int sa_self_energies(qsa_handle *h) {
     return 0;
 }
 
-int sa_read_info(qsa_handle *h) {
-    int info = INT_MAX;
-    QS_CUDA(&h->q, cudaMemcpyAsync(&info, h->d_info, sizeof(int), cudaMemcpyDeviceToHost, h->q.stream));
-    QS_CUDA(&h->q, cudaStreamSynchronize(h->q.stream));
-    if (info != INT_MAX) {
-        h->q.err = "ERROR: ZGETRF failed (singular matrix?) at energy " + std::to_string(info);
-        const int v = INT_MAX;
-        QS_CUDA(&h->q, cudaMemcpyAsync(h->d_info, &v, sizeof(int), cudaMemcpyHostToDevice, h->q.stream));
-        QS_CUDA(&h->q, cudaStreamSynchronize(h->q.stream));
-        return info;
-    }
-    return 0;
-}
-
 // One sweep over all energies: Dyson with (interacting) or without Sigma, Keldysh, pack into
-// out (minus x when given), the sanity sums. interacting = false: the non-interacting G.
-int sa_sweep(qsa_handle *h, double V, bool interacting, double *d_out, const double *d_x) {
+// out (minus x when given), the sanity sums on their way to the host. interacting = false: the
+// non-interacting G.
+int sa_sweep_launch(qsa_handle *h, double V, bool interacting, double *d_out, const double *d_x) {
     const int Na = h->Na, n = h->n;
     const int64_t tot = (int64_t)n * Na * Na;
     cudaStream_t st = h->q.stream;
@@ -590,41 +577,73 @@ int sa_sweep(qsa_handle *h, double V, bool interacting, double *d_out, const dou
         h->q.err = "batched Dyson inversion failed to launch";
         return rc;
     }
-    if ((rc = sa_read_info(h))) return rc;
     SA_RUN(h, K_KELDYSH, sa_keldysh_T<<<grid_for(tot), 256, 0, st>>>(Na, n, h->d_W, h->d_GamL, h->d_GamR, s2 ? h->d_S2L : nullptr,
                                                 s3 ? h->d_S3L : nullptr, h->d_omega, V, h->mu, h->beta, h->d_T));
     SA_RUN(h, K_KELDYSH, sa_keldysh_pack<<<grid_for(tot), 256, 0, st>>>(Na, n, h->d_W, h->d_T, d_x, d_out, h->d_gRd, h->d_gLd));
     // check_gf_sanity sums
     if ((rc = sum_over_energies(&h->q, h->d_gLd, Na, Na, n, h->d_sums, h->d_gRd))) return rc;
-    std::vector<zc> hs(2 * Na);
-    QS_CUDA(&h->q, cudaMemcpyAsync(hs.data(), h->d_sums, sizeof(zc) * 2 * Na, cudaMemcpyDeviceToHost, st));
-    QS_CUDA(&h->q, cudaStreamSynchronize(st));
-    std::vector<zc> sl(hs.begin(), hs.begin() + Na);
+    QS_CUDA(&h->q, cudaMemcpyAsync(h->q.pin, h->d_sums, sizeof(zc) * 2 * Na, cudaMemcpyDeviceToHost, st));
+    QS_CUDA(&h->q, cudaMemcpyAsync(pin_info(&h->q), h->d_info, sizeof(int), cudaMemcpyDeviceToHost, st));
+    return 0;
+}
+
+// its results, once the stream has been waited for
+int sa_sweep_read(qsa_handle *h) {
+    const int Na = h->Na, info = *pin_info(&h->q);
+    if (info != INT_MAX) {
+        h->q.err = "ERROR: ZGETRF failed (singular matrix?) at energy " + std::to_string(info);
+        const int v = INT_MAX;
+        QS_CUDA(&h->q, cudaMemcpyAsync(h->d_info, &v, sizeof(int), cudaMemcpyHostToDevice, h->q.stream));
+        QS_CUDA(&h->q, cudaStreamSynchronize(h->q.stream));
+        return info;
+    }
+    const zc *hs = (const zc *)h->q.pin;
+    std::vector<zc> sl(hs, hs + Na);
     std::vector<double> sr(Na);
     for (int i = 0; i < Na; i++) sr[i] = hs[Na + i].y;
     h->last = check_diag_sanity(Na, sl, sr, h->delta, nullptr);
     return 0;
 }
 
+int sa_sweep(qsa_handle *h, double V, bool interacting, double *d_out, const double *d_x) {
+    const int rc = sa_sweep_launch(h, V, interacting, d_out, d_x);
+    if (rc) return rc;
+    QS_CUDA(&h->q, cudaStreamSynchronize(h->q.stream));
+    return sa_sweep_read(h);
+}
+
 // scf_residual (src/scf.f90:102-136)
-int sa_residual(qsa_handle *h, double V, const double *d_x, double *d_F, bool &abort) {
+int sa_residual_launch(qsa_handle *h, double V, const double *d_x, double *d_F) {
     int rc;
     if ((rc = sa_load_input(h, d_x))) return rc;
     if ((rc = sa_self_energies(h))) return rc;
-    if ((rc = sa_sweep(h, V, true, d_F, d_x))) return rc;
+    return sa_sweep_launch(h, V, true, d_F, d_x);
+}
+int sa_residual_read(qsa_handle *h, double *d_F, bool &abort) {
+    const int rc = sa_sweep_read(h);
+    if (rc) return rc;
     abort = h->last.runaway;
     if (abort) QS_CUDA(&h->q, cudaMemsetAsync(d_F, 0, sizeof(double) * h->n_vec, h->q.stream));
     return 0;
+}
+int sa_residual(qsa_handle *h, double V, const double *d_x, double *d_F, bool &abort) {
+    const int rc = sa_residual_launch(h, V, d_x, d_F);
+    if (rc) return rc;
+    QS_CUDA(&h->q, cudaStreamSynchronize(h->q.stream));
+    return sa_residual_read(h, d_F, abort);
 }
 
 struct SanchoResidual : BroydenResidual {
     qsa_handle *h = nullptr;
     double V = 0.0;
     const double *last_x = nullptr;
-    int operator()(const double *d_x, double *d_F, bool &abort) override {
+    double *last_F = nullptr;
+    int operator()(const double *d_x, double *d_F, bool &) override {
         last_x = d_x;
-        return sa_residual(h, V, d_x, d_F, abort);
+        last_F = d_F;
+        return sa_residual_launch(h, V, d_x, d_F);
     }
+    int complete(bool &abort) override { return sa_residual_read(h, last_F, abort); }
 };
 
 }  // namespace
@@ -687,7 +706,7 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         (rc = up((void **)&h->d_omega, p->omega, (size_t)n * 8)) ||
         (rc = dalloc(q, (void **)&q->d_x, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_F, n_vec * 8)) ||
         (rc = dalloc(q, (void **)&q->d_Fold, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_xold, n_vec * 8)) ||
-        (rc = dalloc(q, (void **)&q->d_red, q->red_len * 8)) || (rc = reduce_scratch(q)) ||
+        (rc = dalloc(q, (void **)&q->d_red, q->red_len * 8)) || (rc = reduce_scratch(q, Na)) ||
         (h->nhist > 0 && ((rc = dalloc(q, &q->d_hdF, broyden_ld(n_vec) * 8 * h->nhist)) ||
                           (rc = dalloc(q, &q->d_hU, broyden_ld(n_vec) * 8 * h->nhist)))) ||
         (rc = dalloc(q, (void **)&h->d_Glt0, Na * zc_)) || (rc = dalloc(q, (void **)&h->d_W, tot * zc_)) ||

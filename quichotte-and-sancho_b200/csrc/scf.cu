@@ -74,6 +74,7 @@ void release_all(qs_handle *h) {
     for (void *p : h->allocs) cudaFreeAsync(p, h->stream);
     h->allocs.clear();
     cudaStreamSynchronize(h->stream);
+    host_scratch_release(h);
 }
 
 // G^<(t=0) on the on-site blocks of the active sites from the SCF vector, then Sigma1
@@ -178,11 +179,9 @@ SanityOut check_diag_sanity(int nb, const std::vector<zc> &sumL, const std::vect
 
 namespace {
 
-int read_info(qs_handle *h, int &info) {
-    int hv[2];
-    QS_CUDA(h, cudaMemcpyAsync(hv, h->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    QS_CUDA(h, cudaStreamSynchronize(h->stream));
-    info = hv[0];
+// the values of d_info once they are in pin_info
+int check_info(qs_handle *h) {
+    const int *hv = pin_info(h);
     if (hv[1] != 0) {  // a bounded tensor-core wait gave up (the kernel freed its TMEM and returned)
         h->err = "tensor-core Keldysh kernel: an mbarrier wait timed out";
         int z = 0;
@@ -190,6 +189,7 @@ int read_info(qs_handle *h, int &info) {
         QS_CUDA(h, cudaStreamSynchronize(h->stream));
         return -3;
     }
+    const int info = hv[0];
     if (info != INT_MAX) {
         h->err = "ERROR: ZGETRF failed (singular matrix?) at energy index " + std::to_string(info);
         int v = INT_MAX;
@@ -198,28 +198,34 @@ int read_info(qs_handle *h, int &info) {
     }
     return 0;
 }
+int enqueue_info(qs_handle *h) {
+    QS_CUDA(h, cudaMemcpyAsync(pin_info(h), h->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    return 0;
+}
+// waits for the stream
+int read_info(qs_handle *h) {
+    const int rc = enqueue_info(h);
+    if (rc) return rc;
+    QS_CUDA(h, cudaStreamSynchronize(h->stream));
+    return check_info(h);
+}
 
-// the sanity of the active states from the sums over energies of the diagonals gRd, gLd
-// already formed in the reduction scratch ([nA] gLd sums, then [nA] gRd sums)
-int sweep_sanity_read(qs_handle *h, SanityOut &s) {
-    zc *sums = (zc *)h->d_red;
-    std::vector<zc> hs(2 * h->nA);
-    QS_CUDA(h, cudaMemcpyAsync(hs.data(), sums, sizeof(zc) * 2 * h->nA, cudaMemcpyDeviceToHost, h->stream));
-    int info, rc;
-    if ((rc = read_info(h, info))) return rc;
-    std::vector<zc> sl(hs.begin(), hs.begin() + h->nA);
+// The sanity of the active states from the sums over energies of the diagonals gRd, gLd
+// already formed in the reduction scratch ([nA] gLd sums, then [nA] gRd sums): the copy to the host,
+// and what is made of it once the stream has been waited for.
+int enqueue_sanity(qs_handle *h) {
+    QS_CUDA(h, cudaMemcpyAsync(h->pin, h->d_red, sizeof(zc) * 2 * h->nA, cudaMemcpyDeviceToHost, h->stream));
+    return enqueue_info(h);
+}
+int read_sanity(qs_handle *h, SanityOut &s) {
+    const int rc = check_info(h);
+    if (rc) return rc;
+    const zc *hs = (const zc *)h->pin;
+    std::vector<zc> sl(hs, hs + h->nA);
     std::vector<double> sr(h->nA);
     for (int i = 0; i < h->nA; i++) sr[i] = hs[h->nA + i].y;
     s = check_diag_sanity(h->nA, sl, sr, h->delta, h->act.data());
     return 0;
-}
-
-// sums over energies of the diagonals gRd, gLd -> sanity of the active states
-int sweep_sanity(qs_handle *h, SanityOut &s) {
-    zc *sums = (zc *)h->d_red;  // [nA] gLd sums, then [nA] gRd sums
-    int rc;
-    if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, sums, h->d_gRd))) return rc;
-    return sweep_sanity_read(h, s);
 }
 
 // order-1 vector: Re, Im of the 2x2 on-site block of G^<(t=0) of each interacting site
@@ -382,7 +388,9 @@ struct Residual2 : BroydenResidual {
     int last_prec = -1, cur_prec = -1;  // 1 = FP32 phase, 0 = FP64, of the last two evaluations
     int evals64 = 0;                    // FP64 evaluations of this solve (the first one captures nothing)
     bool precision_changed() const override { return last_prec >= 0 && last_prec != cur_prec; }
-    int eval(const double *d_x, double *d_F, bool &abort, bool use32) {
+    bool pending = false;               // results to be read by complete()
+    double *F_pending = nullptr;
+    int launch(const double *d_x, double *d_F, bool use32) {
         int rc;
         const bool graph = !use32 && !h->prof_on && !h->graphs_off && (evals64 > 0 || residual2_graph(h, d_x, d_F));
         if (!use32) evals64++;
@@ -391,18 +399,32 @@ struct Residual2 : BroydenResidual {
         } else if ((rc = residual2_launches(h, V, d_x, d_F, use32))) {
             return rc;
         }
+        pending = true;
+        F_pending = d_F;
+        return enqueue_sanity(h);
+    }
+    int complete(bool &abort) override {
+        if (!pending) return 0;
+        pending = false;
         SanityOut s;
-        if ((rc = sweep_sanity_read(h, s))) return rc;
+        const int rc = read_sanity(h, s);
+        if (rc) return rc;
         abort = s.runaway;
-        if (abort) QS_CUDA(h, cudaMemsetAsync(d_F, 0, sizeof(double) * h->n_vec, h->stream));
+        if (abort) QS_CUDA(h, cudaMemsetAsync(F_pending, 0, sizeof(double) * h->n_vec, h->stream));
         return 0;
+    }
+    int eval(const double *d_x, double *d_F, bool &abort, bool use32) {
+        const int rc = launch(d_x, d_F, use32);
+        if (rc) return rc;
+        QS_CUDA(h, cudaStreamSynchronize(h->stream));
+        return complete(abort);
     }
     int operator()(const double *d_x, double *d_F, bool &abort) override {
         iter++;
         last_prec = cur_prec;
         cur_prec = fp32 ? 1 : 0;
         int rc;
-        if (!fp32) return eval(d_x, d_F, abort, false);
+        if (!fp32) return launch(d_x, d_F, false);  // the Broyden loop waits once, for the norms too
         if ((rc = eval(d_x, d_F, abort, true))) return rc;
         if (abort) return 0;
         double fmax;
@@ -441,12 +463,18 @@ struct Residual1 : BroydenResidual {
         QS_CUDA(h, cudaMemcpyAsync(h->d_Sig1, h->Sig1.data(), sizeof(double) * h->Sig1.size(), cudaMemcpyHostToDevice, h->stream));
         int rc;
         if ((rc = sweep(h, M_SCF1, V, true, nullptr, nullptr))) return rc;
+        // the sanity sums and, behind them, the on-site blocks' sums: one wait
+        zc *d = (zc *)h->d_red;
+        std::vector<zc> sums(4 * h->N_sites);
+        if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, d, h->d_gRd))) return rc;
+        if ((rc = sum_over_energies(h, h->d_onsL, 4 * h->N_sites, 4 * h->N_sites, h->n, d + 2 * h->nA))) return rc;
+        if ((rc = enqueue_sanity(h))) return rc;
+        QS_CUDA(h, cudaMemcpyAsync(sums.data(), d + 2 * h->nA, sizeof(zc) * sums.size(), cudaMemcpyDeviceToHost, h->stream));
+        QS_CUDA(h, cudaStreamSynchronize(h->stream));
         SanityOut s;
-        if ((rc = sweep_sanity(h, s))) return rc;
+        if ((rc = read_sanity(h, s))) return rc;
         abort = s.runaway;
         if (!abort) {
-            std::vector<zc> sums;
-            if ((rc = onsite_sums(h, sums))) return rc;
             std::vector<double> Gout((size_t)2 * h->Norb * h->Norb, 0.0);
             std::vector<char> mask(h->site_int.begin(), h->site_int.end());
             gather_onsite(h, sums, mask, Gout);
@@ -454,7 +482,6 @@ struct Residual1 : BroydenResidual {
             for (int64_t i = 0; i < nv; i++) F[i] -= x[i];
         }
         QS_CUDA(h, cudaMemcpyAsync(d_F, F.data(), sizeof(double) * nv, cudaMemcpyHostToDevice, h->stream));
-        QS_CUDA(h, cudaStreamSynchronize(h->stream));
         return 0;
     }
 };
@@ -476,8 +503,7 @@ int final_sweep(qs_handle *h, double V, SanityOut &s) {
     std::vector<double> rs(N + 2);
     QS_CUDA(h, cudaMemcpyAsync(sums.data(), d, sizeof(zc) * sums.size(), cudaMemcpyDeviceToHost, h->stream));
     QS_CUDA(h, cudaMemcpyAsync(rs.data(), dr, sizeof(double) * rs.size(), cudaMemcpyDeviceToHost, h->stream));
-    int info;
-    if ((rc = read_info(h, info))) return rc;
+    if ((rc = read_info(h))) return rc;
     // G_less_obs: on-site blocks of every site, then the intra-atom blocks
     std::fill(h->G_less_obs.begin(), h->G_less_obs.end(), 0.0);
     std::vector<char> all(h->N_sites, 1);
@@ -766,7 +792,7 @@ int qs_create(const qs_problem *p, qs_handle **out) {
         return rc;
     if (h->has_atomL && (rc = dalloc(h, (void **)&h->d_atomL, (size_t)n * h->atom_off.back() * zc_))) return rc;
     h->red_len = std::max<size_t>(broyden_red_len(), (size_t)2 * (4 * h->N_sites + h->atom_off.back() + 2 * N + 2 * nA + 8));
-    if ((rc = dalloc(h, (void **)&h->d_red, h->red_len * 8)) || (rc = reduce_scratch(h))) return rc;
+    if ((rc = dalloc(h, (void **)&h->d_red, h->red_len * 8)) || (rc = reduce_scratch(h, nA))) return rc;
     if ((rc = dalloc(h, (void **)&h->d_info, sizeof(int) * 2)) || (rc = dalloc(h, (void **)&h->d_V, sizeof(double)))) return rc;
     int imax = INT_MAX;
     QS_CUDA(h, cudaMemcpyAsync(h->d_info, &imax, sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -971,8 +997,7 @@ int qs_initial_vector(qs_handle *h, double Volt, double *x) {
         if ((rc = sweep(h, M_INIT2, Volt, false, h->d_x, nullptr))) return rc;
         if ((rc = convert_dl_to_ref(h, h->d_x, h->d_F))) return -rc;
         QS_CUDA(h, cudaMemcpyAsync(x, h->d_F, sizeof(double) * h->n_vec, cudaMemcpyDeviceToHost, h->stream));
-        int info;
-        return read_info(h, info);
+        return read_info(h);
     }
     if (h->order == 1) {
         QS_CUDA(h, cudaMemsetAsync(h->d_Sig1, 0, sizeof(zc) * (size_t)h->Norb * h->Norb, h->stream));
@@ -983,8 +1008,7 @@ int qs_initial_vector(qs_handle *h, double Volt, double *x) {
         std::vector<char> mask(h->site_int.begin(), h->site_int.end());
         gather_onsite(h, sums, mask, G);
         pack_nil(h, G, x);
-        int info;
-        return read_info(h, info);
+        return read_info(h);
     }
     return 0;
 }
@@ -1193,7 +1217,7 @@ int qs_broyden_solve_host(qs_residual_fn residual, void *ctx, double *x, int64_t
     h.red_len = broyden_red_len();
     if ((rc = dalloc(&h, (void **)&h.d_x, n * 8)) || (rc = dalloc(&h, (void **)&h.d_F, n * 8)) ||
         (rc = dalloc(&h, (void **)&h.d_Fold, n * 8)) || (rc = dalloc(&h, (void **)&h.d_xold, n * 8)) ||
-        (rc = dalloc(&h, (void **)&h.d_red, h.red_len * 8)) || (rc = reduce_scratch(&h)) ||
+        (rc = dalloc(&h, (void **)&h.d_red, h.red_len * 8)) || (rc = reduce_scratch(&h, 0)) ||
         (nhist > 0 && ((rc = dalloc(&h, &h.d_hdF, broyden_ld(n) * hist_el * nhist)) || (rc = dalloc(&h, &h.d_hU, broyden_ld(n) * hist_el * nhist))))) {
     } else {
         cudaMemcpyAsync(h.d_x, x, sizeof(double) * n, cudaMemcpyHostToDevice, h.stream);

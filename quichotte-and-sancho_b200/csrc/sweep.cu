@@ -14,6 +14,7 @@
 // Current, the sanity sums) and the pack_gf / unpack_gf layout conversions.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 
 #include "qs_common.cuh"
 #include "reduce.cuh"
@@ -407,7 +408,45 @@ __global__ void __launch_bounds__(256) colsum(const V *__restrict__ A, const V *
     if (rl == 0 && c < ncols) out[blockIdx.z * ncols + c] = tot;
 }
 
-int reduce_scratch(qs_handle *h) {
+namespace {
+constexpr int PIN_SLOTS = 64, PIN_DOUBLES = 2560;
+std::mutex g_pin_mu;
+double *g_pin = nullptr;
+bool g_pin_tried = false, g_pin_used[PIN_SLOTS];
+}  // namespace
+
+void host_scratch(qs_handle *h, int states) {
+    const size_t need = 4 * (size_t)states + 1 + PIN_BROYDEN;
+    h->pin_states = states;
+    if (need <= PIN_DOUBLES) {
+        std::lock_guard<std::mutex> lk(g_pin_mu);
+        if (!g_pin_tried) {
+            g_pin_tried = true;
+            if (cudaHostAlloc((void **)&g_pin, sizeof(double) * PIN_SLOTS * PIN_DOUBLES, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                g_pin = nullptr;
+            }
+        }
+        for (int k = 0; g_pin && k < PIN_SLOTS; k++)
+            if (!g_pin_used[k]) {
+                g_pin_used[k] = true;
+                h->pin = g_pin + (size_t)k * PIN_DOUBLES;
+                return;
+            }
+    }
+    h->pin_own.resize(need);
+    h->pin = h->pin_own.data();
+}
+
+void host_scratch_release(qs_handle *h) {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (g_pin && h->pin >= g_pin && h->pin < g_pin + (size_t)PIN_SLOTS * PIN_DOUBLES)
+        g_pin_used[(h->pin - g_pin) / PIN_DOUBLES] = false;
+    h->pin = nullptr;
+}
+
+int reduce_scratch(qs_handle *h, int states) {
+    host_scratch(h, states);
     int rc = dalloc(h, (void **)&h->d_rpart, sizeof(double) * REDUCE_PART);
     return rc ? rc : dalloc(h, (void **)&h->d_rcnt, sizeof(int) * REDUCE_CNT);
 }
