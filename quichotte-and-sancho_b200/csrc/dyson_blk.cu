@@ -24,7 +24,7 @@
 // Measured on B200, batched inversion (8 N^3 flops a matrix), against the kernels this replaces
 // (row exchanges, 16-wide panels, one block a matrix, or everything through a global workspace):
 // N = 120 8.9 -> 13.9 TFLOP/s; as Dyson of 40 states x 5003 energies 0.99 -> 0.39 ms,
-// 24 x 32768 3.05 -> 0.54 ms, 48 x 4001 1.58 -> 0.36 ms. At N = 120 a matrix takes 280k cycles: the
+// 24 x 32768 3.05 -> 0.48 ms, 48 x 4001 1.58 -> 0.36 ms. At N = 120 a matrix takes 280k cycles: the
 // panels 128k (1070 a column), the updates 125k (107k at the DMMA rate), load and output 30k.
 // Tried instead for N <= 96: the whole matrix in registers, rank-1 updates (4-9 TFLOP/s: the
 // per-step work of every warp, column and row exchange and selects, outweighs the update).
@@ -70,6 +70,9 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
         else if constexpr (PW == 1) __syncwarp();
         else asm volatile("bar.sync 1, %0;\n" ::"n"(32 * PW) : "memory");
     };
+    const bool whole = a.Ain || nA == N;           // every state is active
+    const int di = nthr % N, dj = nthr / N;        // the step from one element of a thread to its next
+    constexpr int NB = PW == 1 ? 6 : 4;
     for (int iw = a.iw0 + blockIdx.x * MPB + slot; iw < a.iw1; iw += gridDim.x * MPB) {
         if (a.Ain) {
             const zc *A = a.Ain + (size_t)(iw - a.iw0) * N * N;
@@ -78,20 +81,34 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
         } else {
             const double w = a.omega[iw];
             const zc *SR = a.Sig + iw * a.sig_ld;
-#pragma unroll 4
-            for (int idx = tid; idx < N * N; idx += nthr) {
-                const int i = idx % N, j = idx / N;
-                zc v = a.Hemb[idx];
-                if (a.use_sigma) {
-                    const int pi = a.pos[i], pj = a.pos[j];
-                    if (pi >= 0 && pj >= 0) {
-                        zc sg = a.Sig1[idx];
-                        if (a.order2) sg = sg + sig_r(SR, pi, pj);
-                        v = v - sg;
+            // NB values a thread at a time: their loads together, those of Sigma2 first
+            int i = tid % N, j = tid / N;
+            for (int idx = tid; idx < N * N; idx += NB * nthr) {
+                zc v[NB], sg[NB];
+                int at_s[NB];
+                bool with[NB];
+#pragma unroll
+                for (int u = 0; u < NB; u++) {
+                    at_s[u] = j < N ? at(i, j, N) : -1;
+                    with[u] = a.use_sigma && j < N;
+                    int pi = i, pj = j;
+                    if (!whole && with[u]) {
+                        pi = a.pos[i];
+                        pj = a.pos[j];
+                        with[u] = pi >= 0 && pj >= 0;
                     }
+                    sg[u] = with[u] && a.order2 ? sig_r(SR, pi, pj) : zc{0, 0};
+                    v[u] = j < N ? a.Hemb[idx + u * nthr] : zc{0, 0};
+                    if (i == j) v[u].x += w;
+                    i += di;
+                    j += dj + (i >= N);
+                    i -= i >= N ? N : 0;
                 }
-                if (i == j) v.x += w;
-                M[at(i, j, N)] = v;
+#pragma unroll
+                for (int u = 0; u < NB; u++) {
+                    if (with[u]) v[u] = v[u] - (a.Sig1[idx + u * nthr] + sg[u]);
+                    if (at_s[u] >= 0) M[at_s[u]] = v[u];
+                }
             }
         }
         // the columns that pad the last tile: zero operands (rows beyond N reach rows beyond N only)
@@ -206,22 +223,29 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
             if (a.info_each) a.info_each[iw - a.iw0] = e.first_zero;
         }
         // scale the rows in place (their lanes know the factors), then write through the permutation
-        if (is_panel && tid < N)
+        if (is_panel && tid < N) {
             for (int j = 0; j < N; j++) {
-                const int o = at(tid, j, N);
-                M[o] = M[o] * scale;
+                zc &m = M[at(tid, j, N)];
+                m = m * scale;
             }
+        }
         sync();
-        const int nout = a.out_mode == 0 ? nA : N;
-        zc *G = a.Gout + (a.out_mode == 0 ? (size_t)iw * nA * nA : (size_t)(iw - a.iw0) * N * N);
-#pragma unroll 4
-        for (int idx = tid; idx < nout * nout; idx += nthr) {
-            int k = idx % nout, c = idx / nout;
-            if (a.out_mode == 0) {
-                k = a.act[k];
-                c = a.act[c];
+        const bool part = a.out_mode == 0 && !whole;  // the active block alone
+        const int nout = part ? nA : N;
+        zc *G = a.out_mode == 0 ? a.Gout + (size_t)iw * nout * nout : a.Gout + (size_t)(iw - a.iw0) * nout * nout;
+        if (part) {
+            for (int idx = tid; idx < nout * nout; idx += nthr) {
+                G[idx] = M[at(e.perm[a.act[idx % nout]], e.step[a.act[idx / nout]], N)];
             }
-            G[idx] = M[at(e.perm[k], e.step[c], N)];
+        } else {
+            int k = tid % N, c = tid / N;
+#pragma unroll 4
+            for (int idx = tid; idx < N * N; idx += nthr) {
+                G[idx] = M[at(e.perm[k], e.step[c], N)];
+                k += di;
+                c += dj + (k >= N);
+                k -= k >= N ? N : 0;
+            }
         }
         sync();
     }
