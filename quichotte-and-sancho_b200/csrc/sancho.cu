@@ -50,6 +50,7 @@
 
 #include "qs_common.cuh"
 #include "qsa200.h"
+#include "reduce.cuh"
 #include "sancho_fft.cuh"
 
 namespace qs {
@@ -339,25 +340,55 @@ __global__ void __launch_bounds__(LT) sa_sigma(int Na, int n, const zc *__restri
 
 // third_order_sigma step 2 (src/self_energies.f90:160-185): per m (or q0) and (i, j)
 //   X^> = sum_k U_k (Y^r_ik Y^>_kj + Y^>_ik Y^a_kj), X^< likewise with Y^<, X^r = sum_k U_k Y^r_ik Y^r_kj
-// for Y = chi (X = D) and Y = phi (X = P). Thread per (p, e), p fastest.
-__global__ void sa_products(int Na, int Nm, const zc *__restrict__ YG, const zc *__restrict__ YL,
-                            const zc *__restrict__ YR, const zc *__restrict__ YA, const double *__restrict__ U,
-                            zc *__restrict__ XG, zc *__restrict__ XL, zc *__restrict__ XR) {
-    const int64_t tot = (int64_t)Nm * Na * Na;
+// for Y = chi (X = D) and Y = phi (X = P), one launch. A thread does a 2 x 2 block of (i, j) at one lag, lags
+// fastest: 14 loads for 4 results and k, where one result a thread took 28. Bound: those loads from
+// L2 (10 sites x 1765 lags: 32 -> 24 us).
+struct SaProducts {
+    const zc *YG[2], *YL[2], *YR[2], *YA[2];
+    zc *XG[2], *XL[2], *XR[2];
+};
+__global__ void __launch_bounds__(128) sa_products(int Na, int Nm, SaProducts a, const double *__restrict__ U) {
+    const int y = blockIdx.y, nb = (Na + 1) / 2;
+    const zc *__restrict__ YG = a.YG[y], *__restrict__ YL = a.YL[y], *__restrict__ YR = a.YR[y], *__restrict__ YA = a.YA[y];
+    const int64_t tot = (int64_t)Nm * nb * nb;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-        const int p = (int)(t % Nm), e = (int)(t / Nm), i = e % Na, j = e / Na;
-        zc g{0, 0}, l{0, 0}, r{0, 0};
+        const int p = (int)(t % Nm), e = (int)(t / Nm), i0 = 2 * (e % nb), j0 = 2 * (e / nb);
+        // (an odd number of sites: the last row and column are computed twice)
+        const int i1 = min(i0 + 1, Na - 1), j1 = min(j0 + 1, Na - 1);
+        zc g[2][2] = {}, l[2][2] = {}, r[2][2] = {};
         for (int k = 0; k < Na; k++) {
-            const size_t ik = ((size_t)i + (size_t)k * Na) * Nm + p, kj = ((size_t)k + (size_t)j * Na) * Nm + p;
             const double u = U[k];
-            const zc rik = YR[ik];
-            g = g + u * (rik * YG[kj] + YG[ik] * YA[kj]);
-            l = l + u * (rik * YL[kj] + YL[ik] * YA[kj]);
-            r = r + u * (rik * YR[kj]);
+            zc ri[2], gi[2], li[2];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const size_t ik = ((size_t)(c ? i1 : i0) + (size_t)k * Na) * Nm + p;
+                ri[c] = u * YR[ik];
+                gi[c] = u * YG[ik];
+                li[c] = u * YL[ik];
+            }
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const size_t kj = ((size_t)k + (size_t)(d ? j1 : j0) * Na) * Nm + p;
+                const zc gk = YG[kj], lk = YL[kj], rk = YR[kj], ak = YA[kj];
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    cfma(g[c][d], ri[c], gk);
+                    cfma(g[c][d], gi[c], ak);
+                    cfma(l[c][d], ri[c], lk);
+                    cfma(l[c][d], li[c], ak);
+                    cfma(r[c][d], ri[c], rk);
+                }
+            }
         }
-        XG[t] = g;
-        XL[t] = l;
-        XR[t] = r;
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const size_t o = ((size_t)(c ? i1 : i0) + (size_t)(d ? j1 : j0) * Na) * Nm + p;
+                a.XG[y][o] = g[c][d];
+                a.XL[y][o] = l[c][d];
+                a.XR[y][o] = r[c][d];
+            }
     }
 }
 
@@ -451,31 +482,39 @@ __global__ void sa_keldysh_pack(int Na, int n, const zc *__restrict__ Gr, const 
 }
 
 // Current (src/observables.f90:18-52): per energy Re Tr{i GammaL [(fL - 1) G^< - fL G^>]}/2pi
-// of G_in, summed over energies (one block)
-__global__ void sa_current(int Na, int n, const zc *__restrict__ EL, const zc *__restrict__ EG,
-                           const zc *__restrict__ GamL, const double *__restrict__ omega, double V, double mu,
-                           double beta, double *__restrict__ out) {
+// of G_in, summed over energies. 32 energies a block, its warps share the (a, c) pairs; the last block adds
+// the partial sums in order (one block for all: 10 sites x 883 energies 157 us, now under 10).
+__global__ void __launch_bounds__(256) sa_current(int Na, int n, const zc *__restrict__ EL, const zc *__restrict__ EG,
+                                                  const zc *__restrict__ GamL, const double *__restrict__ omega, double V,
+                                                  double mu, double beta, double *__restrict__ part, int *__restrict__ cnt,
+                                                  double *__restrict__ out) {
     __shared__ double red[256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    for (int k0 = 32 * blockIdx.x; k0 < n; k0 += 32 * gridDim.x) {
+        const int k = k0 + lane;
+        if (k >= n) continue;
         const double fL = sa_fermi(omega[k], V, mu, beta);
-        zc tr{0.0, 0.0};
-        for (int a = 0; a < Na; a++)
-            for (int c = 0; c < Na; c++) {
-                const zc g = GamL[a + c * Na];
-                const size_t ca = ((size_t)c + (size_t)a * Na) * n + k;
-                const zc v = (fL - 1.0) * EL[ca] - fL * EG[ca];
-                tr = tr + zc{-g.y, g.x} * v;
-            }
-        acc += tr.x / (2.0 * PI);
+        double tr = 0.0;
+#pragma unroll 4
+        for (int e = warp; e < Na * Na; e += 8) {
+            const int a = e % Na, c = e / Na;
+            const zc g = GamL[e];
+            const size_t ca = ((size_t)c + (size_t)a * Na) * n + k;
+            const zc v = (fL - 1.0) * EL[ca] - fL * EG[ca];
+            tr += -g.y * v.x - g.x * v.y;  // Re i g v
+        }
+        acc += tr / (2.0 * PI);
     }
     red[threadIdx.x] = acc;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    for (int w = 128; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[0] = red[0];
+    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    if (!last_block(cnt, gridDim.x)) return;
+    part_reduce(part, gridDim.x, 1, 1, false, red, out);
 }
 
 // write_spectral's A_ii(w) = -2 Im G^r_ii(w) of G_in, [k*Na + i]
@@ -517,10 +556,13 @@ int sa_self_energies(qsa_handle *h) {
     zc *const *E = h->d_E;
     const int64_t tot = (int64_t)Nm * Na * Na;
     auto products = [&]() -> int {
-        SA_RUN(h, K_SIG2B, sa_products<<<grid_for(tot), 256, 0, st>>>(Na, Nm, h->d_chi[0], h->d_chi[1], h->d_chi[2], h->d_chi[3],
-                                                   h->d_U, h->d_D[0], h->d_D[1], h->d_D[2]));
-        SA_RUN(h, K_SIG2B, sa_products<<<grid_for(tot), 256, 0, st>>>(Na, Nm, h->d_phi[0], h->d_phi[1], h->d_phi[2], h->d_phi[3],
-                                                   h->d_U, h->d_P[0], h->d_P[1], h->d_P[2]));
+        SaProducts a;
+        for (int y = 0; y < 2; y++) {
+            zc *const *Y = y ? h->d_phi : h->d_chi, *const *X = y ? h->d_P : h->d_D;
+            a.YG[y] = Y[0], a.YL[y] = Y[1], a.YR[y] = Y[2], a.YA[y] = Y[3];
+            a.XG[y] = X[0], a.XL[y] = X[1], a.XR[y] = X[2];
+        }
+        SA_RUN(h, K_SIG2B, sa_products<<<dim3(grid_for((tot + 3) / 4, 128), 2), 128, 0, st>>>(Na, Nm, a, h->d_U));
         return 0;
     };
     if (h->plan.L) {
@@ -812,8 +854,8 @@ int qsa_solve_scf(qsa_handle *h, double Volt, int fresh_start, qs_scf_result *re
 int qsa_current(qsa_handle *h, double Volt, double *J) {
     qs_handle *q = &h->q;
     QS_CUDA(q, cudaSetDevice(q->device));
-    SA_RUN(h, K_OTHER, sa_current<<<1, 256, 0, q->stream>>>(h->Na, h->n, h->d_E[2], h->d_E[3], h->d_GamL, h->d_omega, Volt, h->mu,
-                                         h->beta, q->d_red));
+    SA_RUN(h, K_OTHER, sa_current<<<std::min((h->n + 31) / 32, REDUCE_BLOCKS), 256, 0, q->stream>>>(h->Na, h->n, h->d_E[2], h->d_E[3],
+                                         h->d_GamL, h->d_omega, Volt, h->mu, h->beta, q->d_rpart, q->d_rcnt, q->d_red));
     double JL = 0.0;
     QS_CUDA(q, cudaMemcpyAsync(&JL, q->d_red, sizeof(double), cudaMemcpyDeviceToHost, q->stream));
     QS_CUDA(q, cudaStreamSynchronize(q->stream));

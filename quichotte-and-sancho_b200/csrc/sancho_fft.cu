@@ -186,7 +186,8 @@ int threads(const SaPlan &p) { return p.L <= 2048 ? 128 : 256; }
 size_t smem(const SaPlan &p) { return sizeof(zc) * (pad(p.L - 1) + 1); }
 
 template <class K, class A> int launch(cudaStream_t st, K kernel, dim3 grid, const SaPlan &p, const A &a) {
-    cudaError_t e = smem_cap((const void *)kernel);
+    // (up to 40 KB need no attribute)
+    cudaError_t e = smem(p) > 40 << 10 ? smem_cap((const void *)kernel) : cudaSuccess;
     if (e == cudaSuccess) {
         count_launch();
         kernel<<<grid, threads(p), smem(p), st>>>(a);
