@@ -616,11 +616,10 @@ def run_sancho(args, device):
     n_it = sum(p["n_iter"] for p in pts)
     conv = sum(int(p["converged"]) for p in pts)
     Na, n = m.N_sites, m.n_omega
-    # algorithmic FP64 work per SCF iteration of the direct sums (complex MAC = 8 flops):
-    # chi and phi 6 MACs per (element, output, summand) over n^2 (output, summand) pairs each,
-    # the particle-hole and particle-particle convolutions 3 MACs each
-    fl_bub = 2 * 6 * 8 * Na * Na * n * n
-    fl_sig = 2 * 3 * 8 * Na * Na * n * n
+    # FP64 work per SCF iteration of the transforms over the energies (5 L log2 L each, L = 2 n): 3 forward and
+    # 10 backward ones per element for Sigma2 and the bubbles, 9 and 2 for Sigma3
+    fl_fft = 5.0 * 2 * n * np.log2(2 * n) * Na * Na
+    fl_bub, fl_sig = 13 * fl_fft, 11 * fl_fft
     ms_bub, ms_sig = prof["bubbles"][0], prof["sigma"][0]
     peak = 37.0  # TFLOP/s, B200 FP64 (nominal; the measured peaks hold no FP64 figure)
     achieved = fl_bub * n_it / (ms_bub * 1e-3) / 1e12 if ms_bub > 0 else 0.0
@@ -647,7 +646,7 @@ def run_sancho(args, device):
             "scf_iterations": [p["n_iter"] for p in pts], "converged": [p["converged"] for p in pts],
             "currents": [p["J"] for p in pts], "seconds_per_scf_iteration": wall / max(n_it, 1),
             "kernel_ms": {k: round(v[0], 3) for k, v in prof.items() if v[1]}, "gpu_launches": launches,
-            "roofline": {"kernel": "sa_bubbles (chi + phi)", "bound": "fp64", "achieved": achieved, "peak": peak,
+            "roofline": {"kernel": "sa_forward, sa_backward (Sigma2, chi, phi)", "bound": "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak, "peak_kind": "nominal",
                          "flop_per_iteration": fl_bub,
                          "sigma_tflops": fl_sig * n_it / (ms_sig * 1e-3) / 1e12 if ms_sig > 0 else 0.0},
@@ -898,25 +897,26 @@ def main():
         nvec = head["n_vec"]
         # spectra of the 12 sequences of every site pair I <= J, at twice the grid's length
         ybytes = 12 * (nA // 2) * (nA // 2 + 1) // 2 * 2 * n * 16.0
-        nh = args.nhist
+        # the Broyden kernels of the timed solves: the norms read F and the previous F, the history update
+        # reads those, both x and the stored dF columns and writes a pair, the update of x reads x, F and the
+        # u columns; the history fills up with the steps, and a solve's last step has the norms alone
+        hel = 4 if BROYDEN["single_history"] else 8
+
+        def step_bytes(s, last):
+            k = min(s - 1, args.nhist)
+            b = 16 if s > 1 else 8
+            return b if last else b + (32 + hel * (k + 1) if k else 0) + 24 + hel * k
+
+        broyden_bytes = nvec * float(sum(step_bytes(s, p["converged"] and s == p["n_iter"]) for p in (f64 or head)["points"]
+                                         for s in range(1, p["n_iter"] + 1)))
         work = {  # algorithmic FLOPs (FP64 compute-bound kernels) or bytes (HBM-bound) per launch
             "dyson_gj": ("fp64", n * 8.0 * N ** 3),                       # G^r: N^3 complex MACs per energy
             "keldysh_scf2": ("fp64", n * 16.0 * nA ** 3),                 # G^< = G SL G^a: 2 nA^3 complex MACs
             "sig2_fwdA": ("hbm", nvec * 8.0 + ybytes),                    # read packed G, write Y
             "sig2_mid": ("hbm", 2.0 * ybytes),                            # read and write Y
             "sig2_invC": ("hbm", 1.5 * ybytes),                           # read Y, write Sigma
-            "broyden": ("hbm", nvec * (64.0 + 12.0 * nh) / 3.0),          # per iteration / 3 launches
+            "broyden": ("hbm", broyden_bytes / max(prof.get("broyden", (0, 1))[1], 1)),
         }
-        # DRAM bytes per launch measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum)
-        # on the 120x120 helix: Dyson and Keldysh per energy at 1024 energies
-        # (profiles/dyson_bgj_helix120_n1024.md, profiles/keldysh_tc_helix120_n1024.md); the
-        # Broyden kernels per vector element (profiles/broyden_kernels_helix120_n1024.md)
-        traffic_per_unit = {"dyson_gj": ((236.776192e6 + 183.729152e6) / 1024, n),
-                            "keldysh_scf2": ((1064.643e6 + 800.101376e6) / 1024, n),
-                            # hist_update_split + x_update + vec_norms of one step (history
-                            # full) per SCF-vector element, averaged over the 3 launches
-                            "broyden": ((4.072997376e9 + 0.356998144e9 + 3.539108352e9 + 0.344236544e9
-                                         + 0.707824128e9) / (3 * 14400 * 1024) / 3, nvec)}
         roof = None
         if fam in work and cnt:
             kind, per_launch = work[fam]
@@ -927,11 +927,8 @@ def main():
             else:
                 achieved, peak, unit = per_launch / t / 1e9, peaks.get("hbm_gbs", 6650.0), "GB/s"
                 src_note = f"hbm_gbs of MEASURED_PEAKS.json ({src})"
-            tpu = traffic_per_unit.get(fam) if (N, nA) == (120, 120) else None
             roof = {"kernel": fam, "bound": kind, "achieved": achieved, "peak": peak, "unit": unit,
-                    "frac": achieved / peak, "traffic": tpu[0] * tpu[1] if tpu else None,
-                    "traffic_note": "DRAM bytes per launch from an ncu capture, scaled per unit" if tpu else None,
-                    "peak_source": src_note,
+                    "frac": achieved / peak, "peak_source": src_note,
                     "per_launch_work": per_launch, "launches": cnt, "avg_launch_ms": ms / cnt}
         prec_name = "fp64" if f64 is not None else "mixed"
         pts = head["points"]

@@ -1,7 +1,7 @@
 /*
  * qsa200.h -- C ABI of the B200 (sm_100a) solver for SANCHO (libqsb200.so): the spinless
  * chain to third order in U, with the second- and third-order self-energies as
- * particle-hole / particle-particle bubble sums over the energy grid.
+ * particle-hole / particle-particle bubbles over the energy grid.
  *
  * Each entry point names the reference routine it replaces (file:line, paths relative to
  * the reference project's SANCHO/ directory). Conventions as in qsb200.h: column-major

@@ -221,19 +221,17 @@ double qs_server_budget_gib(const qs_server *s);
 void qs_server_destroy(qs_server *s);
 
 /* ---- autotuner (no counterpart in the reference) ----
- * Kernel variants whose relative speed depends on the size (kind 0: Dyson, blocked tensor-
- * core Gauss-Jordan: variant 1 in shared memory up to order 120 (nothing else competes there), in
- * the global workspace with one block per SM above it; variant 3 two blocks per SM; beyond order
- * 256 the unblocked one (2); kind 1: Keldysh, tensor-core or CUDA-core GEMMs; kinds 2
- * and 3 (tiles of the Sigma2 kernels) are not decided any more; kind 4: the Keldysh step of a mixed solve's FP32 phase, variant 3 the
- * 3xTF32 kernel on the fifth-generation tensor cores, 1 / 2 the FP64 ones) are timed on the
- * first launch at a new size and the fastest is kept for the process.
+ * Where a step has kernels whose relative speed depends on the size, they are timed on the first
+ * launch at a new size and the fastest is kept for the process. Kind 4 has a choice: the Keldysh step of a
+ * mixed solve's FP32 phase, variant 3 the 3xTF32 kernel on the fifth-generation tensor cores, 1 / 2
+ * the FP64 one. Kinds 0 (Dyson: 1 the blocked Gauss-Jordan up to order 256, 2 the unblocked one) and 1
+ * (Keldysh: 1 FP64 tensor cores up to 256 states, 2 CUDA-core GEMMs) have one form per order, kinds 2
+ * and 3 (tiles of the Sigma2 kernels) are not decided any more.
  * qs_autotune(1) tunes (default), qs_autotune(0) uses the size heuristics only, 2 / 3 force
- * the first (kind 4: the 3xTF32 kernel; else the tensor-core / blocked variant) / last
- * applicable variant, 4 the second of three (kind 0: variant 3; kind 4: the FP64 tensor-core
- * kernel), qs_autotune(-1) forgets the recorded choices. qs_tuned_choice returns
- * the recorded variant (1, 2 or 3) or -1; a decision
- * is keyed by size = order + 1024 * floor(log2(n_omega)) (order N for Dyson, nA for Keldysh). */
+ * the first (kind 4: the 3xTF32 kernel) / last applicable variant, 4 the second of three,
+ * qs_autotune(-1) forgets the recorded choices. qs_tuned_choice returns the recorded variant
+ * (1, 2 or 3) or -1; a decision is keyed by size = order + 1024 * floor(log2(n_omega)) (order N
+ * for Dyson, nA for Keldysh). */
 int qs_autotune(int mode);
 int qs_tuned_choice(int kind, int size);
 
@@ -245,7 +243,7 @@ int qs_tuned_choice(int kind, int size);
 int64_t qs_kernel_launches(void);
 
 /* SCF residuals of this handle replayed from a CUDA graph: the FP64 residual's launches
- * (G^<(t=0), Sigma2, Dyson, Keldysh, the sanity sums) are captured once per (x, F, V) buffer
+ * (G^<(t=0), Sigma2, Dyson, Keldysh, the sanity sums) are captured once per (x, F) buffer
  * pair and replayed by the Broyden loop (not while per-launch profiling is on). */
 int64_t qs_graph_replays(const qs_handle *h);
 

@@ -1,8 +1,7 @@
 // autotune.cu -- a process-wide table of kernel-variant choices, filled by timing.
 //
 // Some steps have more than one kernel whose relative speed depends on the problem size
-// (Dyson: blocked Gauss-Jordan on the FP64 tensor cores or the unblocked kernel; Keldysh:
-// tensor-core or CUDA-core GEMMs). The first launch of a step at a size not yet in the table
+// (the Keldysh step of a mixed solve's FP32 phase: 3xTF32 or FP64). The first launch of a step at a size not yet in the table
 // times every candidate on the handle's own inputs (CUDA events on its stream) and records
 // the fastest; later launches at that size, from any handle of the process, use the
 // recorded choice (each candidate timed twice, the faster run counting). Every candidate
