@@ -1,6 +1,6 @@
 // keldysh_rows.cu -- products with the rows of T = G^r SL in shared memory: the outputs of the final sweep
 // (final_rows, below) and the Keldysh step of the sweep (modes M_INIT2 / M_SCF2, src/scf.f90:333-355) for
-// active blocks of 81 to 256 states: G^< = G^r SL G^r^dagger with SL = i (f_L Gamma_L + f_R Gamma_R) +
+// active blocks of 49 to 256 states: G^< = G^r SL G^r^dagger with SL = i (f_L Gamma_L + f_R Gamma_R) +
 // Sigma2^<, written with G^r into the packed vector minus x.
 //
 // One block per (energy, 32 rows). The rows of G^r are held in shared memory for all k, the other operand
@@ -16,7 +16,8 @@
 // other, so G^r and Sigma^< come from L2; two blocks share an SM up to 128 states, so that one's copies
 // and stores overlap another's products. Measured on B200 per launch: 120 states x 4096 energies
 // 5.1 -> 4.5 ms (one block an SM with 16-deep panels of both operands in shared memory, SL and T through
-// scratch matrices), 192 x 1201 10.1 -> 5.0 ms (32x32-tile CUDA-core GEMMs), the tensor pipe 69 % busy.
+// scratch matrices), 192 x 1201 10.1 -> 5.0 ms (32x32-tile CUDA-core GEMMs), the tensor pipe 69 % busy;
+// 64 x 4096 0.84 -> 0.61, 80 x 4096 1.43 -> 1.22 (one energy a block with both operands in shared memory).
 // Touching a loaded value (its sign) before the step that uses it cost 30 %.
 #include <algorithm>
 

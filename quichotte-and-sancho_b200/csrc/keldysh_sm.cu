@@ -1,5 +1,5 @@
 // keldysh_sm.cu -- the Keldysh step of the sweep (modes M_INIT2 / M_SCF2, src/scf.f90:333-355) for
-// active blocks up to 80: G^< = G^r SL G^r^dagger with SL = i (f_L Gamma_L + f_R Gamma_R) + Sigma2^<,
+// active blocks up to 48: G^< = G^r SL G^r^dagger with SL = i (f_L Gamma_L + f_R Gamma_R) + Sigma2^<,
 // written with G^r into the packed vector minus x.
 //
 // One block per energy with G^r and SL in shared memory, both products on the FP64 tensor cores:
@@ -187,15 +187,15 @@ template <int MT, int MAXT, int MINB> int run(qs_handle *h, const KeldyshArgs &k
 
 }  // namespace
 
-bool keldysh_sm_fits(int nA) { return nA <= 80; }
+// above, blocks of 32 rows are faster: one energy's two matrices leave room for one or two blocks an SM
+// (per launch, 4096 energies: 48 states 0.32 ms here, 0.39 by rows; 56 0.74 and 0.53; 80 1.43 and 1.22)
+bool keldysh_sm_fits(int nA) { return nA <= 48; }
 
 int launch_keldysh_sm(qs_handle *h, const KeldyshArgs &k) {
     switch ((k.nA + 15) / 16) {
         case 1: return run<1, 64, 12>(h, k);
         case 2: return run<2, 128, 7>(h, k);
-        case 3: return run<3, 192, 3>(h, k);
-        case 4: return run<4, 256, 1>(h, k);
-        default: return run<5, 320, 1>(h, k);
+        default: return run<3, 192, 3>(h, k);
     }
 }
 

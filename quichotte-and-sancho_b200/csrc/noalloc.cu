@@ -7,7 +7,7 @@
 // device-wide synchronisation cudaMalloc/cudaFree may cause. Such a caller already holds
 // its matrices and outputs in device memory and only needs the inversion itself.
 //
-// The elimination runs in shared memory up to order 120 and above that in the caller's matrices
+// The elimination runs in shared memory (small orders or batches) or in the caller's matrices
 // themselves, so the call needs no workspace at all: it allocates nothing, keeps nothing between
 // calls, and calls on different matrices may overlap on any streams and threads.
 #include <cstdio>

@@ -323,7 +323,7 @@ struct FinalArgs {
     const int *cidx;  // the contact states, as in KeldyshArgs
     int nc;
 };
-// the Keldysh step with both operands in shared memory (keldysh_sm.cu): nA <= 80
+// the Keldysh step with both operands in shared memory (keldysh_sm.cu): nA <= 48
 int launch_keldysh_sm(qs_handle *h, const KeldyshArgs &k);
 bool keldysh_sm_fits(int nA);
 // the same by blocks of 32 rows (keldysh_rows.cu): nA <= 256
