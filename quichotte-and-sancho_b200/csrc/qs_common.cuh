@@ -104,7 +104,7 @@ constexpr double PI = 3.14159265358979323846;
 constexpr int SMEM_MAX = 232448;  // max dynamic shared memory per block on sm_100 (227 KB)
 
 // The Gauss-Jordan kernel keeps the N x N complex matrix in shared memory when it fits next to its
-// 1.5 KB of static shared memory.
+// 1.6 KB of static shared memory.
 constexpr int DYSON_SMEM_MAXN = 120;
 inline bool dyson_fits_smem(int N) { return N <= DYSON_SMEM_MAXN; }
 

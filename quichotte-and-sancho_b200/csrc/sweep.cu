@@ -501,10 +501,10 @@ int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref) {
 // ---------------------------------------------------------------------------------
 constexpr int GJ_THREADS = 512;  // the unblocked kernel, N <= 512
 
-// Up to 80 states several matrices share an SM's memory (dyson_blk: 80 x 4000 1.31 ms, dyson_l2 1.22, but
-// 50 x 4000 0.46 and 0.52). From there to DYSON_SMEM_MAXN dyson_blk holds one matrix an SM, the faster
-// form while there is one for each SM at most (96 x 148 0.110 ms, dyson_l2 0.136; 120 x 200 0.288 and
-// 0.272, 96 x 4000 2.77 and 1.60); it is also the one that needs no workspace when G is a part of the matrix.
+// Up to 80 states several matrices share an SM's memory (dyson_blk: 64 x 4000 0.79 ms, dyson_l2 0.82; 80 x 148 0.09
+// and 0.13, if 80 x 4000 1.52 and 1.42). From there to DYSON_SMEM_MAXN dyson_blk holds one matrix an SM, the faster
+// form while there is one for each SM at most (96 x 148 0.121 ms, dyson_l2 0.164; 120 x 170 0.342 and
+// 0.300, 96 x 4000 3.21 and 1.91); it is also the one that needs no workspace when G is a part of the matrix.
 static int run_dyson(cudaStream_t st, const DysonArgs &a) {
     if (a.N <= 80 || (dyson_fits_smem(a.N) && (!a.inplace || a.iw1 - a.iw0 <= 148))) return launch_dyson_blk(st, a);
     if (dyson_l2_fits(a.N)) return launch_dyson_l2(st, a);
