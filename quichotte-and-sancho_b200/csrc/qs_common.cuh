@@ -381,6 +381,8 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
 int sum_over_energies(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out,
                       const zc *d_B = nullptr);
 int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncols, int64_t nrows, double *d_out);
+// the same for d_A alone, added in an order that does not depend on the grid (the vector of order 1)
+int sum_in_order(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out);
 // batch N x N column-major matrices inverted in place; d_min (or nullptr) receives the smallest
 // 1 + b of a singular one, d_each[b] 1 + the step of its first zero pivot
 int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each);

@@ -293,7 +293,7 @@ void gather_onsite(const qs_handle *h, const std::vector<zc> &sums, const std::v
 int onsite_sums(qs_handle *h, std::vector<zc> &sums) {
     zc *d = (zc *)h->d_red;
     int rc;
-    if ((rc = sum_over_energies(h, h->d_onsL, 4 * h->N_sites, 4 * h->N_sites, h->n, d))) return rc;
+    if ((rc = sum_in_order(h, h->d_onsL, 4 * h->N_sites, 4 * h->N_sites, h->n, d))) return rc;
     sums.resize(4 * h->N_sites);
     QS_CUDA(h, cudaMemcpyAsync(sums.data(), d, sizeof(zc) * sums.size(), cudaMemcpyDeviceToHost, h->stream));
     QS_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -467,7 +467,7 @@ struct Residual1 : BroydenResidual {
         zc *d = (zc *)h->d_red;
         std::vector<zc> sums(4 * h->N_sites);
         if ((rc = sum_over_energies(h, h->d_gLd, h->nA, h->nA, h->n, d, h->d_gRd))) return rc;
-        if ((rc = sum_over_energies(h, h->d_onsL, 4 * h->N_sites, 4 * h->N_sites, h->n, d + 2 * h->nA))) return rc;
+        if ((rc = sum_in_order(h, h->d_onsL, 4 * h->N_sites, 4 * h->N_sites, h->n, d + 2 * h->nA))) return rc;
         if ((rc = enqueue_sanity(h))) return rc;
         QS_CUDA(h, cudaMemcpyAsync(sums.data(), d + 2 * h->nA, sizeof(zc) * sums.size(), cudaMemcpyDeviceToHost, h->stream));
         QS_CUDA(h, cudaStreamSynchronize(h->stream));

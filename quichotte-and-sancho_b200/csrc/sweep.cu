@@ -408,6 +408,58 @@ __global__ void __launch_bounds__(256) colsum(const V *__restrict__ A, const V *
     if (rl == 0 && c < ncols) out[blockIdx.z * ncols + c] = tot;
 }
 
+// The on-site sums that are the SCF vector at first order, in an order that does not depend on the grid: eight
+// chains a column, rows r = 0..7 (mod 8) in turn, then the chains one after the other. Levels of width 1e-6 t turn the
+// last bits of such a sum into 1e-10 of their spectra. A block has 4 columns: 256 threads bring tiles of 128 rows
+// into shared memory, four under way, 32 of them add. Bound: the chains, one dependent addition for eight rows
+// (40 cycles: 96 columns x 4001 energies 12 us, 24 x 32768 85 us, where colsum takes 6 and 12).
+constexpr int SUM_COLS = 4, SUM_ROWS = 128, SUM_STAGES = 5;
+__global__ void __launch_bounds__(256) chain_sums(const zc *__restrict__ A, int64_t ld, int ncols, int64_t nrows, zc *__restrict__ out) {
+    __shared__ zc tile[SUM_STAGES][SUM_ROWS][SUM_COLS], chain[8][SUM_COLS];
+    const int c0 = blockIdx.x * SUM_COLS, c = threadIdx.x % SUM_COLS, l = threadIdx.x / SUM_COLS;
+    const int tiles = (int)((nrows + SUM_ROWS - 1) / SUM_ROWS);
+    auto load = [&](int t) {
+        if (t < tiles) {
+            for (int r = l; r < SUM_ROWS; r += 256 / SUM_COLS) {
+                const int64_t row = (int64_t)t * SUM_ROWS + r;
+                const bool in = row < nrows && c0 + c < ncols;  // (else zero)
+                const unsigned d = (unsigned)__cvta_generic_to_shared(&tile[t % SUM_STAGES][r][c]);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(in ? A + row * ld + c0 + c : A), "r"(in ? 16 : 0)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int t = 0; t < SUM_STAGES - 1; t++) load(t);
+    zc acc{};
+    for (int t = 0; t < tiles; t++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(SUM_STAGES - 2) : "memory");
+        __syncthreads();
+        load(t + SUM_STAGES - 1);  // where tile t - 1 was
+        if (l < 8) {
+            const zc(*x)[SUM_COLS] = tile[t % SUM_STAGES];
+#pragma unroll
+            for (int r = 0; r < SUM_ROWS; r += 8) acc = acc + x[r + l][c];
+        }
+    }
+    if (l < 8) chain[l][c] = acc;
+    __syncthreads();
+    if (l == 0 && c0 + c < ncols) {
+        zc s = chain[0][c];
+        for (int q = 1; q < 8; q++) s = s + chain[q][c];
+        out[c0 + c] = s;
+    }
+}
+
+int sum_in_order(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out) {
+    if (ncols <= 0) return 0;
+    int pi = prof_begin(h, K_REDUCE);
+    chain_sums<<<(ncols + SUM_COLS - 1) / SUM_COLS, 256, 0, h->stream>>>(d_A, ld, ncols, nrows, d_out);
+    prof_end(h, pi);
+    QS_CUDA(h, cudaGetLastError());
+    return 0;
+}
+
 namespace {
 constexpr int PIN_SLOTS = 64, PIN_DOUBLES = 2560;
 std::mutex g_pin_mu;
