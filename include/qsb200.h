@@ -90,7 +90,8 @@ int qs_current(qs_handle *h, double Volt, double *J_up, double *J_down);
  * pointer may be NULL. */
 int qs_get_observables(qs_handle *h, double *G_less_obs, double *dosd, double *trU, double *trD);
 
-/* Sizes: n_vec (src/green_functions.f90:397-405), nA, Nf. */
+/* Sizes: n_vec (src/green_functions.f90:397-405), nA, and the padded transform length of the reference for this grid
+ * (good_fft_size(2 n - 1)); the solver's own transforms may be of another length >= 2 n - 1. */
 int64_t qs_vector_length(const qs_handle *h);
 int qs_active_states(const qs_handle *h);
 int qs_fft_length(const qs_handle *h);
@@ -171,9 +172,11 @@ int qs_broyden_solve_host(qs_residual_fn residual, void *ctx, double *x, int64_t
  * replaced by their inverses; info[b] = 0, or k+1 for a zero pivot at step k. The work
  * runs asynchronously on `stream` (a cudaStream_t, NULL = legacy default stream); read info
  * after synchronising. The library allocates nothing and keeps no scratch: calls on different
- * matrices may overlap on the GPU. Limits: 1 <= N <= 512 (else QS_ERR_NOALLOC_LIMIT, with a
- * message on stderr). Returns 0 or a CUDA error (< 0). */
- enum { QS_ERR_NOALLOC_LIMIT = -1001 };
+ * matrices may overlap on the GPU. The driver may load a kernel's code on its first launch on a device, which can
+ * take device memory and synchronise: make one call of each size used before memory runs out or a stream capture
+ * begins. (The kernels change at N = 32, 64, 80, 96, 120, 128 and 256, and from 81 to 120 at 148 matrices.) Limits:
+ * 1 <= N <= 512 (else QS_ERR_NOALLOC_LIMIT, with a message on stderr). Returns 0 or a CUDA error (< 0). */
+enum { QS_ERR_NOALLOC_LIMIT = -1001 };
 int qs_invert_batched_noalloc(int N, int batch, double *A, int *info, void *stream);
 
 /* ---- memory (setup_storage's memory estimate, src/green_functions.f90:90-190) ---- */
