@@ -195,8 +195,8 @@ template <typename T, int R, int S> __device__ __forceinline__ void dft(cplx<T> 
 }
 
 // The transform lengths that have kernels, and their split L = R1 R2 with R1 >= R2. The radices
-// are 4..16 and the lengths at most 14 % apart, so that a product of two of them lies a few
-// percent above any length up to 65536.
+// are 4..16 and the lengths 11 to 25 % apart, so that a product of two of them lies a few percent above
+// any length from 400 up to 65536.
 #define QS_FFT_LENGTHS(X) \
     X(4, 4) X(5, 4) X(6, 4) X(7, 4) X(8, 4) X(6, 6) X(8, 5) X(8, 6) X(8, 7) X(8, 8) X(9, 8) X(10, 8) X(12, 8) X(14, 8) \
     X(16, 8) X(12, 12) X(16, 10) X(16, 12) X(16, 14) X(16, 16)

@@ -726,7 +726,7 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         return -(int)e;
     }
     if (h->order >= 2) h->plan = sa_plan(n);
-    // the spectra are up to 14 % longer than the bubbles: direct sums where only those fit
+    // the spectra are up to 14 % longer than the bubbles (18 % below 100 energies): direct sums where only those fit
     size_t room = 0, all = 0;
     const size_t values = nf * ((size_t)(h->order == 3 ? 14 : 3) * h->plan.L + (size_t)10 * n);
     if (cudaMemGetInfo(&room, &all) != cudaSuccess || zc_ * values + 24 * tot * (4 + 2 * p->nhist) > room) h->plan = SaPlan{};

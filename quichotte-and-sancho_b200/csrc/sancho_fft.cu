@@ -19,7 +19,8 @@
 //
 // The direct sums it replaces cost 12 (bubbles) and 6 multiply-adds per pair of energies and element;
 // they remain for grids whose sequences do not fit in shared memory. Bound: the latency of the few
-// launches (10 sites x 883 energies: 15 MFLOP per element, 1.8 MB per array, all in L2).
+// launches (10 sites x 883 energies, order 3: 24 transforms of 1792 values an element, 2.3 MFLOP; 2.9 MB per
+// array, all in L2).
 #include <algorithm>
 
 #include "fft.cuh"
@@ -29,7 +30,7 @@ namespace qs {
 namespace {
 
 __host__ __device__ __forceinline__ int pad(int p) { return p + (p >> 4); }  // bank groups of 8 words
-constexpr int SA_LMAX = 13600;  // pad(L) * 16 bytes within SMEM_MAX
+constexpr int SA_LMAX = 13440;  // the longest product of radices with pad(L) * 16 bytes within SMEM_MAX
 
 // one pass over blocks of Ns = R M values: forward (S < 0) butterfly then twiddle, backward the reverse
 template <int R, int S> __device__ __forceinline__ void pass(zc *s, int L, int Ns, const zc *__restrict__ tw) {
@@ -201,7 +202,7 @@ template <class K, class A> int launch(cudaStream_t st, K kernel, dim3 grid, con
 SaPlan sa_plan(int n) {
     static const int R[] = {16, 14, 12, 10, 9, 8, 7, 6, 5, 4};
     SaPlan best;
-    if (n > (SA_LMAX + 1) / 2) return best;
+    if (2 * n - 1 > SA_LMAX) return best;
     const int need = std::max(2 * n - 1, 16);
     const int nst = need <= 256 ? 2 : need <= 4096 ? 3 : 4;
     for (int a : R)

@@ -11,7 +11,7 @@ struct SaPlan {
     int rad[4] = {1, 1, 1, 1};
 };
 // the shortest one for a grid of n energies (L >= 2 n - 1); L = 0 where a sequence does not fit in
-// shared memory: n above about 6800
+// shared memory: n above 6720
 SaPlan sa_plan(int n);
 
 struct SaFft {

@@ -329,7 +329,7 @@ int residual2_launches(qs_handle *h, double V, const double *d_x, double *d_F, b
 // at the first evaluation of a solve (that one has made every autotuner decision of the sizes). Not
 // with per-launch profiling on (its events are per launch) nor in the FP32 phase; a capture that fails
 // turns graphs off for the handle (eager launches, same results). The voltage is read from device
-// memory: with it in the launches' arguments every solve at a new voltage captured two graphs (16 states
+// memory: with it in the launches' arguments every solve at a new voltage captured two graphs (8 states
 // x 329 energies, 6 steps: 0.35 ms more a solve).
 qs_handle::ResidualGraph *residual2_graph(qs_handle *h, const double *d_x, const double *d_F) {
     for (auto &g : h->graphs)
