@@ -16,8 +16,8 @@
 // inverse and column k its column p_k; the output is written through that permutation.
 //
 // The operations on a value are those of the elimination with row exchanges in panels of 16, bit for bit. Panels of 8
-// with undivided pivot rows took 0.41 ms where these take 0.48 (24 x 32768; 48 x 4000 0.33 and 0.41, 80 x 4096 1.31
-// and 1.53), but rounded differently: spectra of 48 first-order states moved by up to 2e-9 (their sharp levels are
+// with undivided pivot rows took 0.41 ms where these take 0.48 (24 x 32768; 48 x 4000 0.33 and 0.41, 80 x 4096 1.32
+// and 1.55), but rounded differently: spectra of 48 first-order states moved by up to 2e-9 (their sharp levels are
 // not determined better), and results are to stay what they were.
 //
 // Bound: the chain of a panel's column (search, row, barrier, reciprocal, division, 64 DFMA); the
@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(32 * W * MPB, MINB) dyson_blk(DysonArgs a) {
         for (int k0 = 0; k0 < N; k0 += PB) {
             const int kb = min(PB, N - k0);
             if (is_panel) {
-                const bool mine = eliminate_panel(e, PW, tid, N, k0, kb, place, [&](int c) { return M + at(tid, k0 + c, N); }, panel_sync);
+                const bool mine = eliminate_panel(e, PW, tid, N, k0, kb, place, a.zero_of_inf, [&](int c) { return M + at(tid, k0 + c, N); },
+                                                  panel_sync);
                 if (mine) e.step[tid] = (unsigned char)place;
                 const unsigned u = __ballot_sync(0xffffffffu, mine);
                 if (lane == 0) e.used[warp] = u;

@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(32 * W, MINB) dyson_l2(DysonArgs a) {
             for (int h = 0; PB * h < kb; h++) {
                 if (is_panel) {
                     const int c0 = PB * h, nb = min(PB, kb - c0);
-                    const bool mine = eliminate_panel(e, PW, tid, N, k0 + c0, nb, place, [&](int c) { return P + at(tid, c0 + c, N); }, panel_sync);
+                    const bool mine = eliminate_panel(e, PW, tid, N, k0 + c0, nb, place, a.zero_of_inf,
+                                                      [&](int c) { return P + at(tid, c0 + c, N); }, panel_sync);
                     const unsigned u = __ballot_sync(0xffffffffu, mine);
                     if (lane == 0) e.used[h][warp] = u;
                 }

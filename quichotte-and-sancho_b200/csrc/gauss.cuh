@@ -8,7 +8,7 @@ namespace qs {
 constexpr int PB = 16;  // panel width: the k extent of one FP64 tensor-core product
 
 // 1 / a without overflow or underflow of the intermediate |a|^2: a is scaled by the power of two
-// that brings its larger part to [1, 2)
+// that brings its larger part to [1, 2). (An infinite a gives NaN.)
 __device__ __forceinline__ zc scaled_recip(zc a) {
     const unsigned h = max((unsigned)__double2hiint(a.x) & 0x7fffffffu, (unsigned)__double2hiint(a.y) & 0x7fffffffu) >> 20;
     const double s = __hiloint2double((int)(min(max(2046 - (int)h, 1), 2046) << 20), 0);  // 2^(1023 - h)
@@ -18,6 +18,7 @@ __device__ __forceinline__ zc scaled_recip(zc a) {
 
 // |Re| + |Im| >= 0, so its bit pattern orders like its value (a NaN is a large key: a row is
 // always found); 0 marks a row that is used or beyond the matrix
+constexpr unsigned long long INF_KEY = 0x7ff0000000000001ull;
 __device__ __forceinline__ unsigned long long pivot_key(zc v, bool open) {
     return open ? (unsigned long long)__double_as_longlong(cabs1(v)) + 1 : 0;
 }
@@ -57,7 +58,7 @@ template <int PW, int NBUF> struct PanelExchange {
 // that of the elimination with row exchanges too.
 template <int WD, int PW, int NBUF, class SYNC>
 __device__ __forceinline__ bool eliminate_steps(PanelExchange<PW, NBUF> &e, int npw, zc (&R)[WD], int row, int N, int k0, int kb,
-                                                int &place, SYNC sync) {
+                                                int &place, bool zero_of_inf, SYNC sync) {
     const int lane = row & 31, warp = PW == 1 ? 0 : row >> 5;
     bool mine = false;
 #pragma unroll 1
@@ -95,7 +96,8 @@ __device__ __forceinline__ bool eliminate_steps(PanelExchange<PW, NBUF> &e, int 
         // the pivot row over its pivot, a value a lane; a copy for each warp, where its own candidate stood
         zc *S = warp == wb ? e.extra : e.row[b][warp];
         if (lane < WD) {
-            const zc inv = zero || (fz != 0 && fz <= k) ? zc{0, 0} : e.row[b][wb][0], v = e.row[b][wb][lane];
+            const bool none = zero || (fz != 0 && fz <= k) || (zero_of_inf && bk == INF_KEY);
+            const zc inv = none ? zc{0, 0} : e.row[b][wb][0], v = e.row[b][wb][lane];
             S[lane] = lane == 0 ? inv : v * inv;
         }
         if constexpr (NBUF == 1 && PW > 1) sync();
@@ -133,11 +135,11 @@ __device__ __forceinline__ bool eliminate_steps(PanelExchange<PW, NBUF> &e, int 
 // The panel of kb <= 16 columns in shared memory, lane `row` doing its row: value c at col(c)
 template <int WD, int PW, int NBUF, class COL, class SYNC>
 __device__ __forceinline__ bool eliminate_columns(PanelExchange<PW, NBUF> &e, int npw, int row, int N, int k0, int kb, int &place,
-                                                  COL col, SYNC sync) {
+                                                  bool zero_of_inf, COL col, SYNC sync) {
     zc R[WD];
 #pragma unroll
     for (int c = 0; c < WD; c++) R[c] = row < N && c < kb ? *col(c) : zc{0, 0};
-    const bool mine = eliminate_steps<WD>(e, npw, R, row, N, k0, kb, place, sync);
+    const bool mine = eliminate_steps<WD>(e, npw, R, row, N, k0, kb, place, zero_of_inf, sync);
     if (row < N)
 #pragma unroll
         for (int j = 0; j < WD; j++) {
@@ -147,10 +149,10 @@ __device__ __forceinline__ bool eliminate_columns(PanelExchange<PW, NBUF> &e, in
     return mine;
 }
 template <int PW, int NBUF, class COL, class SYNC>
-__device__ __forceinline__ bool eliminate_panel(PanelExchange<PW, NBUF> &e, int npw, int row, int N, int k0, int kb, int &place, COL col,
-                                                SYNC sync) {
-    return kb > 8 ? eliminate_columns<PB>(e, npw, row, N, k0, kb, place, col, sync)
-                  : eliminate_columns<8>(e, npw, row, N, k0, kb, place, col, sync);
+__device__ __forceinline__ bool eliminate_panel(PanelExchange<PW, NBUF> &e, int npw, int row, int N, int k0, int kb, int &place,
+                                                bool zero_of_inf, COL col, SYNC sync) {
+    return kb > 8 ? eliminate_columns<PB>(e, npw, row, N, k0, kb, place, zero_of_inf, col, sync)
+                  : eliminate_columns<8>(e, npw, row, N, k0, kb, place, zero_of_inf, col, sync);
 }
 
 }  // namespace qs

@@ -27,5 +27,5 @@ extern "C" int qs_invert_batched_noalloc(int N, int batch, double *A, int *info,
     cudaStream_t st = (cudaStream_t)stream;
     const cudaError_t e = cudaMemsetAsync(info, 0, sizeof(int) * (size_t)batch, st);  // 0: no zero pivot
     if (e != cudaSuccess) return -(int)e;
-    return qs::invert_batched_dev(st, N, batch, (qs::zc *)A, nullptr, info);
+    return qs::invert_batched_dev(st, N, batch, (qs::zc *)A, nullptr, info, true);
 }

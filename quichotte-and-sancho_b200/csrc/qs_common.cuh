@@ -280,6 +280,7 @@ struct DysonArgs {
     int *info;     // min over energies of (iw + 1) with a zero pivot; INT_MAX if none
     const zc *Ain; // batched-inversion mode: matrices to invert (nullptr for the sweep)
     int *info_each;
+    int zero_of_inf;  // 1 / inf = 0 for a pivot, else NaN: orders below 16, and qs_invert_batched_noalloc
     int inplace;   // kernels whose matrix is in global memory: in Gout itself (N x N each) instead of ws
 };
 // the blocked elimination in shared memory (dyson_blk.cu), N <= DYSON_SMEM_MAXN; 0 or a CUDA error (< 0)
@@ -385,7 +386,7 @@ int sum_over_energies_real(qs_handle *h, const double *d_A, int64_t ld, int ncol
 int sum_in_order(qs_handle *h, const zc *d_A, int64_t ld, int ncols, int64_t nrows, zc *d_out);
 // batch N x N column-major matrices inverted in place; d_min (or nullptr) receives the smallest
 // 1 + b of a singular one, d_each[b] 1 + the step of its first zero pivot
-int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each);
+int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each, bool zero_of_inf = false);
 int convert_ref_to_dl(qs_handle *h, const double *ref, double *dl);
 int convert_dl_to_ref(qs_handle *h, const double *dl, double *ref);
 

@@ -577,7 +577,7 @@ static int launch_dyson(qs_handle *h, DysonArgs &a) {
     return 0;
 }
 
-int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each) {
+int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, int *d_each, bool zero_of_inf) {
     DysonArgs a{};
     a.N = N;
     a.iw1 = batch;
@@ -587,6 +587,7 @@ int invert_batched_dev(cudaStream_t st, int N, int batch, zc *d_A, int *d_min, i
     a.info = d_min;
     a.info_each = d_each;
     a.inplace = 1;
+    a.zero_of_inf = zero_of_inf || N < 16;
     count_launch();
     return run_dyson(st, a);
 }
@@ -622,6 +623,7 @@ int sweep(qs_handle *h, int mode, double V, bool use_sigma, double *d_out, const
     a.use_sigma = use_sigma;
     a.order2 = (h->order == 2);
     a.info = h->d_info;
+    a.zero_of_inf = N < 16;
     int rc;
     if (mode == M_INIT2 || mode == M_SCF2) {
         a.iw0 = 0;
