@@ -174,6 +174,7 @@ struct qs_handle {
     // sweep scratch
     qs::zc *d_G = nullptr;  // Dyson output (G_AA for all energies, or full G for a chunk)
     size_t G_chunk = 0;     // energies per chunk in full-G mode
+    bool small_chunks = false;  // order 2: no memory beyond G_AA of every energy for them
     qs::zc *d_T = nullptr;  // per-CTA GEMM scratch
     size_t T_slots = 0, T_bytes = 0;
     qs::zc *d_Gws = nullptr;  // Gauss-Jordan workspace for orders above the shared-memory limit when nA < N

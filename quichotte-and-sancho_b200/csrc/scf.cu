@@ -665,11 +665,16 @@ size_t sweep_scratch_elems(const qs_handle *h) {
     const size_t per = std::max((size_t)h->Norb * std::max(h->nS, 1), (size_t)h->nA * h->nA);
     return per * std::min<size_t>(148 * 4, (size_t)4 * h->n);
 }
-// d_Y: the FFT intermediates; once Sigma2 is formed, G of the sweep (at least G_AA of every energy
-// and one full matrix), with the blocks' scratch behind it
+// d_Y: the FFT intermediates; once Sigma2 is formed, G of the sweep (G_AA of every energy, or full matrices
+// of a chunk of energies), with the blocks' scratch behind it. Where few states are active G_AA has room for a
+// few full matrices only, and the final sweep would go through the grid in as many launches (192 states, 12 of
+// them active, 1201 energies: 300 chunks, 192 ms a solve of 4 steps, now 28): a chunk has the matrices of three blocks
+// an SM, or as many as 256 MB hold, unless that memory is not there.
 size_t y_elems(const qs_handle *h) {
     const size_t fft = (size_t)12 * sigma2_count_pairs(h) * sigma2_plan(h->n).Nf;
-    const size_t g = std::max((size_t)h->n * h->nA * h->nA, (size_t)h->Norb * h->Norb);
+    const size_t nn = (size_t)h->Norb * h->Norb;
+    const size_t fill = std::min({(size_t)h->n, (size_t)3 * 148, ((size_t)256 << 20) / (nn * sizeof(zc))});
+    const size_t g = std::max((size_t)h->n * h->nA * h->nA, (h->small_chunks ? 1 : std::max<size_t>(fill, 1)) * nn);
     return std::max(fft, g + sweep_scratch_elems(h));
 }
 }  // namespace qs
@@ -734,6 +739,10 @@ int qs_create(const qs_problem *p, qs_handle **out) {
     size_t need = handle_need(h);
     size_t freeb = 0, totb = 0;
     QS_CUDA(h, cudaMemGetInfo(&freeb, &totb));
+    if (need + (512ull << 20) > freeb) {
+        h->small_chunks = true;
+        need = handle_need(h);
+    }
     if (need + (512ull << 20) > freeb) {
         h->err = "qs_create: HBM admission failed: the solve needs " + std::to_string(need >> 20) + " MiB, " +
                  std::to_string(freeb >> 20) + " MiB free";
