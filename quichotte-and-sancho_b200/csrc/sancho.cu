@@ -725,12 +725,7 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         delete h;
         return -(int)e;
     }
-    if (h->order >= 2) h->plan = sa_plan(n);
-    // the spectra are up to 14 % longer than the bubbles (18 % below 100 energies): direct sums where only those fit
-    size_t room = 0, all = 0;
-    const size_t values = nf * ((size_t)(h->order == 3 ? 14 : 3) * h->plan.L + (size_t)10 * n);
-    if (cudaMemGetInfo(&room, &all) != cudaSuccess || zc_ * values + 24 * tot * (4 + 2 * p->nhist) > room) h->plan = SaPlan{};
-    const size_t tm = nf * std::max(h->Nm, h->plan.L);  // bubbles, later their spectra
+    const int64_t n_vec = h->n_vec;
     auto up = [&](void **d, const void *src, size_t bytes) {
         int r = dalloc(q, d, bytes);
         if (r) return r;
@@ -741,40 +736,54 @@ int qsa_create(const qsa_problem *p, qsa_handle **out) {
         }
         return 0;
     };
-    const int64_t n_vec = h->n_vec;
-    q->red_len = broyden_red_len();
-    if ((rc = up((void **)&h->d_H, p->H, nf * zc_)) || (rc = up((void **)&h->d_GamL, p->GammaL, nf * zc_)) ||
-        (rc = up((void **)&h->d_GamR, p->GammaR, nf * zc_)) || (rc = up((void **)&h->d_U, p->U_site, Na * 8)) ||
-        (rc = up((void **)&h->d_omega, p->omega, (size_t)n * 8)) ||
-        (rc = dalloc(q, (void **)&q->d_x, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_F, n_vec * 8)) ||
-        (rc = dalloc(q, (void **)&q->d_Fold, n_vec * 8)) || (rc = dalloc(q, (void **)&q->d_xold, n_vec * 8)) ||
-        (rc = dalloc(q, (void **)&q->d_red, q->red_len * 8)) || (rc = reduce_scratch(q, Na)) ||
-        (h->nhist > 0 && ((rc = dalloc(q, &q->d_hdF, broyden_ld(n_vec) * 8 * h->nhist)) ||
-                          (rc = dalloc(q, &q->d_hU, broyden_ld(n_vec) * 8 * h->nhist)))) ||
-        (rc = dalloc(q, (void **)&h->d_Glt0, Na * zc_)) || (rc = dalloc(q, (void **)&h->d_W, tot * zc_)) ||
-        (rc = dalloc(q, (void **)&h->d_T, tot * zc_)) || (rc = dalloc(q, (void **)&h->d_gRd, (size_t)n * Na * zc_)) ||
-        (rc = dalloc(q, (void **)&h->d_gLd, (size_t)n * Na * zc_)) ||
-        (rc = dalloc(q, (void **)&h->d_spec, (size_t)n * Na * 8)) ||
-        (rc = dalloc(q, (void **)&h->d_sums, 2 * (size_t)Na * zc_)) ||
-        (rc = dalloc(q, (void **)&h->d_info, sizeof(int) * ((size_t)n + 1)))) {
-    }
-    for (int k = 0; k < 4 && !rc; k++) rc = dalloc(q, (void **)&h->d_E[k], tot * zc_);
-    if (!rc && h->plan.L) {
-        rc = dalloc(q, (void **)&h->d_tw, sizeof(zc) * h->plan.L);
-        if (!rc) rc = sa_twiddles(q->stream, h->plan, h->d_tw);
-    }
-    if (!rc && h->order >= 2) {
-        // (the transforms of order 2 need three: the spectra of G^r, G^a, G^<)
-        for (int k = 0; k < (h->order == 2 && h->plan.L ? 3 : 4) && !rc; k++) rc = dalloc(q, (void **)&h->d_chi[k], tm * zc_);
-        if (!rc) rc = dalloc(q, (void **)&h->d_S2R, tot * zc_);
-        if (!rc) rc = dalloc(q, (void **)&h->d_S2L, tot * zc_);
-    }
-    if (!rc && h->order == 3) {
-        for (int k = 0; k < 4 && !rc; k++) rc = dalloc(q, (void **)&h->d_phi[k], tm * zc_);
-        for (int k = 0; k < 3 && !rc; k++) rc = dalloc(q, (void **)&h->d_D[k], tm * zc_);
-        for (int k = 0; k < 3 && !rc; k++) rc = dalloc(q, (void **)&h->d_P[k], tm * zc_);
-        if (!rc) rc = dalloc(q, (void **)&h->d_S3R, tot * zc_);
-        if (!rc) rc = dalloc(q, (void **)&h->d_S3L, tot * zc_);
+    auto allocate = [&]() -> int {
+        const size_t tm = nf * std::max(h->Nm, h->plan.L);  // bubbles, later their spectra
+        int r = 0;
+        q->red_len = broyden_red_len();
+        if ((r = up((void **)&h->d_H, p->H, nf * zc_)) || (r = up((void **)&h->d_GamL, p->GammaL, nf * zc_)) ||
+            (r = up((void **)&h->d_GamR, p->GammaR, nf * zc_)) || (r = up((void **)&h->d_U, p->U_site, Na * 8)) ||
+            (r = up((void **)&h->d_omega, p->omega, (size_t)n * 8)) ||
+            (r = dalloc(q, (void **)&q->d_x, n_vec * 8)) || (r = dalloc(q, (void **)&q->d_F, n_vec * 8)) ||
+            (r = dalloc(q, (void **)&q->d_Fold, n_vec * 8)) || (r = dalloc(q, (void **)&q->d_xold, n_vec * 8)) ||
+            (r = dalloc(q, (void **)&q->d_red, q->red_len * 8)) || (r = reduce_scratch(q, Na)) ||
+            (h->nhist > 0 && ((r = dalloc(q, &q->d_hdF, broyden_ld(n_vec) * 8 * h->nhist)) ||
+                              (r = dalloc(q, &q->d_hU, broyden_ld(n_vec) * 8 * h->nhist)))) ||
+            (r = dalloc(q, (void **)&h->d_Glt0, Na * zc_)) || (r = dalloc(q, (void **)&h->d_W, tot * zc_)) ||
+            (r = dalloc(q, (void **)&h->d_T, tot * zc_)) || (r = dalloc(q, (void **)&h->d_gRd, (size_t)n * Na * zc_)) ||
+            (r = dalloc(q, (void **)&h->d_gLd, (size_t)n * Na * zc_)) ||
+            (r = dalloc(q, (void **)&h->d_spec, (size_t)n * Na * 8)) ||
+            (r = dalloc(q, (void **)&h->d_sums, 2 * (size_t)Na * zc_)) ||
+            (r = dalloc(q, (void **)&h->d_info, sizeof(int) * ((size_t)n + 1))))
+            return r;
+        for (int k = 0; k < 4 && !r; k++) r = dalloc(q, (void **)&h->d_E[k], tot * zc_);
+        if (!r && h->plan.L) {
+            r = dalloc(q, (void **)&h->d_tw, sizeof(zc) * h->plan.L);
+            if (!r) r = sa_twiddles(q->stream, h->plan, h->d_tw);
+        }
+        if (!r && h->order >= 2) {
+            // (the transforms of order 2 need three: the spectra of G^r, G^a, G^<)
+            for (int k = 0; k < (h->order == 2 && h->plan.L ? 3 : 4) && !r; k++) r = dalloc(q, (void **)&h->d_chi[k], tm * zc_);
+            if (!r) r = dalloc(q, (void **)&h->d_S2R, tot * zc_);
+            if (!r) r = dalloc(q, (void **)&h->d_S2L, tot * zc_);
+        }
+        if (!r && h->order == 3) {
+            for (int k = 0; k < 4 && !r; k++) r = dalloc(q, (void **)&h->d_phi[k], tm * zc_);
+            for (int k = 0; k < 3 && !r; k++) r = dalloc(q, (void **)&h->d_D[k], tm * zc_);
+            for (int k = 0; k < 3 && !r; k++) r = dalloc(q, (void **)&h->d_P[k], tm * zc_);
+            if (!r) r = dalloc(q, (void **)&h->d_S3R, tot * zc_);
+            if (!r) r = dalloc(q, (void **)&h->d_S3L, tot * zc_);
+        }
+        return r;
+    };
+    if (h->order >= 2) h->plan = sa_plan(n);
+    rc = allocate();
+    if (rc == -2 && h->plan.L) {
+        // the spectra are up to 14 % longer than the bubbles (18 % below 100 energies): direct sums where only those fit
+        release_all(q);
+        q->err.clear();
+        q->bytes_allocated = 0;
+        h->plan = SaPlan{};
+        rc = allocate();
     }
     if (!rc) {
         const int v = INT_MAX;

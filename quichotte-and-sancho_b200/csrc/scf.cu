@@ -57,6 +57,7 @@ int dalloc(qs_handle *h, void **p, size_t bytes) {
     cudaError_t e = cudaMallocAsync(p, bytes, h->stream);
     if (e != cudaSuccess) {
         h->err = "cudaMallocAsync of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e);
+        cudaGetLastError();  // (the check after a later launch must not find it)
         *p = nullptr;
         return -2;
     }
