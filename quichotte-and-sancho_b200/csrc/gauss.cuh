@@ -18,7 +18,7 @@ __device__ __forceinline__ zc scaled_recip(zc a) {
 
 // |Re| + |Im| >= 0, so its bit pattern orders like its value (a NaN is a large key: a row is
 // always found); 0 marks a row that is used or beyond the matrix
-constexpr unsigned long long INF_KEY = 0x7ff0000000000001ull;
+constexpr unsigned long long INF_KEY = 0x7ff0000000000001ull;  // of an infinite sum
 __device__ __forceinline__ unsigned long long pivot_key(zc v, bool open) {
     return open ? (unsigned long long)__double_as_longlong(cabs1(v)) + 1 : 0;
 }
@@ -42,8 +42,8 @@ template <int PW, int NBUF> struct PanelExchange {
     zc row[NBUF][PW][PB];  // each panel warp's candidate: 1 / pivot, then the rest of its row
     zc extra[PB];
     unsigned long long key[NBUF][PW];
-    int at[NBUF][PW];                       // its place << 16 | its row
-    int first_zero;                         // 1 + the first step with a zero pivot (LAPACK's INFO), 0 if none
+    int at[NBUF][PW];             // its place << 16 | its row
+    int first_zero;               // 1 + the first step with a zero pivot (LAPACK's INFO), 0 if none
     unsigned char perm[32 * PW];  // pivot row of a step
 };
 
